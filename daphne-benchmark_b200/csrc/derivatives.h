@@ -33,7 +33,30 @@ struct EvalArgs {  // (GridDev is in ndt_types.h)
     // rounds); null: every chunk is handed out and inactive ones skipped.
     int *active_chunks = nullptr;
     int *num_active = nullptr;
+    // FP32 pass: with at most wide_chunks chunks to evaluate, the wide kernel
+    // takes them (derivatives_wide.cu; 0: never), which needs the lane sums of
+    // its columns (kWideFloats per column of wide_chunks chunks) and two
+    // counters per chunk (zero between passes).  min_chunks: a host-side lower
+    // bound of the chunks of every pass (0: none).
+    int wide_chunks = 0;
+    int min_chunks = 0;
+    float *lane_sums = nullptr;
+    int *split_state = nullptr;
 };
+
+constexpr int kWideFloats = 37 * 32;  // 37 FP32 sums of 32 lanes
+constexpr int kWideResident = 3;      // blocks of the wide kernel per SM
+constexpr int kWideWaves = 5;
+// Chunks up to which the wide kernel is taken: kWideWaves columns per resident
+// block (555 chunks of 128-point tiles on 148 SMs).  A wave of it takes 10-15
+// us, a pass of the other kernel at least 46 us (one chunk, any number of
+// chunks up to 888); with many waves it loses, since its block barriers leave
+// issue slots idle (c5-scale batches: 73 ms against 45 ms).  Measured limits of
+// 1 / 2 / 3 / 5 / 9 waves, 256 learned-init alignments: 11.20 / 11.09 / 10.93 /
+// 10.86 / 11.07 ms.
+inline int wide_chunk_limit(int sms, int tile) { return kWideWaves * kWideResident * sms / (tile / 32); }
+int prepare_derivatives_wide();
+void launch_derivatives_wide(const EvalArgs &args, int sms, cudaStream_t st);
 
 constexpr int kOwn = 27;        // accepted pairs of one point per collect call, at most (3 x 3 x 3 probes)
 constexpr int kChunkBig = 8;    // tiles per large chunk of the FP32 pass by default (the FP64 pass: 1)

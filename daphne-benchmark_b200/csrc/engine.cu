@@ -171,7 +171,8 @@ struct ndt_ctx {
     // batch
     DevBuf chunks, chunk_begin, num_chunks, big_begin, small_begin, num_big, round_no, dev_launches;
     DevBuf points, offsets, guesses, states, tiles, tile_begin, num_tiles, partials, exc, out_T, out_conv, out_fit,
-        out_status, active, counters, p6, trans, flag_q, flag_n, flag_overflow, work_counter, active_chunks, num_active;
+        out_status, active, counters, p6, trans, flag_q, flag_n, flag_overflow, work_counter, active_chunks, num_active,
+        lane_sums, split_state;
     HostBuf h_offsets, h_active, h_counters, h_out;
     ndt_counters last{};
     long long launches = 0;
@@ -472,7 +473,7 @@ int build_grid(ndt_ctx *c, const float4 *d_map, int m) {
 constexpr unsigned kFlagCap = 1u << 20;     // default side-queue capacity (pairs per derivative pass)
 constexpr unsigned kFlagCapMax = 1u << 24;  // largest capacity ndt_set_side_queue_capacity accepts
 
-int prepare_flag_queue(ndt_ctx *c, EvalArgs &ea) {
+int prepare_scratch(ndt_ctx *c, EvalArgs &ea) {
     CK(c->flag_q.ensure(sizeof(int4) * c->flag_cap));
     CK(c->flag_n.ensure(sizeof(unsigned)));
     CK(c->flag_overflow.ensure(sizeof(int)));
@@ -482,6 +483,18 @@ int prepare_flag_queue(ndt_ctx *c, EvalArgs &ea) {
     ea.flag_overflow = c->flag_overflow.as<int>();
     CK(c->work_counter.ensure(sizeof(int)));
     ea.work_counter = c->work_counter.as<int>();
+    // the wide kernel's scratch
+    const int tile = kDerivVariants[c->variant].tile;
+    const int wide = wide_chunk_limit(c->num_sms, tile);
+    const size_t slots = (size_t)wide_chunk_limit(c->num_sms, 32);  // columns, and more than any tile's chunks
+    CK(c->lane_sums.ensure(sizeof(float) * kWideFloats * slots));
+    if (!c->split_state.p) {
+        CK(c->split_state.ensure(2 * sizeof(int) * slots));
+        CK(cudaMemsetAsync(c->split_state.p, 0, 2 * sizeof(int) * slots, c->stream));
+    }
+    ea.lane_sums = c->lane_sums.as<float>();
+    ea.split_state = c->split_state.as<int>();
+    ea.wide_chunks = wide;
     return NDT_OK;
 }
 
@@ -702,7 +715,7 @@ int run_batch(ndt_ctx *c, int B, const float4 *d_points, const int *d_offsets, i
     ea.d2 = c->d2;
     ea.compat = c->prm.compat;
     ea.counters = c->counters.as<Counters>();
-    if (int rc2 = prepare_flag_queue(c, ea)) return rc2;
+    if (int rc2 = prepare_scratch(c, ea)) return rc2;
     R.d_offsets = d_offsets;
     R.d_guesses = d_guesses;
     R.d_out = d_out;
@@ -724,6 +737,8 @@ int run_batch(ndt_ctx *c, int B, const float4 *d_points, const int *d_offsets, i
     // is fixed.
     R.fixed = R.P.compat && (R.P.step_max - R.P.step_min) > 0;
     R.max_rounds = R.fixed ? R.P.max_iterations + 3 : R.P.watchdog_evals + 1;
+    // every pass of a fixed batch hands out all its chunks, of at most kb tiles each
+    if (R.fixed) ea.min_chunks = total / (tile * R.kb);
     if (!R.fixed && R.precision == 0) {
         // alignments finish at different rounds: each FP32 pass hands out only the chunks of active ones
         CK(c->active_chunks.ensure(sizeof(int) * (size_t)max_tiles));
@@ -1028,7 +1043,7 @@ void ndt_destroy(ndt_ctx *c) {
                       &c->partials, &c->exc, &c->out_T, &c->out_conv,
                       &c->out_fit, &c->out_status, &c->active, &c->counters, &c->p6, &c->trans,
                       &c->flag_q, &c->flag_n, &c->flag_overflow, &c->work_counter, &c->active_chunks,
-                      &c->num_active};
+                      &c->num_active, &c->lane_sums, &c->split_state};
     for (DevBuf *b : bufs) b->release();
     HostBuf *hb[] = {&c->h_offsets, &c->h_active, &c->h_counters, &c->h_out};
     for (HostBuf *b : hb) b->release();
@@ -1238,7 +1253,7 @@ int ndt_score_batch_device(ndt_ctx *c, int B, const float *d_points, const int *
     ea.d2 = c->d2;
     ea.compat = c->prm.compat;
     ea.counters = c->counters.as<Counters>();
-    if (int rc2 = prepare_flag_queue(c, ea)) return rc2;
+    if (int rc2 = prepare_scratch(c, ea)) return rc2;
     R.d_offsets = d_offsets;
     R.d_guesses = d_poses;
     R.round_no = c->round_no.as<int>();
@@ -1249,6 +1264,7 @@ int ndt_score_batch_device(ndt_ctx *c, int B, const float *d_points, const int *
     R.precision = c->prm.precision;
     R.variant = c->variant;
     R.sms = c->num_sms;
+    ea.min_chunks = total_points / (tile * R.kb);
     if (int rc = enqueue_prologue(c, R, st)) return rc;
     int rc = launch_derivatives(R.ea, R.precision, R.variant, R.sms, st);
     if (rc) return cuda_fail(c, (cudaError_t)rc, "launch_derivatives");
@@ -1523,7 +1539,7 @@ int ndt_derivatives(ndt_ctx *c, const float *scan, const float *trans, int n, co
     ea.d2 = c->d2;
     ea.compat = c->prm.compat;
     ea.counters = c->counters.as<Counters>();
-    if (int rc2 = prepare_flag_queue(c, ea)) return rc2;
+    if (int rc2 = prepare_scratch(c, ea)) return rc2;
     rc = launch_derivatives(ea, c->prm.precision, c->variant, c->num_sms, st);
     if (rc) return cuda_fail(c, (cudaError_t)rc, "launch_derivatives");
     int nt = 0;
