@@ -207,99 +207,136 @@ __device__ __forceinline__ void copy_state(AlignState *dst, const AlignState *sr
     for (int i = lane; i < kStateVecs; i += 32) d[i] = s[i];
 }
 
-__global__ void init_kernel(AlignState *__restrict__ states, const float *__restrict__ guesses,
-                            const int *__restrict__ offsets, int B, StepParams P, double *__restrict__ exc) {
-    __shared__ AlignState s_st[kStateWarps];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int b = blockIdx.x * kStateWarps + warp;
-    if (b >= B) return;
-    for (int k = lane; k < kPartial; k += 32) exc[(size_t)b * kPartial + k] = 0.0;
-    AlignState &s = s_st[warp];
-    if (lane == 0) {
-        for (int k = 0; k < 16; ++k) s.T[k] = guesses[16 * (size_t)b + k];
-        pose_vector(P.compat != 0, s.T, s.p);
-        if (!P.compat) build_tm_corrected(s.T, s.p);
-        for (int i = 0; i < 6; ++i) {
-            s.x_t[i] = s.p[i];
-            s.dir[i] = 0.0;
-            s.g[i] = 0.0;
-        }
-        for (int k = 0; k < 36; ++k) s.H[k] = 0.0;
-        s.score = 0.0;
-        s.phi_0 = s.d_phi_0 = s.a_l = s.f_l = s.g_l = s.a_u = s.f_u = s.g_u = s.a_t = 0.0;
-        s.phi_t = s.d_phi_t = s.psi_t = s.d_psi_t = 0.0;
-        s.step_max = P.step_max;
-        s.step_min = P.step_min;
-        s.nr_iterations = 0;
-        s.step_iterations = 0;
-        s.open_interval = 1;
-        s.interval_converged = 0;
-        s.converged = 0;
-        s.evals = 0;
-        s.status = 0;
-        s.n = offsets[b + 1] - offsets[b];
-        set_angles(s, s.p, P.compat);
-        s.eval_mode = kEvalFull;
-        s.phase = kPhaseInitEval;
+// The state of an alignment before its first evaluation (one thread).
+__device__ void init_state(AlignState &s, const float *__restrict__ guess, int n, const StepParams &P) {
+    for (int k = 0; k < 16; ++k) s.T[k] = guess[k];
+    pose_vector(P.compat != 0, s.T, s.p);
+    if (!P.compat) build_tm_corrected(s.T, s.p);
+    for (int i = 0; i < 6; ++i) {
+        s.x_t[i] = s.p[i];
+        s.dir[i] = 0.0;
+        s.g[i] = 0.0;
     }
-    __syncwarp();
-    copy_state(states + b, &s, lane);
+    for (int k = 0; k < 36; ++k) s.H[k] = 0.0;
+    s.score = 0.0;
+    s.phi_0 = s.d_phi_0 = s.a_l = s.f_l = s.g_l = s.a_u = s.f_u = s.g_u = s.a_t = 0.0;
+    s.phi_t = s.d_phi_t = s.psi_t = s.d_psi_t = 0.0;
+    s.step_max = P.step_max;
+    s.step_min = P.step_min;
+    s.nr_iterations = 0;
+    s.step_iterations = 0;
+    s.open_interval = 1;
+    s.interval_converged = 0;
+    s.converged = 0;
+    s.evals = 0;
+    s.status = 0;
+    s.n = n;
+    set_angles(s, s.p, P.compat);
+    s.eval_mode = kEvalFull;
+    s.phase = kPhaseInitEval;
 }
 
 // FP64 sum of the alignment's chunk partials in chunk order (deterministic;
 // each lane sums the values k = lane, lane + 32 with its loads issued 8 at a
-// time), then lane 0 advances the state machine.
-__global__ void step_kernel(AlignState *__restrict__ states, const double *__restrict__ partials,
-                            const int *__restrict__ chunk_begin, double *__restrict__ exc, int B, StepParams P,
-                            int *__restrict__ active, Counters *__restrict__ counters) {
+// time), then lane 0 advances the state machine; the chunks of an alignment
+// that asks for another evaluation go to the active list (their order in it
+// changes no result, since each chunk writes its own partial slot).  The last
+// block to finish ends the round: the counters that separate launches would
+// have to clear or read (four memsets, the list's compaction, the loop
+// condition: 10 us of a 21 us round tail) are set here.
+__global__ void step_kernel(AlignState *__restrict__ states, const double *__restrict__ partials, TileLists L,
+                            double *__restrict__ exc, int B, StepParams P, RoundEnd end) {
     __shared__ double s_v[kStateWarps][kPartial];
     __shared__ AlignState s_st[kStateWarps];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (counters && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&counters->rounds, 1ull);
+    RoundCtl *ctl = end.ctl;
     const int b = blockIdx.x * kStateWarps + warp;
-    if (b >= B) return;
     AlignState *st = states + b;
-    const int mode = st->eval_mode;
-    if (mode == kEvalNone) return;
-    const int c0 = chunk_begin[b], c1 = chunk_begin[b + 1];
-    for (int k = lane; k < kPartial; k += 32) {
-        double v = 0.0;
-        int c = c0;
-        for (; c + 8 <= c1; c += 8) {
-            double t[8];
+    const int mode = b < B ? st->eval_mode : kEvalNone;
+    if (mode != kEvalNone) {
+        const int c0 = L.chunk_begin[b], c1 = L.chunk_begin[b + 1];
+        for (int k = lane; k < kPartial; k += 32) {
+            double v = 0.0;
+            int c = c0;
+            for (; c + 8 <= c1; c += 8) {
+                double t[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) t[u] = partials[(size_t)(c + u) * kPartial + k];
+                for (int u = 0; u < 8; ++u) t[u] = partials[(size_t)(c + u) * kPartial + k];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) v += t[u];
+                for (int u = 0; u < 8; ++u) v += t[u];
+            }
+            for (; c < c1; ++c) v += partials[(size_t)c * kPartial + k];
+            double *e = exc + (size_t)b * kPartial + k;
+            v += *e;
+            *e = 0.0;
+            s_v[warp][k] = v;
         }
-        for (; c < c1; ++c) v += partials[(size_t)c * kPartial + k];
-        double *e = exc + (size_t)b * kPartial + k;
-        v += *e;
-        *e = 0.0;
-        s_v[warp][k] = v;
+        AlignState &s = s_st[warp];
+        copy_state(&s, st, lane);
+        __syncwarp();
+        unsigned long long at = 0;
+        int nb = 0, ns = 0, b0 = 0, s0 = 0;
+        if (lane == 0) {
+            const double *v = s_v[warp];
+            if (mode == kEvalFull || mode == kEvalGradient) {
+                s.score = v[0];
+                for (int i = 0; i < 6; ++i) s.g[i] = v[1 + i];
+            }
+            if (mode == kEvalFull || mode == kEvalHessian) {
+                for (int k = 0; k < 36; ++k) s.H[k] = v[7 + k];
+            } else {
+                for (int k = 0; k < 36; ++k) s.H[k] = 0.0;  // computeDerivatives zeroes it (kernel.cpp:667)
+            }
+            s.evals++;
+            s.eval_mode = kEvalNone;
+            advance(s, P);
+            if (s.eval_mode != kEvalNone) {
+                atomicAdd(&ctl->next_active, 1);
+                if (L.active_chunks) {
+                    b0 = L.big_begin[b];
+                    nb = L.big_begin[b + 1] - b0;
+                    s0 = L.small_begin[b];
+                    ns = L.small_begin[b + 1] - s0;
+                    at = atomicAdd(&ctl->next_list, (unsigned long long)nb << 32 | (unsigned)ns);
+                }
+            }
+            atomicAdd(&ctl->counters.evaluations, 1ull);
+        }
+        __syncwarp();
+        copy_state(st, &s, lane);
+        if (L.active_chunks) {
+            at = __shfl_sync(0xffffffffu, at, 0);
+            nb = __shfl_sync(0xffffffffu, nb, 0);
+            ns = __shfl_sync(0xffffffffu, ns, 0);
+            b0 = __shfl_sync(0xffffffffu, b0, 0);
+            s0 = __shfl_sync(0xffffffffu, s0, 0);
+            const int at_big = (int)(at >> 32), at_small = (int)(at & 0xffffffffu);
+            const int total_big = *L.num_big;
+            for (int j = lane; j < nb; j += 32) L.active_chunks[at_big + j] = b0 + j;
+            for (int j = lane; j < ns; j += 32) L.active_chunks[L.capacity - 1 - (at_small + j)] = total_big + s0 + j;
+        }
     }
-    AlignState &s = s_st[warp];
-    copy_state(&s, st, lane);
-    __syncwarp();
-    if (lane == 0) {
-        const double *v = s_v[warp];
-        if (mode == kEvalFull || mode == kEvalGradient) {
-            s.score = v[0];
-            for (int i = 0; i < 6; ++i) s.g[i] = v[1 + i];
-        }
-        if (mode == kEvalFull || mode == kEvalHessian) {
-            for (int k = 0; k < 36; ++k) s.H[k] = v[7 + k];
-        } else {
-            for (int k = 0; k < 36; ++k) s.H[k] = 0.0;  // computeDerivatives zeroes it (kernel.cpp:667)
-        }
-        s.evals++;
-        s.eval_mode = kEvalNone;
-        advance(s, P);
-        if (s.eval_mode != kEvalNone) atomicAdd(active, 1);
-        if (counters) atomicAdd(&counters->evaluations, 1ull);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    if (atomicAdd(&ctl->ticket, 1) != (int)gridDim.x - 1) return;
+    __threadfence();
+    const int active = atomicExch(&ctl->next_active, 0);
+    const unsigned long long list = atomicExch(&ctl->next_list, 0ull);
+    ctl->active = active;
+    ctl->num_active[0] = (int)(list >> 32);
+    ctl->num_active[1] = (int)(list & 0xffffffffu);
+    ctl->work_counter = 0;
+    ctl->flag_n = 0;
+    ctl->ticket = 0;
+    ctl->counters.rounds += 1;
+    const int r = ++ctl->round_no;
+    if (end.graph) {
+        // another round while an alignment asked for an evaluation and the round
+        // budget (the evaluation watchdog) is not spent, so the loop always ends
+        *end.launches += (unsigned long long)end.per_round;
+        cudaGraphSetConditional(end.loop, (active > 0 && r < end.max_rounds) ? 1u : 0u);
     }
-    __syncwarp();
-    copy_state(st, &s, lane);
 }
 
 __global__ void finalize_kernel(const AlignState *__restrict__ states, int B, float *__restrict__ out,
@@ -390,32 +427,33 @@ __global__ void scan3_kernel(ScanArgs a, int n) {
     if (total && t == nt - 1) *total = run;
 }
 
-// One warp per alignment writes its tiles, its chunks (large ones at the
-// front of the list, small ones after every large one) and its slot range.
-__global__ void tile_fill_kernel(const int *__restrict__ offsets, int B, int tile, int kb, int ks, TileLists L) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= B) return;
-    const int lo = offsets[warp], hi = offsets[warp + 1];
-    const int t0 = L.tile_begin[warp], t1 = L.tile_begin[warp + 1];
+// One warp writes its alignment's tiles, its chunks (large ones at the front
+// of the list, small ones after every large one), its slot range and its
+// entries of the first pass's active list.
+__device__ __forceinline__ void fill_lists(const int *__restrict__ offsets, int b, int B, int tile, int kb, int ks,
+                                           const TileLists &L) {
+    const int lane = threadIdx.x & 31;
+    const int lo = offsets[b], hi = offsets[b + 1];
+    const int t0 = L.tile_begin[b], t1 = L.tile_begin[b + 1];
     for (int t = t0 + lane; t < t1; t += 32) {
         Tile x;
-        x.align = warp;
+        x.align = b;
         x.start = lo + (t - t0) * tile;
         x.end = min(hi, x.start + tile);
         x.slot = t;
         L.tiles[t] = x;
     }
-    const int b0 = L.big_begin[warp], nb = L.big_begin[warp + 1] - b0;
-    const int s0 = L.small_begin[warp], ns = L.small_begin[warp + 1] - s0;
+    const int b0 = L.big_begin[b], nb = L.big_begin[b + 1] - b0;
+    const int s0 = L.small_begin[b], ns = L.small_begin[b + 1] - s0;
     const int slot0 = b0 + s0;
     const int total_big = *L.num_big;
     if (lane == 0) {
-        L.chunk_begin[warp] = slot0;
-        if (warp == B - 1) L.chunk_begin[B] = *L.num_chunks = slot0 + nb + ns;
+        L.chunk_begin[b] = slot0;
+        if (b == B - 1) L.chunk_begin[B] = *L.num_chunks = slot0 + nb + ns;
     }
     for (int j = lane; j < nb + ns; j += 32) {
         Chunk x;
-        x.align = warp;
+        x.align = b;
         int pos;
         if (j < nb) {
             x.first = t0 + j * kb;
@@ -428,6 +466,104 @@ __global__ void tile_fill_kernel(const int *__restrict__ offsets, int B, int til
         }
         x.slot = slot0 + j;
         L.chunks[pos] = x;
+        if (L.active_chunks) L.active_chunks[j < nb ? pos : L.capacity - 1 - (s0 + j - nb)] = pos;
+    }
+}
+
+__global__ void tile_fill_kernel(const int *__restrict__ offsets, int B, int tile, int kb, int ks, TileLists L) {
+    const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (b < B) fill_lists(offsets, b, B, tile, kb, ks, L);
+}
+
+// Start of a batch, one warp per alignment: its lists and its state.  Thread
+// 0 also sets the first pass's active-list counts.
+__global__ void fill_init_kernel(const int *__restrict__ offsets, int B, int tile, int kb, int ks, TileLists L,
+                                 AlignState *__restrict__ states, const float *__restrict__ guesses, StepParams P,
+                                 double *__restrict__ exc, RoundCtl *__restrict__ ctl) {
+    __shared__ AlignState s_st[kStateWarps];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int b = blockIdx.x * kStateWarps + warp;
+    if (b >= B) return;
+    if (b == 0 && lane == 0) {
+        ctl->num_active[0] = *L.num_big;
+        ctl->num_active[1] = L.small_begin[B];
+    }
+    for (int k = lane; k < kPartial; k += 32) exc[(size_t)b * kPartial + k] = 0.0;
+    AlignState &s = s_st[warp];
+    if (lane == 0) init_state(s, guesses + 16 * (size_t)b, offsets[b + 1] - offsets[b], P);
+    fill_lists(offsets, b, B, tile, kb, ks, L);
+    __syncwarp();
+    copy_state(states + b, &s, lane);
+}
+
+// Tile and chunk counts per alignment and their exclusive scans by one block
+// (up to kOneBlockLists alignments: three launches in one), and the round
+// control cleared.
+__device__ __forceinline__ void clear_ctl(RoundCtl *ctl, int reset_counters, int t) {
+    static_assert(sizeof(RoundCtl) % 4 == 0 && sizeof(Counters) % 8 == 0, "cleared by words");
+    const int head = (int)((sizeof(RoundCtl) - sizeof(Counters)) / 4), all = (int)(sizeof(RoundCtl) / 4);
+    if (t < (reset_counters ? all : head)) reinterpret_cast<int *>(ctl)[t] = 0;
+}
+
+__global__ void clear_ctl_kernel(RoundCtl *ctl, int reset_counters) { clear_ctl(ctl, reset_counters, threadIdx.x); }
+
+__global__ void __launch_bounds__(1024) lists_kernel(const int *__restrict__ offsets, int B, int tile, int kb, int ks,
+                                                     TileLists L, RoundCtl *ctl, int reset_counters) {
+    __shared__ int s_warp[3][32];
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    clear_ctl(ctl, reset_counters, t);
+    const int per = (B + 1023) / 1024;
+    const int lo = min(B, t * per), hi = min(B, lo + per);
+    int sum[3] = {0, 0, 0};
+    for (int b = lo; b < hi; ++b) {
+        const int n = offsets[b + 1] - offsets[b];
+        const int tiles = n > 0 ? (n + tile - 1) / tile : 0;
+        int nb, ns;
+        chunk_plan(tiles, kb, ks, nb, ns);
+        sum[0] += tiles;
+        sum[1] += nb;
+        sum[2] += ns;
+    }
+    int incl[3] = {sum[0], sum[1], sum[2]};
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const int v = __shfl_up_sync(0xffffffffu, incl[q], o);
+            if (lane >= o) incl[q] += v;
+        }
+    if (lane == 31)
+        for (int q = 0; q < 3; ++q) s_warp[q][w] = incl[q];
+    __syncthreads();
+    if (w < 3) {
+        const int v = s_warp[w][lane];
+        int inc2 = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, inc2, o);
+            if (lane >= o) inc2 += u;
+        }
+        s_warp[w][lane] = inc2 - v;
+    }
+    __syncthreads();
+    int run[3];
+    for (int q = 0; q < 3; ++q) run[q] = s_warp[q][w] + incl[q] - sum[q];
+    for (int b = lo; b < hi; ++b) {
+        L.tile_begin[b] = run[0];
+        L.big_begin[b] = run[1];
+        L.small_begin[b] = run[2];
+        const int n = offsets[b + 1] - offsets[b];
+        const int tiles = n > 0 ? (n + tile - 1) / tile : 0;
+        int nb, ns;
+        chunk_plan(tiles, kb, ks, nb, ns);
+        run[0] += tiles;
+        run[1] += nb;
+        run[2] += ns;
+    }
+    if (t == 1023) {  // (its run ends at B)
+        L.tile_begin[B] = *L.num_tiles = run[0];
+        L.big_begin[B] = *L.num_big = run[1];
+        L.small_begin[B] = run[2];
     }
 }
 
@@ -457,7 +593,7 @@ int launch_prepare_eval(AlignState *d_state, const double *d_p6, int n, double *
     return (int)cudaGetLastError();
 }
 
-int launch_tiles(const int *d_offsets, int B, int tile, int kb, int ks, const TileLists &L, cudaStream_t st) {
+static void launch_scans(const int *d_offsets, int B, int tile, int kb, int ks, const TileLists &L, cudaStream_t st) {
     tile_count_kernel<<<(B + 1 + 255) / 256, 256, 0, st>>>(d_offsets, B, tile, kb, ks, L);
     ScanArgs a;
     a.data[0] = L.tile_begin;
@@ -467,21 +603,33 @@ int launch_tiles(const int *d_offsets, int B, int tile, int kb, int ks, const Ti
     a.data[2] = L.small_begin;
     a.total[2] = nullptr;
     scan3_kernel<<<3, 1024, 0, st>>>(a, B + 1);
+}
+
+int launch_tiles(const int *d_offsets, int B, int tile, int kb, int ks, const TileLists &L, cudaStream_t st) {
+    launch_scans(d_offsets, B, tile, kb, ks, L, st);
     tile_fill_kernel<<<(B * 32 + 255) / 256, 256, 0, st>>>(d_offsets, B, tile, kb, ks, L);
     return (int)cudaGetLastError();
 }
 
-int launch_init(AlignState *d_states, const float *d_guesses, const int *d_offsets, int B, const StepParams &P,
-                double *d_exc, cudaStream_t st) {
-    init_kernel<<<(B + kStateWarps - 1) / kStateWarps, 32 * kStateWarps, 0, st>>>(d_states, d_guesses, d_offsets, B,
-                                                                                  P, d_exc);
+int launch_prologue(const int *d_offsets, int B, int tile, int kb, int ks, const TileLists &L, AlignState *d_states,
+                    const float *d_guesses, const StepParams &P, double *d_exc, RoundCtl *d_ctl, bool reset_counters,
+                    cudaStream_t st, int *launches) {
+    if (B <= kOneBlockLists) {
+        lists_kernel<<<1, 1024, 0, st>>>(d_offsets, B, tile, kb, ks, L, d_ctl, reset_counters ? 1 : 0);
+    } else {
+        clear_ctl_kernel<<<1, 64, 0, st>>>(d_ctl, reset_counters ? 1 : 0);
+        launch_scans(d_offsets, B, tile, kb, ks, L, st);
+    }
+    fill_init_kernel<<<(B + kStateWarps - 1) / kStateWarps, 32 * kStateWarps, 0, st>>>(
+        d_offsets, B, tile, kb, ks, L, d_states, d_guesses, P, d_exc, d_ctl);
+    *launches = prologue_launches(B);
     return (int)cudaGetLastError();
 }
 
-int launch_step(AlignState *d_states, const double *d_partials, const int *d_chunk_begin, double *d_exc, int B,
-                const StepParams &P, int *d_active, Counters *d_counters, cudaStream_t st) {
-    step_kernel<<<(B + kStateWarps - 1) / kStateWarps, 32 * kStateWarps, 0, st>>>(d_states, d_partials, d_chunk_begin,
-                                                                                  d_exc, B, P, d_active, d_counters);
+int launch_step(AlignState *d_states, const double *d_partials, const TileLists &L, double *d_exc, int B,
+                const StepParams &P, const RoundEnd &end, cudaStream_t st) {
+    step_kernel<<<(B + kStateWarps - 1) / kStateWarps, 32 * kStateWarps, 0, st>>>(d_states, d_partials, L, d_exc, B,
+                                                                                  P, end);
     return (int)cudaGetLastError();
 }
 

@@ -27,12 +27,14 @@ struct EvalArgs {  // (GridDev is in ndt_types.h)
     unsigned flag_cap;     // queue capacity
     int *flag_overflow;    // set when the queue overflowed
     int *work_counter;     // FP32 pass: next chunk (reset by launch_derivatives)
-    // FP32 pass, optional: the pass first compacts the chunks whose alignment
-    // asks for an evaluation into active_chunks (capacity: the chunk count)
-    // and hands out only those (batches whose alignments finish at different
-    // rounds); null: every chunk is handed out and inactive ones skipped.
+    // FP32 pass, optional: the chunks of the alignments that ask for an
+    // evaluation (batches whose alignments finish at different rounds), listed
+    // by the step kernel; null: every chunk is handed out and inactive ones
+    // skipped.  num_active: large and small chunks in the list.
     int *active_chunks = nullptr;
-    int *num_active = nullptr;
+    const int *num_active = nullptr;
+    int active_capacity = 0;
+    bool reset = true;     // launch_derivatives clears flag_n and work_counter (else the caller has)
     // FP32 pass: with at most wide_chunks chunks to evaluate, the wide kernel
     // takes them (derivatives_wide.cu; 0: never), which needs the lane sums of
     // its columns (kWideFloats per column of wide_chunks chunks) and two
@@ -90,7 +92,12 @@ extern const DerivVariant kDerivVariants[kNumDerivVariants];
 int launch_derivatives(const EvalArgs &args, int precision, int variant, int sms, cudaStream_t st);
 // The FP64 pass alone (256-point tiles).
 int launch_derivatives_f64(const EvalArgs &args, int sms, cudaStream_t st);
-// Kernel launches per launch_derivatives call (FP32: pass + flagged pairs; FP64: pass).
-constexpr int kDerivLaunchesFP32 = 2;
+// Kernel launches of one launch_derivatives call (FP32: one or both kernels of
+// the pass, and the flagged pairs; FP64: the pass).
+inline bool launches_wide(const EvalArgs &a) { return a.wide_chunks > 0 && a.min_chunks <= a.wide_chunks; }
+inline bool launches_many(const EvalArgs &a) { return a.max_tiles > a.wide_chunks; }
+inline int derivative_launches(const EvalArgs &a, int precision) {
+    return precision == 1 ? 1 : 1 + (launches_wide(a) ? 1 : 0) + (launches_many(a) ? 1 : 0);
+}
 
 }  // namespace ndt

@@ -271,23 +271,6 @@ __device__ __forceinline__ void eval_steps(const WarpPairs &P, const unsigned (*
     }
 }
 
-// The chunks of the alignments that ask for an evaluation, in a list the FP32
-// pass hands out (warp-aggregated appends; the order of the list does not
-// change any result, since each chunk writes its own partial slot).
-__global__ void active_chunks_kernel(const __grid_constant__ EvalArgs args) {
-    const int nc = *args.num_chunks;
-    const int lane = threadIdx.x & 31;
-    for (int base = blockIdx.x * blockDim.x; base < nc; base += gridDim.x * blockDim.x) {
-        const int c = base + threadIdx.x;
-        const bool act = c < nc && args.states[args.chunks[c].align].eval_mode != kEvalNone;
-        const unsigned bal = __ballot_sync(0xffffffffu, act);
-        int at = 0;
-        if (lane == 0 && bal) at = atomicAdd(args.num_active, __popc(bal));
-        at = __shfl_sync(0xffffffffu, at, 0);
-        if (act) args.active_chunks[at + __popc(bal & ((1u << lane) - 1u))] = c;
-    }
-}
-
 // COMPAT: the reference's Hessian form and pose build (else corrected); WIN: the
 // map has a probe-window table (the neighbour search compiles only the paths it
 // can take, a smaller instruction footprint).
@@ -323,7 +306,7 @@ __global__ void __launch_bounds__(TILE, MINB) derivative_f32_kernel(const __grid
     P.d1 = (float)args.d1;
     P.d2 = (float)args.d2;
 
-    const int nc = args.num_active ? *args.num_active : *args.num_chunks;
+    const int nc = pass_chunks(args);
     if (nc <= args.wide_chunks) return;  // the wide kernel's
     for (int k = 0; k < kAcc; ++k) P.acc[k * TILE] = 0.0f;
     if (lane == 0) s_pairs[warp] = 0;
@@ -340,7 +323,7 @@ __global__ void __launch_bounds__(TILE, MINB) derivative_f32_kernel(const __grid
     for (int it = 0; it <= nc; ++it) {
         if (threadIdx.x == 0) {
             const int k = atomicAdd(args.work_counter, 1);
-            s_chunk[parity] = k < nc ? (args.active_chunks ? args.active_chunks[k] : k) : -1;
+            s_chunk[parity] = k < nc ? active_chunk(args, k) : -1;
         }
         __syncthreads();
         const int chunk = s_chunk[parity];
@@ -493,14 +476,12 @@ int launch_derivatives(const EvalArgs &args, int precision, int variant, int sms
     if (args.tile_size != v.tile) return (int)cudaErrorInvalidValue;
     long long want = (long long)sms * v.min_blocks;
     int blocks = (int)(want < args.max_tiles ? want : args.max_tiles);
-    cudaMemsetAsync(args.flag_n, 0, sizeof(unsigned), st);
-    cudaMemsetAsync(args.work_counter, 0, sizeof(int), st);
-    if (args.active_chunks) {
-        cudaMemsetAsync(args.num_active, 0, sizeof(int), st);
-        active_chunks_kernel<<<sms * 4, 256, 0, st>>>(args);
+    if (args.reset) {
+        cudaMemsetAsync(args.flag_n, 0, sizeof(unsigned), st);
+        cudaMemsetAsync(args.work_counter, 0, sizeof(int), st);
     }
-    if (args.wide_chunks > 0 && args.min_chunks <= args.wide_chunks) launch_derivatives_wide(args, sms, st);
-    if (args.max_tiles > args.wide_chunks) {
+    if (launches_wide(args)) launch_derivatives_wide(args, sms, st);
+    if (launches_many(args)) {
         switch (variant) {
             case 0: launch_one<256, 2>(args, blocks, st); break;
             case 1: launch_one<256, 1>(args, blocks, st); break;

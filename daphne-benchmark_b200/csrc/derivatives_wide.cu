@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(kBlock, kWideResident) derivative_wide_kernel(
     float *contrib = reinterpret_cast<float *>(sm.step[warp]) + lane;
     const float d1 = (float)args.d1, d2 = (float)args.d2;
 
-    const int nc = args.num_active ? *args.num_active : *args.num_chunks;
+    const int nc = pass_chunks(args);
     if (nc > args.wide_chunks) return;  // the other kernel's
     const int items = nc * W;  // (chunk, column)
     if (threadIdx.x == 0) {
@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(kBlock, kWideResident) derivative_wide_kernel(
         parity ^= 1;
         if (item >= items) break;
         const int slot_k = item / W, w = item % W;
-        const Chunk ck = args.chunks[args.active_chunks ? args.active_chunks[slot_k] : slot_k];
+        const Chunk ck = args.chunks[active_chunk(args, slot_k)];
         const AlignState *st = args.states + ck.align;
         if (threadIdx.x == 0) s_mode = st->eval_mode;
         if (threadIdx.x < 12) s_T[threadIdx.x] = st->T[threadIdx.x];

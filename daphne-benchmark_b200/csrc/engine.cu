@@ -111,10 +111,9 @@ struct RunPlan {
     int *d_conv;
     double *d_fit;
     int *d_status;
-    int *active;
-    int *round_no;
+    RoundCtl *ctl;
     unsigned long long *dev_launches;
-    int B, tile, kb, ks, max_rounds, precision, variant, sms, fixed;
+    int B, tile, kb, ks, max_rounds, precision, variant, sms, fixed, first;
 };
 
 struct BatchGraph {
@@ -169,10 +168,9 @@ struct ndt_ctx {
     int grid_nl = 0;
     ndt::SortedMap grid_sorted{nullptr, nullptr};
     // batch
-    DevBuf chunks, chunk_begin, num_chunks, big_begin, small_begin, num_big, round_no, dev_launches;
+    DevBuf chunks, chunk_begin, num_chunks, big_begin, small_begin, num_big, dev_launches;
     DevBuf points, offsets, guesses, states, tiles, tile_begin, num_tiles, partials, exc, out_T, out_conv, out_fit,
-        out_status, active, counters, p6, trans, flag_q, flag_n, flag_overflow, work_counter, active_chunks, num_active,
-        lane_sums, split_state;
+        out_status, ctl, p6, trans, flag_q, active_chunks, lane_sums, split_state;
     HostBuf h_offsets, h_active, h_counters, h_out;
     ndt_counters last{};
     long long launches = 0;
@@ -475,14 +473,14 @@ constexpr unsigned kFlagCapMax = 1u << 24;  // largest capacity ndt_set_side_que
 
 int prepare_scratch(ndt_ctx *c, EvalArgs &ea) {
     CK(c->flag_q.ensure(sizeof(int4) * c->flag_cap));
-    CK(c->flag_n.ensure(sizeof(unsigned)));
-    CK(c->flag_overflow.ensure(sizeof(int)));
+    CK(c->ctl.ensure(sizeof(RoundCtl)));
+    RoundCtl *ctl = c->ctl.as<RoundCtl>();
     ea.flag_q = c->flag_q.as<int4>();
-    ea.flag_n = c->flag_n.as<unsigned>();
+    ea.flag_n = &ctl->flag_n;
     ea.flag_cap = c->flag_cap;
-    ea.flag_overflow = c->flag_overflow.as<int>();
-    CK(c->work_counter.ensure(sizeof(int)));
-    ea.work_counter = c->work_counter.as<int>();
+    ea.flag_overflow = &ctl->flag_overflow;
+    ea.work_counter = &ctl->work_counter;
+    ea.counters = &ctl->counters;
     // the wide kernel's scratch
     const int tile = kDerivVariants[c->variant].tile;
     const int wide = wide_chunk_limit(c->num_sms, tile);
@@ -527,37 +525,24 @@ int chunk_big(const ndt_ctx *c) { return c->prm.precision == 1 ? 1 : c->chunk_ti
 int chunk_small(const ndt_ctx *c) { return c->prm.precision == 1 ? 1 : std::min(kChunkSmall, c->chunk_tiles); }
 
 // Device-side batch: everything already on the device.
-// Round-loop condition of a batch graph: another round while an alignment
-// asked for an evaluation and the round budget (the evaluation watchdog) is
-// not spent, so the loop always ends.
-__global__ void round_cond_kernel(cudaGraphConditionalHandle h, const int *active, int *round_no, int max_rounds,
-                                  unsigned long long *launches, int per_round) {
-    const int r = ++*round_no;
-    *launches += (unsigned long long)per_round;
-    cudaGraphSetConditional(h, (*active > 0 && r < max_rounds) ? 1u : 0u);
-}
-
-int enqueue_prologue(ndt_ctx *c, const RunPlan &R, cudaStream_t st) {
-    CK(cudaMemsetAsync(R.ea.flag_overflow, 0, sizeof(int), st));
-    CK(cudaMemsetAsync(R.round_no, 0, sizeof(int), st));
-    int rc = launch_tiles(R.d_offsets, R.B, R.tile, R.kb, R.ks, R.L, st);
-    if (rc) return cuda_fail(c, (cudaError_t)rc, "launch_tiles");
-    rc = launch_init(R.ea.states, R.d_guesses, R.d_offsets, R.B, R.P, R.ea.exc, st);
-    if (rc) return cuda_fail(c, (cudaError_t)rc, "launch_init");
+int enqueue_prologue(ndt_ctx *c, const RunPlan &R, cudaStream_t st, int *launches) {
+    int rc = launch_prologue(R.d_offsets, R.B, R.tile, R.kb, R.ks, R.L, R.ea.states, R.d_guesses, R.P, R.ea.exc, R.ctl,
+                             R.first != 0, st, launches);
+    if (rc) return cuda_fail(c, (cudaError_t)rc, "launch_prologue");
     return NDT_OK;
 }
 
-// One round: the derivative pass, then the step kernel (which counts in
-// *active the alignments that ask for another evaluation).
-int enqueue_round(ndt_ctx *c, const RunPlan &R, cudaStream_t st, bool profile) {
+// One round: the derivative pass, then the step kernel (which counts the
+// alignments that ask for another evaluation, prepares the next pass and, in
+// a batch graph, sets the loop's condition).
+int enqueue_round(ndt_ctx *c, const RunPlan &R, cudaStream_t st, bool profile, const RoundEnd &end) {
     cudaEvent_t e0 = profile ? next_event(c) : nullptr;
     if (e0) CK(cudaEventRecord(e0, st));
     int rc = launch_derivatives(R.ea, R.precision, R.variant, R.sms, st);
     if (rc) return cuda_fail(c, (cudaError_t)rc, "launch_derivatives");
     cudaEvent_t e1 = profile ? next_event(c) : nullptr;
     if (e1) CK(cudaEventRecord(e1, st));
-    CK(cudaMemsetAsync(R.active, 0, sizeof(int), st));
-    rc = launch_step(R.ea.states, R.ea.partials, R.L.chunk_begin, R.ea.exc, R.B, R.P, R.active, R.ea.counters, st);
+    rc = launch_step(R.ea.states, R.ea.partials, R.L, R.ea.exc, R.B, R.P, end, st);
     if (rc) return cuda_fail(c, (cudaError_t)rc, "launch_step");
     return NDT_OK;
 }
@@ -569,12 +554,20 @@ int enqueue_epilogue(ndt_ctx *c, const RunPlan &R, cudaStream_t st) {
 }
 
 // Kernel launches of one round (derivative pass + step kernel).
-int round_launches(const RunPlan &R) {
-    return 1 + (R.precision == 1 ? 1 : kDerivLaunchesFP32 + (R.ea.active_chunks ? 1 : 0));
+int round_launches(const RunPlan &R) { return 1 + derivative_launches(R.ea, R.precision); }
+
+RoundEnd round_end(const RunPlan &R) {
+    RoundEnd e;
+    std::memset(&e, 0, sizeof(e));
+    e.ctl = R.ctl;
+    e.max_rounds = R.max_rounds;
+    e.launches = R.dev_launches;
+    e.per_round = round_launches(R);
+    return e;
 }
 
 // The batch as one CUDA graph: prologue, a conditional WHILE node whose body
-// is one round plus round_cond_kernel, epilogue.  Built by stream capture
+// is one round (its step kernel sets the loop's condition), epilogue.  Built by stream capture
 // (the round body on the auxiliary stream, into the WHILE node's body graph).
 int build_batch_graph(ndt_ctx *c, const RunPlan &R, cudaGraphExec_t *out) {
     cudaGraph_t g = nullptr;
@@ -597,7 +590,8 @@ int build_batch_graph(ndt_ctx *c, const RunPlan &R, cudaGraphExec_t *out) {
         cudaGraphDestroy(g);
         return cuda_fail(c, e, "cudaStreamBeginCaptureToGraph");
     }
-    if (int rc = enqueue_prologue(c, R, st)) return abort_capture(rc);
+    int nl = 0;
+    if (int rc = enqueue_prologue(c, R, st, &nl)) return abort_capture(rc);
     cudaStreamCaptureStatus cs;
     cudaGraph_t cg = nullptr;
     const cudaGraphNode_t *deps = nullptr;
@@ -620,13 +614,10 @@ int build_batch_graph(ndt_ctx *c, const RunPlan &R, cudaGraphExec_t *out) {
     cudaGraph_t body = np.conditional.phGraph_out[0];
     e = cudaStreamBeginCaptureToGraph(c->aux_stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return abort_capture(cuda_fail(c, e, "cudaStreamBeginCaptureToGraph (body)"));
-    int rc = enqueue_round(c, R, c->aux_stream, false);
-    if (!rc) {
-        round_cond_kernel<<<1, 1, 0, c->aux_stream>>>(h, R.active, R.round_no, R.max_rounds, R.dev_launches,
-                                                       round_launches(R) + 1);
-        e = cudaGetLastError();
-        if (e != cudaSuccess) rc = cuda_fail(c, e, "round_cond_kernel");
-    }
+    RoundEnd end = round_end(R);
+    end.loop = h;
+    end.graph = 1;
+    int rc = enqueue_round(c, R, c->aux_stream, false, end);
     cudaGraph_t body_out = nullptr;
     e = cudaStreamEndCapture(c->aux_stream, &body_out);
     if (rc) return abort_capture(rc);
@@ -688,15 +679,9 @@ int run_batch(ndt_ctx *c, int B, const float4 *d_points, const int *d_offsets, i
     if (int rc0 = prepare_lists(c, B, max_tiles, R.L)) return rc0;
     CK(c->partials.ensure(sizeof(double) * kPartial * (size_t)max_tiles));
     CK(c->exc.ensure(sizeof(double) * kPartial * (size_t)B));
-    CK(c->active.ensure(sizeof(int)));
-    CK(c->counters.ensure(sizeof(Counters)));
     CK(c->h_active.ensure(sizeof(int)));
-    CK(c->round_no.ensure(sizeof(int)));
     cudaStream_t st = c->stream;
-    if (first) {
-        CK(cudaMemsetAsync(c->counters.p, 0, sizeof(Counters), st));
-        c->ev_used = 0;
-    }
+    if (first) c->ev_used = 0;
     R.P = step_params(c->prm);
     EvalArgs &ea = R.ea;
     ea.grid = grid_dev(c);
@@ -714,7 +699,6 @@ int run_batch(ndt_ctx *c, int B, const float4 *d_points, const int *d_offsets, i
     ea.d1 = c->d1;
     ea.d2 = c->d2;
     ea.compat = c->prm.compat;
-    ea.counters = c->counters.as<Counters>();
     if (int rc2 = prepare_scratch(c, ea)) return rc2;
     R.d_offsets = d_offsets;
     R.d_guesses = d_guesses;
@@ -722,8 +706,9 @@ int run_batch(ndt_ctx *c, int B, const float4 *d_points, const int *d_offsets, i
     R.d_conv = d_conv;
     R.d_fit = d_fit;
     R.d_status = d_status;
-    R.active = c->active.as<int>();
-    R.round_no = c->round_no.as<int>();
+    R.ctl = c->ctl.as<RoundCtl>();
+    R.first = first ? 1 : 0;
+    ea.reset = false;  // the prologue and the step kernel clear the pass's counters
     R.dev_launches = c->dev_launches.as<unsigned long long>();
     R.B = B;
     R.tile = tile;
@@ -742,9 +727,9 @@ int run_batch(ndt_ctx *c, int B, const float4 *d_points, const int *d_offsets, i
     if (!R.fixed && R.precision == 0) {
         // alignments finish at different rounds: each FP32 pass hands out only the chunks of active ones
         CK(c->active_chunks.ensure(sizeof(int) * (size_t)max_tiles));
-        CK(c->num_active.ensure(sizeof(int)));
-        ea.active_chunks = c->active_chunks.as<int>();
-        ea.num_active = c->num_active.as<int>();
+        R.L.active_chunks = ea.active_chunks = c->active_chunks.as<int>();
+        R.L.capacity = ea.active_capacity = max_tiles;
+        ea.num_active = R.ctl->num_active;
     }
 
     if (c->use_graphs && !c->profiling) {
@@ -753,18 +738,20 @@ int run_batch(ndt_ctx *c, int B, const float4 *d_points, const int *d_offsets, i
         cudaGraphExec_t exec = nullptr;
         if (int rc = get_batch_graph(c, R, &exec)) return rc;
         CK(cudaGraphLaunch(exec, st));
-        c->launches += 5;  // tiles (3), init, finalize; the rounds count themselves on the device
+        c->launches += 1 + prologue_launches(B);  // (finalize); the rounds count themselves on the device
         return NDT_OK;
     }
     long long nl = 0;
-    if (int rc = enqueue_prologue(c, R, st)) return rc;
-    nl += 4;
+    int np = 0;
+    if (int rc = enqueue_prologue(c, R, st, &np)) return rc;
+    nl += np;
+    const RoundEnd end = round_end(R);
     const int poll_every = 4;
     for (int r = 0; r < R.max_rounds; ++r) {
-        if (int rc = enqueue_round(c, R, st, c->profiling)) return rc;
+        if (int rc = enqueue_round(c, R, st, c->profiling, end)) return rc;
         nl += round_launches(R);
         if (!R.fixed && (r + 1) % poll_every == 0) {
-            CK(cudaMemcpyAsync(c->h_active.p, c->active.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+            CK(cudaMemcpyAsync(c->h_active.p, &R.ctl->active, sizeof(int), cudaMemcpyDeviceToHost, st));
             CK(cudaStreamSynchronize(st));
             if (*c->h_active.as<int>() == 0) break;
         }
@@ -777,7 +764,8 @@ int run_batch(ndt_ctx *c, int B, const float4 *d_points, const int *d_offsets, i
 
 int read_counters(ndt_ctx *c) {
     CK(c->h_counters.ensure(sizeof(Counters)));
-    CK(cudaMemcpyAsync(c->h_counters.p, c->counters.p, sizeof(Counters), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(c->h_counters.p, &c->ctl.as<RoundCtl>()->counters, sizeof(Counters), cudaMemcpyDeviceToHost,
+                       c->stream));
     CK(cudaStreamSynchronize(c->stream));
     const Counters *k = c->h_counters.as<Counters>();
     c->last.rounds = (int64_t)k->rounds;
@@ -1039,11 +1027,10 @@ void ndt_destroy(ndt_ctx *c) {
                       &c->icov64, &c->count, &c->cell, &c->seg_start, &c->seg_cell,
                       &c->scratch, &c->meta, &c->points, &c->offsets, &c->guesses, &c->states,
                       &c->tiles, &c->tile_begin, &c->num_tiles, &c->chunks, &c->chunk_begin, &c->num_chunks,
-                      &c->big_begin, &c->small_begin, &c->num_big, &c->round_no, &c->dev_launches,
+                      &c->big_begin, &c->small_begin, &c->num_big, &c->dev_launches,
                       &c->partials, &c->exc, &c->out_T, &c->out_conv,
-                      &c->out_fit, &c->out_status, &c->active, &c->counters, &c->p6, &c->trans,
-                      &c->flag_q, &c->flag_n, &c->flag_overflow, &c->work_counter, &c->active_chunks,
-                      &c->num_active, &c->lane_sums, &c->split_state};
+                      &c->out_fit, &c->out_status, &c->ctl, &c->p6, &c->trans,
+                      &c->flag_q, &c->active_chunks, &c->lane_sums, &c->split_state};
     for (DevBuf *b : bufs) b->release();
     HostBuf *hb[] = {&c->h_offsets, &c->h_active, &c->h_counters, &c->h_out};
     for (HostBuf *b : hb) b->release();
@@ -1230,10 +1217,7 @@ int ndt_score_batch_device(ndt_ctx *c, int B, const float *d_points, const int *
     if (int rc0 = prepare_lists(c, B, max_tiles, R.L)) return rc0;
     CK(c->partials.ensure(sizeof(double) * kPartial * (size_t)max_tiles));
     CK(c->exc.ensure(sizeof(double) * kPartial * (size_t)B));
-    CK(c->counters.ensure(sizeof(Counters)));
-    CK(c->round_no.ensure(sizeof(int)));
     cudaStream_t st = c->stream;
-    CK(cudaMemsetAsync(c->counters.p, 0, sizeof(Counters), st));
     c->ev_used = 0;
     R.P = step_params(c->prm);
     EvalArgs &ea = R.ea;
@@ -1252,11 +1236,12 @@ int ndt_score_batch_device(ndt_ctx *c, int B, const float *d_points, const int *
     ea.d1 = c->d1;
     ea.d2 = c->d2;
     ea.compat = c->prm.compat;
-    ea.counters = c->counters.as<Counters>();
     if (int rc2 = prepare_scratch(c, ea)) return rc2;
     R.d_offsets = d_offsets;
     R.d_guesses = d_poses;
-    R.round_no = c->round_no.as<int>();
+    R.ctl = c->ctl.as<RoundCtl>();
+    R.first = 1;
+    ea.reset = false;
     R.B = B;
     R.tile = tile;
     R.kb = chunk_big(c);
@@ -1265,12 +1250,13 @@ int ndt_score_batch_device(ndt_ctx *c, int B, const float *d_points, const int *
     R.variant = c->variant;
     R.sms = c->num_sms;
     ea.min_chunks = total_points / (tile * R.kb);
-    if (int rc = enqueue_prologue(c, R, st)) return rc;
+    int np = 0;
+    if (int rc = enqueue_prologue(c, R, st, &np)) return rc;
     int rc = launch_derivatives(R.ea, R.precision, R.variant, R.sms, st);
     if (rc) return cuda_fail(c, (cudaError_t)rc, "launch_derivatives");
     rc = launch_score(R.ea.partials, R.L.chunk_begin, R.ea.exc, B, d_score, st);
     if (rc) return cuda_fail(c, (cudaError_t)rc, "launch_score");
-    c->launches += 4 + (R.precision == 1 ? 1 : kDerivLaunchesFP32) + 1;
+    c->launches += np + derivative_launches(R.ea, R.precision) + 1;
     return NDT_OK;
 }
 
@@ -1426,7 +1412,7 @@ int ndt_kernel_variant_shape(int variant, int *tile, int *blocks_per_sm) {
 
 int ndt_get_counters(ndt_ctx *c, ndt_counters *out) {
     if (!c || !out) return NDT_E_ARG;
-    if (!c->counters.p) {
+    if (!c->ctl.p) {
         std::memset(out, 0, sizeof(*out));
         return NDT_OK;
     }
@@ -1507,7 +1493,7 @@ int ndt_derivatives(ndt_ctx *c, const float *scan, const float *trans, int n, co
     CK(c->partials.ensure(sizeof(double) * kPartial * (size_t)max_tiles));
     CK(c->exc.ensure(sizeof(double) * kPartial));
     CK(c->p6.ensure(sizeof(double) * 6));
-    CK(c->counters.ensure(sizeof(Counters)));
+    CK(c->ctl.ensure(sizeof(RoundCtl)));
     CK(c->h_offsets.ensure(sizeof(int) * 2));
     int *off = c->h_offsets.as<int>();
     off[0] = 0;
@@ -1516,7 +1502,7 @@ int ndt_derivatives(ndt_ctx *c, const float *scan, const float *trans, int n, co
     CK(cudaMemcpyAsync(c->trans.p, trans, sizeof(float4) * (size_t)n, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(c->offsets.p, off, sizeof(int) * 2, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(c->p6.p, p6, sizeof(double) * 6, cudaMemcpyHostToDevice, st));
-    CK(cudaMemsetAsync(c->counters.p, 0, sizeof(Counters), st));
+    CK(cudaMemsetAsync(c->ctl.p, 0, sizeof(RoundCtl), st));
     int rc = launch_tiles(c->offsets.as<int>(), 1, tile, chunk_big(c), chunk_small(c), L, st);
     if (rc) return cuda_fail(c, (cudaError_t)rc, "launch_tiles");
     rc = launch_prepare_eval(c->states.as<AlignState>(), c->p6.as<double>(), n, c->exc.as<double>(), c->prm.compat,
@@ -1538,7 +1524,6 @@ int ndt_derivatives(ndt_ctx *c, const float *scan, const float *trans, int n, co
     ea.d1 = c->d1;
     ea.d2 = c->d2;
     ea.compat = c->prm.compat;
-    ea.counters = c->counters.as<Counters>();
     if (int rc2 = prepare_scratch(c, ea)) return rc2;
     rc = launch_derivatives(ea, c->prm.precision, c->variant, c->num_sms, st);
     if (rc) return cuda_fail(c, (cudaError_t)rc, "launch_derivatives");

@@ -103,6 +103,22 @@ struct Counters {
     unsigned long long rounds;  // lockstep rounds (derivative pass + step) of the batch
 };
 
+// Device-side control of a batch's rounds.  Zero when a batch starts; the last
+// block of each round's step kernel sets what the next pass reads.
+struct RoundCtl {
+    int32_t work_counter;    // next chunk of the current derivative pass
+    uint32_t flag_n;         // side-queue length of the current pass
+    int32_t flag_overflow;   // a pass queued more pairs than the queue holds
+    int32_t active;          // alignments that asked for another evaluation in the last step
+    int32_t num_active[2];   // chunks in the active list: large, small
+    int32_t next_active;     // while a step runs: alignments that asked so far,
+    int32_t ticket;          //   blocks done,
+    unsigned long long next_list;  // large << 32 | small chunks listed so far
+    int32_t round_no;
+    int32_t pad;
+    Counters counters;
+};
+
 struct Tile {
     int32_t align;
     int32_t start;   // first point (global index into the concatenated scans)
@@ -135,6 +151,11 @@ struct TileLists {
     int *big_begin;    // B + 1: scratch (large chunks before each alignment)
     int *small_begin;  // B + 1: scratch (small chunks before each alignment)
     int *num_big;      // total large chunks
+    // optional (corrected-mode FP32 batches): the chunks of the alignments that
+    // ask for an evaluation, large ones from the front, small ones from the
+    // back (see active_chunk in pair_f32.cuh)
+    int *active_chunks = nullptr;
+    int capacity = 0;  // entries of active_chunks
 };
 
 }  // namespace ndt

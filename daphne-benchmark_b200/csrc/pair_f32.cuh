@@ -173,6 +173,18 @@ __device__ __forceinline__ void contract(const PairSums &F, float x0, float x1, 
     }
 }
 
+// Chunks of this pass, and the k-th of them: of the active list (large chunks
+// from its front, small ones from its back, so that the small ones come last),
+// or of all chunks.
+__device__ __forceinline__ int pass_chunks(const EvalArgs &args) {
+    return args.active_chunks ? args.num_active[0] + args.num_active[1] : *args.num_chunks;
+}
+__device__ __forceinline__ int active_chunk(const EvalArgs &args, int k) {
+    if (!args.active_chunks) return k;
+    const int nb = args.num_active[0];
+    return args.active_chunks[k < nb ? k : args.active_capacity - 1 - (k - nb)];
+}
+
 // Queues a pair with a flagged voxel for flagged_kernel (FP64).
 __device__ __forceinline__ void queue_flagged(const EvalArgs &args, int align, int point, int slot) {
     const unsigned q = atomicAdd(args.flag_n, 1u);
