@@ -15,6 +15,7 @@
 
 #include "align.h"
 #include "ndt_math.cuh"
+#include "warp_solve.cuh"
 
 namespace ndt {
 
@@ -24,21 +25,48 @@ constexpr double kMu = 1.e-4;     // sufficient decrease (kernel.cpp:1042)
 constexpr double kNu = 0.9;       // curvature condition (kernel.cpp:1044)
 constexpr int kMaxStepIterations = 10;  // kernel.cpp:1039
 
-__device__ void set_angles(AlignState &s, const double *pose, bool compat) {
-    double a[kAngle];
-    angle_terms(pose, a, compat);
-    for (int k = 0; k < kAngle; ++k) {
-        s.angd[k] = a[k];
-        s.angf[k] = (float)a[k];
+// What one warp needs to step an alignment: the state's copy in shared memory
+// and the cosines and sines of its angles (3) and half angles (3).
+struct StepSmem {
+    AlignState st;
+    double c[6], s[6];
+    double v[kPartial];  // the evaluation's sums
+};
+
+__device__ __forceinline__ int bcast0(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+
+// The cosines and sines of pose p's angles, one angle per lane (the whole
+// warp calls this and the three functions below).
+__device__ __forceinline__ void warp_trig(StepSmem &m, const double *p) {
+    const int lane = threadIdx.x & 31;
+    if (lane < 6) {
+        const double a = p[3 + lane % 3];
+        const double x = lane < 3 ? a : half_angle(a);
+        m.c[lane] = cos(x);
+        m.s[lane] = sin(x);
     }
+    __syncwarp();
 }
 
-__device__ void set_pose(AlignState &s, const StepParams &P) {
-    if (P.compat)
-        build_tm_compat(s.T, s.x_t);
-    else
-        build_tm_corrected(s.T, s.x_t);
-    set_angles(s, s.x_t, P.compat);
+// The angle terms of pose p, after warp_trig.
+__device__ __forceinline__ void warp_angles(StepSmem &m, const double *p, bool compat) {
+    const int lane = threadIdx.x & 31;
+    if (lane == 0) angle_terms(p, m.c, m.s, m.st.angd, compat);
+    __syncwarp();
+    for (int k = lane; k < kAngle; k += 32) m.st.angf[k] = (float)m.st.angd[k];
+}
+
+// The transform and the angle terms of the trial pose.
+__device__ __forceinline__ void warp_set_pose(StepSmem &m, const StepParams &P) {
+    warp_trig(m, m.st.x_t);
+    if ((threadIdx.x & 31) == 1) {  // (beside the angle terms, which lane 0 writes)
+        if (P.compat)
+            build_tm_compat(m.st.T, m.c + 3, m.s + 3);
+        else
+            build_tm_corrected(m.st.T, m.st.x_t, m.c, m.s);
+    }
+    warp_angles(m, m.st.x_t, P.compat != 0);
+    __syncwarp();
 }
 
 __device__ __forceinline__ double dot6(const double *a, const double *b) {
@@ -59,24 +87,24 @@ __device__ bool request(AlignState &s, const StepParams &P, int mode, int phase)
     return true;
 }
 
-// Start of a Newton iteration (kernel.cpp:1214-1245) and of the step-length
-// search up to its first evaluation (:1019-1066).  Returns true when an
-// evaluation was requested; false when the step ended without one (then the
-// caller continues with newton_end) or the alignment finished (phase Done).
-__device__ bool newton_start(AlignState &s, const StepParams &P) {
-    double A[6][6], b[6], dp[6];
-    for (int i = 0; i < 6; ++i) {
-        b[i] = -s.g[i];
-        for (int j = 0; j < 6; ++j) A[i][j] = s.H[6 * i + j];
-    }
-    solve6(dp, A, b);
+// What lane 0 leaves the warp to do next.
+enum StepAct : int {
+    kActNone = 0,    // nothing: an evaluation is requested or the alignment is done
+    kActPose = 1,    // set the trial pose, then request evaluation `mode` in `phase`
+    kActNewton = 2,  // start a Newton iteration
+    kActEnd = 3,     // the step ended without an evaluation: newton_end
+};
+
+// Start of a Newton iteration from its step dp (kernel.cpp:1214-1245) and of
+// the step-length search up to its first evaluation (:1019-1066).
+__device__ int newton_start(AlignState &s, const StepParams &P, const double *dp) {
     double norm = sqrt(dp[0] * dp[0] + dp[1] * dp[1] + dp[2] * dp[2] + dp[3] * dp[3] + dp[4] * dp[4] + dp[5] * dp[5]);
     if (P.compat) norm = 1;  // kernel.cpp:1231
     if (norm == 0 || norm != norm) {
         s.converged = norm == norm;
         s.phase = kPhaseDone;
         s.eval_mode = kEvalNone;
-        return false;
+        return kActNone;
     }
     for (int i = 0; i < 6; ++i) s.dir[i] = dp[i] / norm;
     // computeStepLengthMT(p, dir, step_init = norm, step_max, step_min)
@@ -85,7 +113,7 @@ __device__ bool newton_start(AlignState &s, const StepParams &P) {
     if (s.d_phi_0 >= 0) {
         if (s.d_phi_0 == 0) {
             s.a_t = 0;  // not a descent direction: step 0, no evaluation
-            return false;
+            return kActEnd;
         }
         s.d_phi_0 *= -1;
         for (int i = 0; i < 6; ++i) s.dir[i] *= -1;
@@ -106,8 +134,7 @@ __device__ bool newton_start(AlignState &s, const StepParams &P) {
     a_t = std_max(a_t, s.step_min);
     s.a_t = a_t;
     for (int i = 0; i < 6; ++i) s.x_t[i] = s.p[i] + s.dir[i] * a_t;
-    set_pose(s, P);
-    return request(s, P, kEvalFull, kPhaseMTFirst);
+    return kActPose;
 }
 
 // Pose update and convergence test after a step (kernel.cpp:1246-1266).
@@ -127,8 +154,8 @@ __device__ bool newton_end(AlignState &s, const StepParams &P) {
 }
 
 // Loop test of the line search (kernel.cpp:1076) and its next trial point
-// (:1078-1099).  Returns true when an evaluation was requested.
-__device__ bool mt_continue(AlignState &s, const StepParams &P) {
+// (:1078-1099).
+__device__ int mt_continue(AlignState &s, const StepParams &P) {
     if (!s.interval_converged && s.step_iterations < kMaxStepIterations &&
         !(s.psi_t <= 0 && s.d_phi_t <= -kNu * s.d_phi_0)) {
         double a_t;
@@ -140,17 +167,19 @@ __device__ bool mt_continue(AlignState &s, const StepParams &P) {
         a_t = std_max(a_t, s.step_min);
         s.a_t = a_t;
         for (int i = 0; i < 6; ++i) s.x_t[i] = s.p[i] + s.dir[i] * a_t;
-        set_pose(s, P);
-        return request(s, P, kEvalGradient, kPhaseMTIter);
+        return kActPose;
     }
-    if (s.step_iterations) return request(s, P, kEvalHessian, kPhaseMTHess);  // computeHessian (:1141-1142)
-    return false;
+    if (s.step_iterations) {  // computeHessian (:1141-1142)
+        request(s, P, kEvalHessian, kPhaseMTHess);
+        return kActNone;
+    }
+    return kActEnd;
 }
 
-// Consume the evaluation result held in s.score/g/H and advance until the
-// next evaluation is requested or the alignment is done.
-__device__ void advance(AlignState &s, const StepParams &P) {
-    int phase = s.phase;
+// Consumes the evaluation result held in s.score/g/H (lane 0) up to the next
+// thing the warp does.
+__device__ int consume(AlignState &s, const StepParams &P) {
+    const int phase = s.phase;
     if (phase == kPhaseMTFirst || phase == kPhaseMTIter) {
         s.phi_t = -s.score;
         s.d_phi_t = -(dot6(s.g, s.dir));
@@ -172,33 +201,70 @@ __device__ void advance(AlignState &s, const StepParams &P) {
             s.interval_converged = ic;
             s.step_iterations++;
         }
-        if (mt_continue(s, P)) return;
-        if (s.phase == kPhaseDone) return;
-        if (newton_end(s, P)) return;
-    } else if (phase == kPhaseMTHess) {
-        if (newton_end(s, P)) return;
-    } else if (phase != kPhaseInitEval) {
-        return;
+        return mt_continue(s, P);
     }
-    // bounded: each pass either requests an evaluation, finishes, or
-    // completes a Newton iteration without one (d_phi_0 == 0)
-    for (int guard = 0; guard < 1024; ++guard) {
-        if (newton_start(s, P)) return;
-        if (s.phase == kPhaseDone) return;
-        if (newton_end(s, P)) return;
-    }
-    s.status = NDT_ST_WATCHDOG_DEV;
-    s.converged = 0;
-    s.phase = kPhaseDone;
-    s.eval_mode = kEvalNone;
+    if (phase == kPhaseMTHess) return kActEnd;
+    return phase == kPhaseInitEval ? kActNewton : kActNone;
 }
 
-// One warp per alignment; lane 0 works on a shared-memory copy of the
-// alignment's state (the state machine is serial FP64 code that touches
-// hundreds of fields), and the warp moves the state between global and
-// shared memory in 16-byte pieces.
+// Advances the alignment until the next evaluation is requested or it is
+// done.  Lane 0 runs the state machine; the parts that are long serial chains
+// of FP64 operations (the 6x6 solve, the trigonometry) are the warp's: the
+// step is bound by the latency of these chains (7.6 -> 5.2 us for one
+// alignment, 16.1 -> 10.4 us on average over the rounds of 1024, against all
+// of it on lane 0).
+__device__ void advance(StepSmem &m, const StepParams &P) {
+    const int lane = threadIdx.x & 31;
+    AlignState &s = m.st;
+    int act = kActNone, first = 0;
+    if (lane == 0) {
+        act = consume(s, P);
+        first = act == kActPose;  // the line search goes on: its gradient at the trial point
+    }
+    act = bcast0(act);
+    first = bcast0(first);
+    // bounded: each pass either requests an evaluation, finishes, or
+    // completes a Newton iteration without one (d_phi_0 == 0)
+    for (int guard = 0; guard <= 1024; ++guard) {
+        if (act == kActEnd) {
+            if (lane == 0) act = newton_end(s, P) ? kActNone : kActNewton;
+            act = bcast0(act);
+        }
+        if (act == kActNewton) {
+            if (guard == 1024) break;
+            __syncwarp();
+            double dp[6];
+            warp_solve6(s.H, s.g, dp);
+            if (lane == 0) act = newton_start(s, P, dp);
+            act = bcast0(act);
+        }
+        if (act == kActPose) {
+            __syncwarp();
+            warp_set_pose(m, P);
+            if (lane == 0) {
+                if (first)
+                    request(s, P, kEvalGradient, kPhaseMTIter);
+                else
+                    request(s, P, kEvalFull, kPhaseMTFirst);
+            }
+            return;
+        }
+        if (act == kActNone) return;
+    }
+    if (lane == 0) {
+        s.status = NDT_ST_WATCHDOG_DEV;
+        s.converged = 0;
+        s.phase = kPhaseDone;
+        s.eval_mode = kEvalNone;
+    }
+}
+
+// One warp per alignment, on a shared-memory copy of the alignment's state
+// (the state machine is serial FP64 code that touches hundreds of fields),
+// which the warp moves between global and shared memory in 16-byte pieces.
 constexpr int kStateWarps = 4;
 constexpr int kStateVecs = (int)(sizeof(AlignState) / sizeof(uint4));
+constexpr int kStatePieces = (kStateVecs + 31) / 32;  // per lane
 static_assert(sizeof(AlignState) % sizeof(uint4) == 0, "AlignState is copied in 16-byte pieces");
 
 __device__ __forceinline__ void copy_state(AlignState *dst, const AlignState *src, int lane) {
@@ -207,38 +273,45 @@ __device__ __forceinline__ void copy_state(AlignState *dst, const AlignState *sr
     for (int i = lane; i < kStateVecs; i += 32) d[i] = s[i];
 }
 
-// The state of an alignment before its first evaluation (one thread).
-__device__ void init_state(AlignState &s, const float *__restrict__ guess, int n, const StepParams &P) {
-    for (int k = 0; k < 16; ++k) s.T[k] = guess[k];
-    pose_vector(P.compat != 0, s.T, s.p);
-    if (!P.compat) build_tm_corrected(s.T, s.p);
-    for (int i = 0; i < 6; ++i) {
-        s.x_t[i] = s.p[i];
-        s.dir[i] = 0.0;
-        s.g[i] = 0.0;
+// The state of an alignment before its first evaluation (the whole warp).
+__device__ void init_state(StepSmem &m, const float *__restrict__ guess, int n, const StepParams &P) {
+    const int lane = threadIdx.x & 31;
+    AlignState &s = m.st;
+    if (lane < 16) s.T[lane] = guess[lane];
+    for (int k = lane; k < 36; k += 32) s.H[k] = 0.0;
+    __syncwarp();
+    if (lane == 0) {
+        pose_vector(P.compat != 0, s.T, s.p);
+        for (int i = 0; i < 6; ++i) {
+            s.x_t[i] = s.p[i];
+            s.dir[i] = 0.0;
+            s.g[i] = 0.0;
+        }
+        s.score = 0.0;
+        s.phi_0 = s.d_phi_0 = s.a_l = s.f_l = s.g_l = s.a_u = s.f_u = s.g_u = s.a_t = 0.0;
+        s.phi_t = s.d_phi_t = s.psi_t = s.d_psi_t = 0.0;
+        s.step_max = P.step_max;
+        s.step_min = P.step_min;
+        s.nr_iterations = 0;
+        s.step_iterations = 0;
+        s.open_interval = 1;
+        s.interval_converged = 0;
+        s.converged = 0;
+        s.evals = 0;
+        s.status = 0;
+        s.n = n;
+        s.eval_mode = kEvalFull;
+        s.phase = kPhaseInitEval;
     }
-    for (int k = 0; k < 36; ++k) s.H[k] = 0.0;
-    s.score = 0.0;
-    s.phi_0 = s.d_phi_0 = s.a_l = s.f_l = s.g_l = s.a_u = s.f_u = s.g_u = s.a_t = 0.0;
-    s.phi_t = s.d_phi_t = s.psi_t = s.d_psi_t = 0.0;
-    s.step_max = P.step_max;
-    s.step_min = P.step_min;
-    s.nr_iterations = 0;
-    s.step_iterations = 0;
-    s.open_interval = 1;
-    s.interval_converged = 0;
-    s.converged = 0;
-    s.evals = 0;
-    s.status = 0;
-    s.n = n;
-    set_angles(s, s.p, P.compat);
-    s.eval_mode = kEvalFull;
-    s.phase = kPhaseInitEval;
+    __syncwarp();
+    warp_trig(m, s.p);
+    if (!P.compat && lane == 1) build_tm_corrected(s.T, s.p, m.c, m.s);
+    warp_angles(m, s.p, P.compat != 0);
 }
 
 // FP64 sum of the alignment's chunk partials in chunk order (deterministic;
-// each lane sums the values k = lane, lane + 32 with its loads issued 8 at a
-// time), then lane 0 advances the state machine; the chunks of an alignment
+// lane l sums the values l and l + 32, the loads of 8 chunks in flight, the
+// state's copy beside them), then the warp advances the state machine; the chunks of an alignment
 // that asks for another evaluation go to the active list (their order in it
 // changes no result, since each chunk writes its own partial slot).  The last
 // block to finish ends the round: the counters that separate launches would
@@ -246,50 +319,64 @@ __device__ void init_state(AlignState &s, const float *__restrict__ guess, int n
 // condition: 10 us of a 21 us round tail) are set here.
 __global__ void step_kernel(AlignState *__restrict__ states, const double *__restrict__ partials, TileLists L,
                             double *__restrict__ exc, int B, StepParams P, RoundEnd end) {
-    __shared__ double s_v[kStateWarps][kPartial];
-    __shared__ AlignState s_st[kStateWarps];
+    __shared__ StepSmem s_m[kStateWarps];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     RoundCtl *ctl = end.ctl;
     const int b = blockIdx.x * kStateWarps + warp;
     AlignState *st = states + b;
     const int mode = b < B ? st->eval_mode : kEvalNone;
     if (mode != kEvalNone) {
+        StepSmem &m = s_m[warp];
+        AlignState &s = m.st;
         const int c0 = L.chunk_begin[b], c1 = L.chunk_begin[b + 1];
-        for (int k = lane; k < kPartial; k += 32) {
-            double v = 0.0;
-            int c = c0;
-            for (; c + 8 <= c1; c += 8) {
-                double t[8];
+        uint4 piece[kStatePieces];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) t[u] = partials[(size_t)(c + u) * kPartial + k];
+        for (int q = 0; q < kStatePieces; ++q)
+            if (lane + 32 * q < kStateVecs) piece[q] = reinterpret_cast<const uint4 *>(st)[lane + 32 * q];
+        const bool two = lane + 32 < kPartial;
+        double *e = exc + (size_t)b * kPartial + lane;
+        const double e0 = e[0], e1 = two ? e[32] : 0.0;
+        double v0 = 0.0, v1 = 0.0;
+        for (int c = c0; c < c1; c += 8) {
+            double t0[8], t1[8];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) v += t[u];
+            for (int u = 0; u < 8; ++u) {
+                const double *p = partials + (size_t)(c + u) * kPartial + lane;
+                t0[u] = c + u < c1 ? p[0] : 0.0;
+                t1[u] = two && c + u < c1 ? p[32] : 0.0;
             }
-            for (; c < c1; ++c) v += partials[(size_t)c * kPartial + k];
-            double *e = exc + (size_t)b * kPartial + k;
-            v += *e;
-            *e = 0.0;
-            s_v[warp][k] = v;
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (c + u < c1) {
+                    v0 += t0[u];
+                    v1 += t1[u];
+                }
         }
-        AlignState &s = s_st[warp];
-        copy_state(&s, st, lane);
+        m.v[lane] = v0 + e0;
+        e[0] = 0.0;
+        if (two) {
+            m.v[lane + 32] = v1 + e1;
+            e[32] = 0.0;
+        }
+#pragma unroll
+        for (int q = 0; q < kStatePieces; ++q)
+            if (lane + 32 * q < kStateVecs) reinterpret_cast<uint4 *>(&s)[lane + 32 * q] = piece[q];
         __syncwarp();
+        // the evaluation's result (computeDerivatives without a Hessian zeroes it, kernel.cpp:667)
+        const bool grad = mode == kEvalFull || mode == kEvalGradient;
+        const bool hess = mode == kEvalFull || mode == kEvalHessian;
+        if (grad && lane < 6) s.g[lane] = m.v[1 + lane];
+        for (int k = lane; k < 36; k += 32) s.H[k] = hess ? m.v[7 + k] : 0.0;
+        if (lane == 0) {
+            if (grad) s.score = m.v[0];
+            s.evals++;
+            s.eval_mode = kEvalNone;
+        }
+        __syncwarp();
+        advance(m, P);
         unsigned long long at = 0;
         int nb = 0, ns = 0, b0 = 0, s0 = 0;
         if (lane == 0) {
-            const double *v = s_v[warp];
-            if (mode == kEvalFull || mode == kEvalGradient) {
-                s.score = v[0];
-                for (int i = 0; i < 6; ++i) s.g[i] = v[1 + i];
-            }
-            if (mode == kEvalFull || mode == kEvalHessian) {
-                for (int k = 0; k < 36; ++k) s.H[k] = v[7 + k];
-            } else {
-                for (int k = 0; k < 36; ++k) s.H[k] = 0.0;  // computeDerivatives zeroes it (kernel.cpp:667)
-            }
-            s.evals++;
-            s.eval_mode = kEvalNone;
-            advance(s, P);
             if (s.eval_mode != kEvalNone) {
                 atomicAdd(&ctl->next_active, 1);
                 if (L.active_chunks) {
@@ -480,7 +567,7 @@ __global__ void tile_fill_kernel(const int *__restrict__ offsets, int B, int til
 __global__ void fill_init_kernel(const int *__restrict__ offsets, int B, int tile, int kb, int ks, TileLists L,
                                  AlignState *__restrict__ states, const float *__restrict__ guesses, StepParams P,
                                  double *__restrict__ exc, RoundCtl *__restrict__ ctl) {
-    __shared__ AlignState s_st[kStateWarps];
+    __shared__ StepSmem s_m[kStateWarps];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int b = blockIdx.x * kStateWarps + warp;
     if (b >= B) return;
@@ -489,11 +576,10 @@ __global__ void fill_init_kernel(const int *__restrict__ offsets, int B, int til
         ctl->num_active[1] = L.small_begin[B];
     }
     for (int k = lane; k < kPartial; k += 32) exc[(size_t)b * kPartial + k] = 0.0;
-    AlignState &s = s_st[warp];
-    if (lane == 0) init_state(s, guesses + 16 * (size_t)b, offsets[b + 1] - offsets[b], P);
+    init_state(s_m[warp], guesses + 16 * (size_t)b, offsets[b + 1] - offsets[b], P);
     fill_lists(offsets, b, B, tile, kb, ks, L);
     __syncwarp();
-    copy_state(states + b, &s, lane);
+    copy_state(states + b, &s_m[warp].st, lane);
 }
 
 // Tile and chunk counts per alignment and their exclusive scans by one block

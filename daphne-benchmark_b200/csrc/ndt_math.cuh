@@ -26,11 +26,12 @@ __device__ __forceinline__ double std_max(double a, double b) { return (a < b) ?
 // d^2/db^2 (cy cz, -cy sz, sy) = (-cy cz, cy sz, -sy), has +sy in the
 // reference's h_ang_d1 (kernel.cpp:795-797); compat keeps it, the corrected
 // mode uses -sy.
-__device__ inline void angle_terms(const double *p, double *o, bool compat) {
+// c[3], s[3]: the cosines and sines of the three angles p[3..5].
+__device__ inline void angle_terms(const double *p, const double *c, const double *s, double *o, bool compat) {
     double cx, cy, cz, sx, sy, sz;
-    if (fabs(p[3]) < 10e-5) { cx = 1.0; sx = 0.0; } else { cx = cos(p[3]); sx = sin(p[3]); }
-    if (fabs(p[4]) < 10e-5) { cy = 1.0; sy = 0.0; } else { cy = cos(p[4]); sy = sin(p[4]); }
-    if (fabs(p[5]) < 10e-5) { cz = 1.0; sz = 0.0; } else { cz = cos(p[5]); sz = sin(p[5]); }
+    if (fabs(p[3]) < 10e-5) { cx = 1.0; sx = 0.0; } else { cx = c[0]; sx = s[0]; }
+    if (fabs(p[4]) < 10e-5) { cy = 1.0; sy = 0.0; } else { cy = c[1]; sy = s[1]; }
+    if (fabs(p[5]) < 10e-5) { cz = 1.0; sz = 0.0; } else { cz = c[2]; sz = s[2]; }
     // j_ang a .. h
     o[0] = (-sx * sz + cx * sy * cz);  o[1] = (-sx * cz - cx * sy * sz);  o[2] = (-cx * cy);
     o[3] = (cx * sz + sx * sy * cz);   o[4] = (cx * cz - sx * sy * sz);   o[5] = (-sx * cy);
@@ -59,23 +60,29 @@ __device__ inline void angle_terms(const double *p, double *o, bool compat) {
     h[42] = (-sx * sz + cx * sy * cz); h[43] = (-cx * sy * sz - sx * cz); h[44] = 0;
 }
 
+__device__ inline void angle_terms(const double *p, double *o, bool compat) {
+    const double c[3] = {cos(p[3]), cos(p[4]), cos(p[5])}, s[3] = {sin(p[3]), sin(p[4]), sin(p[5])};
+    angle_terms(p, c, s, o, compat);
+}
+
+// Half of an angle as the reference's pose build takes it, in float.
+__device__ inline double half_angle(double a) { return (double)(float)(0.5f * a); }
+
 // Reference pose build (buildTransformationMatrix, kernel.cpp:949-1013):
 // float quaternion products with permuted components; writes the rotation
-// block and row 3 only, the translation column keeps its value.
-__device__ inline void build_tm_compat(float *M, const double *t) {
-    const float q_ha = 0.5f * t[3];
-    const float q_w = cos((double)q_ha);
-    const float q_x = sin((double)q_ha);
+// block and row 3 only, the translation column keeps its value.  hc[3], hs[3]:
+// the cosines and sines of the three half angles.
+__device__ inline void build_tm_compat(float *M, const double *hc, const double *hs) {
+    const float q_w = hc[0];
+    const float q_x = hs[0];
     const float q_y = 0.0f, q_z = 0.0f;
-    const float q_ha2 = 0.5f * t[4];
-    const float q_w2 = cos((double)q_ha2);
+    const float q_w2 = hc[1];
     const float q_x2 = 0.0f;
-    const float q_y2 = sin((double)q_ha2);
+    const float q_y2 = hs[1];
     const float q_z2 = 0.0f;
-    const float q_ha3 = 0.5f * t[5];
-    const float q_w3 = cos((double)q_ha3);
+    const float q_w3 = hc[2];
     const float q_x3 = 0.0f, q_y3 = 0.0f;
-    const float q_z3 = sin((double)q_ha3);
+    const float q_z3 = hs[2];
     const float r_x = q_w * q_w2 - q_x * q_x2 - q_y * q_y2 - q_z * q_z2;
     const float r_y = q_w * q_x2 + q_x * q_w2 + q_y * q_z2 - q_z * q_y2;
     const float r_z = q_w * q_y2 + q_y * q_w2 + q_z * q_x2 - q_x * q_z2;
@@ -100,26 +107,43 @@ __device__ inline void build_tm_compat(float *M, const double *t) {
     M[10] = 1.0f - (txx + tyy);
 }
 
+__device__ inline void build_tm_compat(float *M, const double *t) {
+    double hc[3], hs[3];
+    for (int k = 0; k < 3; ++k) {
+        hc[k] = cos(half_angle(t[3 + k]));
+        hs[k] = sin(half_angle(t[3 + k]));
+    }
+    build_tm_compat(M, hc, hs);
+}
+
 // Rotation R = Rx(a) Ry(b) Rz(c) (the parametrisation eq. 6.19 / 6.21
-// differentiate), row major.
-__device__ inline void rot_xyz(const double *p, double *R) {
-    double ca = cos(p[3]), sa = sin(p[3]);
-    double cb = cos(p[4]), sb = sin(p[4]);
-    double cc = cos(p[5]), sc = sin(p[5]);
+// differentiate), row major, from the angles' cosines and sines.
+__device__ inline void rot_xyz(const double *c, const double *s, double *R) {
+    const double ca = c[0], sa = s[0], cb = c[1], sb = s[1], cc = c[2], sc = s[2];
     R[0] = cb * cc;                R[1] = -cb * sc;               R[2] = sb;
     R[3] = ca * sc + sa * sb * cc; R[4] = ca * cc - sa * sb * sc; R[5] = -sa * cb;
     R[6] = sa * sc - ca * sb * cc; R[7] = sa * cc + ca * sb * sc; R[8] = ca * cb;
 }
 
+__device__ inline void rot_xyz(const double *p, double *R) {
+    const double c[3] = {cos(p[3]), cos(p[4]), cos(p[5])}, s[3] = {sin(p[3]), sin(p[4]), sin(p[5])};
+    rot_xyz(c, s, R);
+}
+
 // Corrected pose build: T = Trans(p0..2) * Rx * Ry * Rz, FP64 then rounded.
-__device__ inline void build_tm_corrected(float *M, const double *p) {
+__device__ inline void build_tm_corrected(float *M, const double *p, const double *c, const double *s) {
     double R[9];
-    rot_xyz(p, R);
+    rot_xyz(c, s, R);
     for (int r = 0; r < 3; ++r) {
         for (int c = 0; c < 3; ++c) M[4 * r + c] = (float)R[3 * r + c];
         M[4 * r + 3] = (float)p[r];
     }
     M[12] = 0.0f; M[13] = 0.0f; M[14] = 0.0f; M[15] = 1.0f;
+}
+
+__device__ inline void build_tm_corrected(float *M, const double *p) {
+    const double c[3] = {cos(p[3]), cos(p[4]), cos(p[5])}, s[3] = {sin(p[3]), sin(p[4]), sin(p[5])};
+    build_tm_corrected(M, p, c, s);
 }
 
 // Pose vector of a 4x4: translation column + angles.  compat: the reference's
