@@ -300,7 +300,7 @@ __device__ void init_state(StepSmem &m, const float *__restrict__ guess, int n, 
         s.evals = 0;
         s.status = 0;
         s.n = n;
-        s.eval_mode = kEvalFull;
+        s.eval_mode = P.first_mode;
         s.phase = kPhaseInitEval;
     }
     __syncwarp();
@@ -451,6 +451,9 @@ __device__ __forceinline__ void chunk_plan(int t, int kb, int ks, int &nb, int &
     ns = (rest + ks - 1) / ks;
 }
 
+// The scan that alignment b reads (TileLists::scans).
+__device__ __forceinline__ int scan_of(const TileLists &L, int b) { return L.scans > 0 ? b % L.scans : b; }
+
 // Tile list: ceil(n_b / tile) tiles per alignment, in alignment order; the
 // large and small chunk counts per alignment.
 __global__ void tile_count_kernel(const int *__restrict__ offsets, int B, int tile, int kb, int ks, TileLists L) {
@@ -462,7 +465,8 @@ __global__ void tile_count_kernel(const int *__restrict__ offsets, int B, int ti
         L.small_begin[B] = 0;
         return;
     }
-    const int n = offsets[b + 1] - offsets[b];
+    const int sb = scan_of(L, b);
+    const int n = offsets[sb + 1] - offsets[sb];
     const int t = n > 0 ? (n + tile - 1) / tile : 0;
     int nb, ns;
     chunk_plan(t, kb, ks, nb, ns);
@@ -520,7 +524,8 @@ __global__ void scan3_kernel(ScanArgs a, int n) {
 __device__ __forceinline__ void fill_lists(const int *__restrict__ offsets, int b, int B, int tile, int kb, int ks,
                                            const TileLists &L) {
     const int lane = threadIdx.x & 31;
-    const int lo = offsets[b], hi = offsets[b + 1];
+    const int sb = scan_of(L, b);
+    const int lo = offsets[sb], hi = offsets[sb + 1];
     const int t0 = L.tile_begin[b], t1 = L.tile_begin[b + 1];
     for (int t = t0 + lane; t < t1; t += 32) {
         Tile x;
@@ -576,7 +581,8 @@ __global__ void fill_init_kernel(const int *__restrict__ offsets, int B, int til
         ctl->num_active[1] = L.small_begin[B];
     }
     for (int k = lane; k < kPartial; k += 32) exc[(size_t)b * kPartial + k] = 0.0;
-    init_state(s_m[warp], guesses + 16 * (size_t)b, offsets[b + 1] - offsets[b], P);
+    const int sb = scan_of(L, b);
+    init_state(s_m[warp], guesses + 16 * (size_t)b, offsets[sb + 1] - offsets[sb], P);
     fill_lists(offsets, b, B, tile, kb, ks, L);
     __syncwarp();
     copy_state(states + b, &s_m[warp].st, lane);
@@ -602,7 +608,8 @@ __global__ void __launch_bounds__(1024) lists_kernel(const int *__restrict__ off
     const int lo = min(B, t * per), hi = min(B, lo + per);
     int sum[3] = {0, 0, 0};
     for (int b = lo; b < hi; ++b) {
-        const int n = offsets[b + 1] - offsets[b];
+        const int sb = scan_of(L, b);
+        const int n = offsets[sb + 1] - offsets[sb];
         const int tiles = n > 0 ? (n + tile - 1) / tile : 0;
         int nb, ns;
         chunk_plan(tiles, kb, ks, nb, ns);
@@ -638,7 +645,8 @@ __global__ void __launch_bounds__(1024) lists_kernel(const int *__restrict__ off
         L.tile_begin[b] = run[0];
         L.big_begin[b] = run[1];
         L.small_begin[b] = run[2];
-        const int n = offsets[b + 1] - offsets[b];
+        const int sb = scan_of(L, b);
+        const int n = offsets[sb + 1] - offsets[sb];
         const int tiles = n > 0 ? (n + tile - 1) / tile : 0;
         int nb, ns;
         chunk_plan(tiles, kb, ks, nb, ns);

@@ -16,6 +16,7 @@ struct StepParams {
     double step_max;   // step_size
     double step_min;   // eps / 2
     int watchdog_evals;
+    int first_mode;    // the first evaluation (kEvalFull; kEvalScore for a score pass)
 };
 
 // Tiles of `tile` points and chunks (large: kb tiles, small: ks tiles) for

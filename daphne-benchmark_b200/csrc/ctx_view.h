@@ -23,6 +23,11 @@ struct CtxEvalView {
 
 // Fills *v from the context; returns 0, or NDT_E_ARG for a null argument.
 int ctx_eval_view(ndt_ctx *c, CtxEvalView *v);
+// NDT scores of B poses on the context's stream (arguments checked by the
+// caller): pose b is scored with scan b % scans of the packed d_points /
+// d_offsets (scans + 1 entries), total_points >= the scans' points.
+int ctx_score_batch(ndt_ctx *c, int B, int scans, const float *d_points, const int *d_offsets, int total_points,
+                    const float *d_poses, double *d_score);
 // Records an error message on the context (ndt_last_error).
 void ctx_set_error(ndt_ctx *c, const char *msg);
 

@@ -105,7 +105,7 @@ __global__ void flagged_kernel(const __grid_constant__ EvalArgs args) {
         const int4 e = args.flag_q[q];
         const AlignState &st = args.states[e.x];
         const int mode = st.eval_mode;
-        const bool hess = mode != kEvalGradient;
+        const bool hess = eval_level(mode) == kLevelHessian;
         const float4 x = args.points[e.y];
         float px, py, pz;
         if (args.trans) {
@@ -152,10 +152,10 @@ struct F32Smem {
 // shuffle tree, also in FP64 (B200 issues FP64 adds at half the FP32 rate, and
 // the sums of FP32 values stay exact or nearly so).  Fixed order, so the
 // result does not depend on timing.  A chunk in which no warp found a pair
-// writes its zeros directly.
+// writes its zeros directly.  Only the first `values` are summed up.
 template <int W>
 __device__ void reduce_run(F32Smem<W> &sm, double *s_tot, const unsigned *s_pairs, double *out, double kR,
-                           bool compat) {
+                           bool compat, int values) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     __syncthreads();
     unsigned np = 0;
@@ -168,7 +168,7 @@ __device__ void reduce_run(F32Smem<W> &sm, double *s_tot, const unsigned *s_pair
     // (not unrolled: the unrolled loop adds ~11 KB of code to a kernel whose hot
     // loop is already larger than the instruction cache)
 #pragma unroll 1
-    for (int k = warp; k < kAcc; k += W) {
+    for (int k = warp; k < values; k += W) {
         double sum = 0.0;
 #pragma unroll
         for (int r = 0; r < W; ++r) {
@@ -183,13 +183,14 @@ __device__ void reduce_run(F32Smem<W> &sm, double *s_tot, const unsigned *s_pair
     __syncthreads();
     if (threadIdx.x < kPartial) {
         const int k = threadIdx.x;
-        double v;
-        if (k < 7)
-            v = s_tot[k];
-        else if (k < 43)
-            v = h_entry(s_tot, (k - 7) / 6, (k - 7) % 6, kR, compat);
-        else
+        double v = 0.0;
+        if (k < 7) {
+            if (k < values) v = s_tot[k];
+        } else if (k == 43) {
             v = (double)np;
+        } else if (values == kAcc) {
+            v = h_entry(s_tot, (k - 7) / 6, (k - 7) % 6, kR, compat);
+        }
         out[k] = v;
     }
 }
@@ -204,7 +205,7 @@ struct WarpPairs {
     int stride;
     int align;
     float d1, d2;
-    bool hess;
+    int level;
 };
 
 // The evaluation steps after one collect call of a warp: first the dense
@@ -263,11 +264,11 @@ __device__ __forceinline__ void eval_steps(const WarpPairs &P, const unsigned (*
                 if (code & 32u)
                     queue_flagged(*P.args, P.align, pi, slot);
                 else
-                    add_pair(*P.grid, F, slot, ex, ey, ez, P.d1, P.d2, P.hess);
+                    add_pair(*P.grid, F, slot, ex, ey, ez, P.d1, P.d2, P.level);
             }
         }
         if (cnt > 0 && !(from_ring && (rcode & 32u)))
-            contract<true>(F, xe.x, xe.y, xe.z, P.ang, P.acc, P.stride, P.d2, P.hess, COMPAT);
+            contract<true>(F, xe.x, xe.y, xe.z, P.ang, P.acc, P.stride, P.d2, P.level, COMPAT);
     }
 }
 
@@ -338,7 +339,7 @@ __global__ void __launch_bounds__(TILE, MINB) derivative_f32_kernel(const __grid
         const int mode = s_mode;
         if (mode == kEvalNone) continue;  // s_mode is rewritten only after the next chunk's barrier
         P.align = ck.align;
-        P.hess = mode != kEvalGradient;
+        P.level = eval_level(mode);
         for (int ti = ck.first; ti < ck.end; ++ti) {
             const Tile tile = args.tiles[ti];
             const int i = tile.start + threadIdx.x;
@@ -402,7 +403,8 @@ __global__ void __launch_bounds__(TILE, MINB) derivative_f32_kernel(const __grid
         }
         // end of the chunk (the last collect call emptied the ring): the block's sums
         head = tail = 0;
-        reduce_run<kW>(sm, s_tot, s_pairs, args.partials + (size_t)ck.slot * kPartial, compat ? -args.d2 : 1.0, compat);
+        reduce_run<kW>(sm, s_tot, s_pairs, args.partials + (size_t)ck.slot * kPartial, compat ? -args.d2 : 1.0, compat,
+                       level_values(P.level));
         __syncthreads();
         if (lane == 0) s_pairs[warp] = 0;
     }

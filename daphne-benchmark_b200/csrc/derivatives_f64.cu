@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(kTile64, 1) derivative_f64_kernel(const __grid
         __syncthreads();
         const int mode = s_mode;
         if (mode == kEvalNone) continue;
-        const bool hess = mode != kEvalGradient;
+        const bool hess = eval_level(mode) == kLevelHessian;
         const int i = tile.start + threadIdx.x;
         const bool valid = i < tile.end;
         const float4 x = valid ? args.points[i] : make_float4(0.f, 0.f, 0.f, 0.f);

@@ -126,8 +126,8 @@ __global__ void __launch_bounds__(kBlock, kWideResident) derivative_wide_kernel(
         __syncthreads();
         const int mode = s_mode;
         if (mode == kEvalNone) continue;  // s_mode is rewritten only after the next item's barrier
-        const bool hess = mode != kEvalGradient;
-        const int values = hess ? kAcc : 7;
+        const int level = eval_level(mode);
+        const int values = level_values(level);
         const int ntiles = ck.end - ck.first;
 
         // Groups of up to kStepWarps tiles, one warp each.  `serial`: a tile's
@@ -282,22 +282,21 @@ __global__ void __launch_bounds__(kBlock, kWideResident) derivative_wide_kernel(
                         if (code & 32u)
                             queue_flagged(args, ck.align, i, slot);
                         else
-                            add_pair(grid, F, slot, px, py, pz, d1, d2, hess);
+                            add_pair(grid, F, slot, px, py, pz, d1, d2, level);
                     }
                 }
                 if (cnt > 0 && !(from_ring && (rcode & 32u)))
-                    contract<false>(F, x.x, x.y, x.z, s_ang, contrib, 32, d2, hess, COMPAT);
+                    contract<false>(F, x.x, x.y, x.z, s_ang, contrib, 32, d2, level, COMPAT);
                 else
                     for (int k = 0; k < values; ++k) contrib[32 * k] = 0.0f;
             }
             __syncthreads();  // every step's contributions are in place
 #pragma unroll 1
-            for (int k = warp; k < kAcc; k += kStepWarps) {
+            for (int k = warp; k < values; k += kStepWarps) {
                 if (!COMPAT && (k == 31 || k == 34 || k == 35)) continue;  // (lower triangle of R: not used)
                 float v = fresh ? 0.0f : sm.carry[k][lane];
-                if (k < values)
-                    for (int q = 0; q < steps; ++q)
-                        v += __uint_as_float(sm.step[(order >> (4 * q)) & 15u][32 * k + lane]);
+                for (int q = 0; q < steps; ++q)
+                    v += __uint_as_float(sm.step[(order >> (4 * q)) & 15u][32 * k + lane]);
                 if (!done)
                     sm.carry[k][lane] = v;
                 else
@@ -344,7 +343,7 @@ __global__ void __launch_bounds__(kBlock, kWideResident) derivative_wide_kernel(
             // half the FP32 rate, and the sums of FP32 values stay exact or nearly
             // so), then over the lanes with a fixed shuffle tree
 #pragma unroll 1
-            for (int k = warp; k < kAcc; k += kStepWarps) {
+            for (int k = warp; k < values; k += kStepWarps) {
                 double sum = 0.0;
 #pragma unroll
                 for (int q = 0; q < W; ++q)
@@ -356,13 +355,14 @@ __global__ void __launch_bounds__(kBlock, kWideResident) derivative_wide_kernel(
             __syncthreads();
             if (threadIdx.x < kPartial) {
                 const int k = threadIdx.x;
-                double v;
-                if (k < 7)
-                    v = s_tot[k];
-                else if (k < 43)
-                    v = h_entry(s_tot, (k - 7) / 6, (k - 7) % 6, COMPAT ? -args.d2 : 1.0, COMPAT);
-                else
+                double v = 0.0;
+                if (k < 7) {
+                    if (k < values) v = s_tot[k];
+                } else if (k == 43) {
                     v = (double)np;
+                } else if (values == kAcc) {
+                    v = h_entry(s_tot, (k - 7) / 6, (k - 7) % 6, COMPAT ? -args.d2 : 1.0, COMPAT);
+                }
                 out[k] = v;
             }
         }

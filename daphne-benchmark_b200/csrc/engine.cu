@@ -243,6 +243,7 @@ StepParams step_params(const ndt_params &p) {
     s.step_max = p.step_size;
     s.step_min = p.transformation_epsilon / 2;
     s.watchdog_evals = p.watchdog_evals > 0 ? p.watchdog_evals : 1024;
+    s.first_mode = kEvalFull;
     return s;
 }
 
@@ -956,6 +957,65 @@ int ctx_eval_view(ndt_ctx *c, CtxEvalView *v) {
     return NDT_OK;
 }
 
+// Scores of B poses, pose b with scan b % scans (total_points: of the scans).
+int ctx_score_batch(ndt_ctx *c, int B, int scans, const float *d_points, const int *d_offsets, int total_points,
+                    const float *d_poses, double *d_score) {
+    const int tile = c->prm.precision == 1 ? kTile : kDerivVariants[c->variant].tile;
+    const long long all_points = (long long)total_points * ((B + scans - 1) / scans);
+    const long long tiles = all_points / tile + B + 1;
+    if (tiles > 2147483647LL) return fail(c, NDT_E_CAPACITY, "too many scan points to score");
+    const int max_tiles = (int)tiles;
+    CK(c->states.ensure(sizeof(AlignState) * (size_t)B));
+    RunPlan R;
+    std::memset(&R, 0, sizeof(R));
+    if (int rc0 = prepare_lists(c, B, max_tiles, R.L)) return rc0;
+    CK(c->partials.ensure(sizeof(double) * kPartial * (size_t)max_tiles));
+    CK(c->exc.ensure(sizeof(double) * kPartial * (size_t)B));
+    cudaStream_t st = c->stream;
+    c->ev_used = 0;
+    R.P = step_params(c->prm);
+    R.P.first_mode = kEvalScore;
+    R.L.scans = scans < B ? scans : 0;
+    EvalArgs &ea = R.ea;
+    ea.grid = grid_dev(c);
+    ea.points = (const float4 *)d_points;
+    ea.trans = nullptr;
+    ea.tiles = c->tiles.as<Tile>();
+    ea.num_tiles = c->num_tiles.as<int>();
+    ea.chunks = R.L.chunks;
+    ea.num_chunks = R.L.num_chunks;
+    ea.max_tiles = max_tiles;
+    ea.tile_size = tile;
+    ea.states = c->states.as<AlignState>();
+    ea.partials = c->partials.as<double>();
+    ea.exc = c->exc.as<double>();
+    ea.d1 = c->d1;
+    ea.d2 = c->d2;
+    ea.compat = c->prm.compat;
+    if (int rc2 = prepare_scratch(c, ea)) return rc2;
+    R.d_offsets = d_offsets;
+    R.d_guesses = d_poses;
+    R.ctl = c->ctl.as<RoundCtl>();
+    R.first = 1;
+    ea.reset = false;
+    R.B = B;
+    R.tile = tile;
+    R.kb = chunk_big(c);
+    R.ks = chunk_small(c);
+    R.precision = c->prm.precision;
+    R.variant = c->variant;
+    R.sms = c->num_sms;
+    ea.min_chunks = (int)(all_points / (tile * R.kb));
+    int np = 0;
+    if (int rc = enqueue_prologue(c, R, st, &np)) return rc;
+    int rc = launch_derivatives(R.ea, R.precision, R.variant, R.sms, st);
+    if (rc) return cuda_fail(c, (cudaError_t)rc, "launch_derivatives");
+    rc = launch_score(R.ea.partials, R.L.chunk_begin, R.ea.exc, B, d_score, st);
+    if (rc) return cuda_fail(c, (cudaError_t)rc, "launch_score");
+    c->launches += np + derivative_launches(R.ea, R.precision) + 1;
+    return NDT_OK;
+}
+
 void ctx_set_error(ndt_ctx *c, const char *msg) {
     if (c) c->err = msg;
 }
@@ -1209,55 +1269,7 @@ int ndt_score_batch_device(ndt_ctx *c, int B, const float *d_points, const int *
     if (int rc = set_device(c)) return rc;
     if (!c->have_map) return fail(c, NDT_E_NOMAP, "no map set");
     if (B <= 0 || total_points < 0) return fail(c, NDT_E_ARG, "empty batch");
-    const int tile = c->prm.precision == 1 ? kTile : kDerivVariants[c->variant].tile;
-    const int max_tiles = total_points / tile + B + 1;
-    CK(c->states.ensure(sizeof(AlignState) * (size_t)B));
-    RunPlan R;
-    std::memset(&R, 0, sizeof(R));
-    if (int rc0 = prepare_lists(c, B, max_tiles, R.L)) return rc0;
-    CK(c->partials.ensure(sizeof(double) * kPartial * (size_t)max_tiles));
-    CK(c->exc.ensure(sizeof(double) * kPartial * (size_t)B));
-    cudaStream_t st = c->stream;
-    c->ev_used = 0;
-    R.P = step_params(c->prm);
-    EvalArgs &ea = R.ea;
-    ea.grid = grid_dev(c);
-    ea.points = (const float4 *)d_points;
-    ea.trans = nullptr;
-    ea.tiles = c->tiles.as<Tile>();
-    ea.num_tiles = c->num_tiles.as<int>();
-    ea.chunks = R.L.chunks;
-    ea.num_chunks = R.L.num_chunks;
-    ea.max_tiles = max_tiles;
-    ea.tile_size = tile;
-    ea.states = c->states.as<AlignState>();
-    ea.partials = c->partials.as<double>();
-    ea.exc = c->exc.as<double>();
-    ea.d1 = c->d1;
-    ea.d2 = c->d2;
-    ea.compat = c->prm.compat;
-    if (int rc2 = prepare_scratch(c, ea)) return rc2;
-    R.d_offsets = d_offsets;
-    R.d_guesses = d_poses;
-    R.ctl = c->ctl.as<RoundCtl>();
-    R.first = 1;
-    ea.reset = false;
-    R.B = B;
-    R.tile = tile;
-    R.kb = chunk_big(c);
-    R.ks = chunk_small(c);
-    R.precision = c->prm.precision;
-    R.variant = c->variant;
-    R.sms = c->num_sms;
-    ea.min_chunks = total_points / (tile * R.kb);
-    int np = 0;
-    if (int rc = enqueue_prologue(c, R, st, &np)) return rc;
-    int rc = launch_derivatives(R.ea, R.precision, R.variant, R.sms, st);
-    if (rc) return cuda_fail(c, (cudaError_t)rc, "launch_derivatives");
-    rc = launch_score(R.ea.partials, R.L.chunk_begin, R.ea.exc, B, d_score, st);
-    if (rc) return cuda_fail(c, (cudaError_t)rc, "launch_score");
-    c->launches += np + derivative_launches(R.ea, R.precision) + 1;
-    return NDT_OK;
+    return ctx_score_batch(c, B, B, d_points, d_offsets, total_points, d_poses, d_score);
 }
 
 int ndt_set_batch_graphs(ndt_ctx *c, int on) {

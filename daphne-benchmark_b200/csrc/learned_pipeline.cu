@@ -59,7 +59,7 @@ struct Buf {
 struct LearnedBuffers {
     Buf h_points, h_offsets, h_guesses, h_out, h_conv, h_fit, h_status, h_choice;  // device copies of host batches
     Buf starts, y, cand, scores, start, choice_tmp;
-    Buf judge_count, judge_prefix, judge_dec, rep, rep_off;
+    Buf judge_count, judge_prefix, judge_dec;
     Buf lvl_count[NDT_LEARNED_MAX_LEVELS], lvl_prefix[NDT_LEARNED_MAX_LEVELS], lvl_dec[NDT_LEARNED_MAX_LEVELS];
     Buf out[NDT_LEARNED_MAX_LEVELS], conv[NDT_LEARNED_MAX_LEVELS], fit[NDT_LEARNED_MAX_LEVELS],
         status[NDT_LEARNED_MAX_LEVELS];
@@ -69,7 +69,7 @@ void learned_buffers_free(LearnedBuffers *lb) {
     if (!lb) return;
     Buf *all[] = {&lb->h_points, &lb->h_offsets, &lb->h_guesses, &lb->h_out, &lb->h_conv, &lb->h_fit,
                   &lb->h_status, &lb->h_choice, &lb->starts, &lb->y, &lb->cand, &lb->scores, &lb->start, &lb->choice_tmp, &lb->judge_count,
-                  &lb->judge_prefix, &lb->judge_dec, &lb->rep, &lb->rep_off};
+                  &lb->judge_prefix, &lb->judge_dec};
     for (Buf *b : all)
         if (b->p) cudaFree(b->p);
     for (int l = 0; l < NDT_LEARNED_MAX_LEVELS; ++l) {
@@ -133,22 +133,6 @@ __global__ void subsample_kernel(const float4 *__restrict__ pts, const int *__re
     const int s = offsets[b], n = offsets[b + 1] - s;
     const int o = prefix[b], m = prefix[b + 1] - o;
     for (int j = threadIdx.x; j < m; j += blockDim.x) out[o + j] = pts[s + (int)(((long long)j * n) / m)];
-}
-
-// Candidate c of C = (K + 1) B reads scan c % B: its subsample copied to its
-// own range of `rep` (the score pass takes one point range per candidate).
-__global__ void replicate_kernel(const float4 *__restrict__ sub, const int *__restrict__ prefix, int B, int C,
-                                 float4 *__restrict__ rep, int *__restrict__ rep_off) {
-    const int c = blockIdx.x;
-    const int b = c % B, k = c / B;
-    const int S = prefix[B];
-    const int src = prefix[b], m = prefix[b + 1] - src;
-    const long long dst = (long long)k * S + src;
-    if (threadIdx.x == 0) {
-        rep_off[c] = (int)dst;
-        if (c == C - 1) rep_off[C] = (int)((long long)(k + 1) * S);
-    }
-    for (int j = threadIdx.x; j < m; j += blockDim.x) rep[dst + j] = sub[src + j];
 }
 
 // Start k of scan b (candidate k B + b): the guess moved by the k-th offset
@@ -316,19 +300,13 @@ int ndt_align_batch_learned_device(ndt_mlp *c, ndt_ctx *const *levels, int n_lev
     LCK(cudaMemcpyAsync(cand + 16 * (size_t)K * B, d_guesses, sizeof(float) * 16 * (size_t)B,
                         cudaMemcpyDeviceToDevice, s_net));
 
-    // 3. the judge's subsample, one copy per candidate
+    // 3. the judge's subsample (the candidates of a scan share it)
     long long judge_bound = 0;
     if (int rc = subsample(c, s_net, d_points, d_offsets, B, lp->judge_points, lb.judge_count, lb.judge_prefix,
                            lb.judge_dec, total_points, &judge_bound))
         return rc;
-    const long long rep_bound = judge_bound * (K + 1);
-    if (rep_bound >= (1LL << 31)) return fail(c, NDT_E_CAPACITY, "ndt_align_batch_learned_device: judge subsample "
-                                                                 "too large (lower judge_points)");
-    LCK(lb.rep.ensure(sizeof(float4) * (size_t)std::max<long long>(1, rep_bound)));
-    LCK(lb.rep_off.ensure(sizeof(int) * (size_t)(C + 1)));
-    replicate_kernel<<<(int)C, 256, 0, s_net>>>(lb.judge_dec.as<float4>(), lb.judge_prefix.as<int>(), B, (int)C,
-                                                lb.rep.as<float4>(), lb.rep_off.as<int>());
-    LCK(cudaGetLastError());
+    if (judge_bound * (K + 1) >= (1LL << 31))
+        return fail(c, NDT_E_CAPACITY, "ndt_align_batch_learned_device: judge subsample too large (lower judge_points)");
     // subsamples of the refinement levels that read fewer points
     const float *lvl_pts[NDT_LEARNED_MAX_LEVELS];
     const int *lvl_off[NDT_LEARNED_MAX_LEVELS];
@@ -356,8 +334,8 @@ int ndt_align_batch_learned_device(ndt_mlp *c, ndt_ctx *const *levels, int n_lev
     LCK(cudaStreamWaitEvent(s_lvl[J], c->ev[0], 0));
     LCK(lb.scores.ensure(sizeof(double) * (size_t)C));
     LCK(lb.start.ensure(sizeof(float) * 16 * (size_t)B));
-    if (int rc = ndt_score_batch_device(levels[J], (int)C, lb.rep.as<float>(), lb.rep_off.as<int>(), (int)rep_bound,
-                                        cand, lb.scores.as<double>())) {
+    if (int rc = ndt::ctx_score_batch(levels[J], (int)C, B, lb.judge_dec.as<float>(), lb.judge_prefix.as<int>(),
+                                      (int)judge_bound, cand, lb.scores.as<double>())) {
         c->msg = std::string("judge: ") + ndt_last_error(levels[J]);
         return rc;
     }

@@ -20,7 +20,18 @@ enum EvalMode : int32_t {
     kEvalFull = 1,      // score, gradient, Hessian (computeDerivatives(..., true))
     kEvalGradient = 2,  // score, gradient; Hessian reset to 0 (computeDerivatives(..., false))
     kEvalHessian = 3,   // Hessian only (computeHessian)
+    kEvalScore = 4,     // score alone (the judge of pose candidates)
 };
+
+// What an evaluation sums up, by its mode: the score (1 value), the gradient
+// as well (7), the Hessian as well (all).
+enum EvalLevel : int { kLevelScore = 0, kLevelGradient = 1, kLevelHessian = 2 };
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline constexpr int eval_level(int mode) {
+    return mode == kEvalScore ? kLevelScore : (mode == kEvalGradient ? kLevelGradient : kLevelHessian);
+}
 
 // Phases of the per-alignment registration state machine (one Newton
 // iteration = solve + More-Thuente step length + pose update).
@@ -156,6 +167,7 @@ struct TileLists {
     // back (see active_chunk in pair_f32.cuh)
     int *active_chunks = nullptr;
     int capacity = 0;  // entries of active_chunks
+    int scans = 0;     // > 0: alignment b reads scan b % scans (offsets hold scans + 1 entries)
 };
 
 }  // namespace ndt

@@ -40,7 +40,7 @@ __device__ __forceinline__ void zero(PairSums &F) {
 }
 
 __device__ __forceinline__ void pair_sums(PairSums &F, float p0, float p1, float p2, float c00, float c01, float c02,
-                                          float c11, float c12, float c22, float d1, float d2, bool hess) {
+                                          float c11, float c12, float c22, float d1, float d2, int level) {
     const float q0 = fmaf(c00, p0, fmaf(c01, p1, c02 * p2));
     const float q1 = fmaf(c01, p0, fmaf(c11, p1, c12 * p2));
     const float q2 = fmaf(c02, p0, fmaf(c12, p1, c22 * p2));
@@ -48,8 +48,9 @@ __device__ __forceinline__ void pair_sums(PairSums &F, float p0, float p1, float
     const float e = expf(-d2 * xCx * 0.5f);
     const float e2 = d2 * e;
     if (!(e2 <= 1.0f && e2 >= 0.0f)) return;  // kernel.cpp:456 (also rejects NaN)
-    const float w = d1 * e2;
     F.s = fmaf(-d1, e, F.s);
+    if (level == kLevelScore) return;
+    const float w = d1 * e2;
     // every multiply-add is written as fmaf or as separately rounded
     // operations, so the FP32 results do not depend on the compiler's
     // contraction choices (which can change with the surrounding code)
@@ -57,7 +58,7 @@ __device__ __forceinline__ void pair_sums(PairSums &F, float p0, float p1, float
     F.u0 = fmaf(w, q0, F.u0);
     F.u1 = fmaf(w, q1, F.u1);
     F.u2 = fmaf(w, q2, F.u2);
-    if (!hess) return;
+    if (level != kLevelHessian) return;
     F.q00 = fmaf(wq0, q0, F.q00);
     F.q01 = fmaf(wq0, q1, F.q01);
     F.q02 = fmaf(wq0, q2, F.q02);
@@ -87,22 +88,23 @@ __device__ __forceinline__ void sym_mul(float m00, float m01, float m02, float m
 // ang = the alignment's FP32 angle terms (j_ang a..h, h_ang a2..f3, 3 each).
 template <bool ADD>
 __device__ __forceinline__ void contract(const PairSums &F, float x0, float x1, float x2, const float *ang,
-                                         float *acc, int stride, float d2, bool hess, bool compat) {
+                                         float *acc, int stride, float d2, int level, bool compat) {
     auto put = [](float *p, float v) { *p = ADD ? *p + v : v; };
+    put(acc, F.s);
+    if (level == kLevelScore) return;
     // J_3 = (0, J13, J23), J_4 = (J04, J14, J24), J_5 = (J05, J15, J25)
     // (computePointDerivatives, kernel.cpp:512-521)
     const float J13 = dot3f(x0, x1, x2, ang + 0), J23 = dot3f(x0, x1, x2, ang + 3);
     const float J04 = dot3f(x0, x1, x2, ang + 6), J14 = dot3f(x0, x1, x2, ang + 9);
     const float J24 = dot3f(x0, x1, x2, ang + 12), J05 = dot3f(x0, x1, x2, ang + 15);
     const float J15 = dot3f(x0, x1, x2, ang + 18), J25 = dot3f(x0, x1, x2, ang + 21);
-    put(acc, F.s);
     put(acc + 1 * stride, F.u0);
     put(acc + 2 * stride, F.u1);
     put(acc + 3 * stride, F.u2);
     put(acc + 4 * stride, fmaf(J13, F.u1, J23 * F.u2));
     put(acc + 5 * stride, fmaf(J04, F.u0, fmaf(J14, F.u1, J24 * F.u2)));
     put(acc + 6 * stride, fmaf(J05, F.u0, fmaf(J15, F.u1, J25 * F.u2)));
-    if (!hess) return;
+    if (level != kLevelHessian) return;
     // P = W - d2 Q
     const float nd2 = -d2;
     const float P00 = fmaf(nd2, F.q00, F.w00), P01 = fmaf(nd2, F.q01, F.w01), P02 = fmaf(nd2, F.q02, F.w02);
@@ -173,6 +175,10 @@ __device__ __forceinline__ void contract(const PairSums &F, float x0, float x1, 
     }
 }
 
+__device__ __forceinline__ int level_values(int level) {
+    return level == kLevelScore ? 1 : (level == kLevelGradient ? 7 : kAcc);
+}
+
 // Chunks of this pass, and the k-th of them: of the active list (large chunks
 // from its front, small ones from its back, so that the small ones come last),
 // or of all chunks.
@@ -194,13 +200,13 @@ __device__ __forceinline__ void queue_flagged(const EvalArgs &args, int align, i
 // x' = x_trans - mean (kernel.cpp:692-694) from the (hi, lo) float split of
 // the FP64 mean, and the pair's sums.
 __device__ __forceinline__ void add_pair(const GridDev &g, PairSums &F, int slot, float px, float py, float pz, float d1,
-                                         float d2, bool hess) {
+                                         float d2, int level) {
     const float4 *r = g.vox32 + 3 * slot;  // one 48-byte record
     const float4 hi = __ldg(r), lo = __ldg(r + 1), cc = __ldg(r + 2);
     const float p0 = __fsub_rn(__fsub_rn(px, hi.x), lo.x);
     const float p1 = __fsub_rn(__fsub_rn(py, hi.y), lo.y);
     const float p2 = __fsub_rn(__fsub_rn(pz, hi.z), lo.z);
-    pair_sums(F, p0, p1, p2, hi.w, lo.w, cc.x, cc.y, cc.z, cc.w, d1, d2, hess);
+    pair_sums(F, p0, p1, p2, hi.w, lo.w, cc.x, cc.y, cc.z, cc.w, d1, d2, level);
 }
 
 }  // namespace ndt

@@ -67,3 +67,31 @@ def test_wide_equals_many_far_coordinates(pkg, chunk_tiles):
         assert ctx.counters()["probes"] > 27 * len(scan)  # the generic path, more than one collect call
     # (voxels this far out go through the FP64 side queue: room for every copy's pairs)
     _same(pkg, prm, cloud, [scan], [guess], chunk_tiles, 6, side_pairs=1 << 24)
+
+
+@pytest.mark.parametrize("compat", [0, 1])
+@pytest.mark.parametrize("n,copies", [(1, 1), (130, 1), (2600, 1), (2600, COPIES)])
+def test_score_pass_equals_full_evaluation(pkg, compat, n, copies):
+    """A score pass sums the score alone; it is the score of the full
+    evaluation (score, gradient, Hessian) bit for bit, on both kernels."""
+    torch = pytest.importorskip("torch")
+    cfg = pkg.synth.small_config("score", 12000, 34.0, 12, 700, seed=78, dt=0.4, dyaw_deg=3.0, radius=16.0)
+    scene = pkg.synth.make_scene(cfg)
+    a = pkg.synth.make_alignment(cfg, scene, 0, n_points=n)
+    T = a.guess.reshape(4, 4)
+    x, y, z = a.scan[:, 0], a.scan[:, 1], a.scan[:, 2]
+    trans = np.ones_like(a.scan)
+    for r in range(3):  # float, left to right, as the derivative pass transforms
+        trans[:, r] = ((T[r, 0] * x + T[r, 1] * y) + T[r, 2] * z) + T[r, 3]
+    prm = (pkg.ndt.reference_params if compat else pkg.ndt.corrected_params)(1.0)
+    with pkg.ndt.Context(prm) as ctx:
+        ctx.set_map(scene.map)
+        full, _, _ = ctx.derivatives(a.scan, trans, np.zeros(6))
+        pts = torch.from_numpy(np.tile(a.scan, (copies, 1))).cuda()
+        off = torch.arange(copies + 1, dtype=torch.int32).cuda() * n
+        poses = torch.from_numpy(np.tile(a.guess, (copies, 1))).cuda()
+        out = torch.zeros(copies, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        ctx.score_batch_device(copies, pts.data_ptr(), off.data_ptr(), copies * n, poses.data_ptr(), out.data_ptr())
+        ctx.synchronize()
+    assert (out.cpu().numpy().view(np.uint64) == np.float64(full).view(np.uint64)).all()
