@@ -78,7 +78,7 @@ __device__ __forceinline__ int part_of(const T *first, int np, long long t) {
 }
 
 __global__ void key_kernel(const float4 *__restrict__ pts, int n, const __grid_constant__ Parts P,
-                           uint32_t *__restrict__ keys, uint32_t *__restrict__ vals, int *__restrict__ parent) {
+                           uint32_t *__restrict__ keys, int *__restrict__ parent) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int q = part_of(P.off, P.np, i);
@@ -87,7 +87,6 @@ __global__ void key_kernel(const float4 *__restrict__ pts, int n, const __grid_c
     const int cy = cell_of(p.y, P.minv[q][1], P.cell[q], P.dim[q][1]);
     const int cz = cell_of(p.z, P.minv[q][2], P.cell[q], P.dim[q][2]);
     keys[i] = (uint32_t)(P.base[q] + cx + (long long)P.dim[q][0] * (cy + (long long)P.dim[q][1] * cz));
-    vals[i] = (uint32_t)i;
     parent[i] = i;
 }
 
@@ -297,8 +296,8 @@ int labels_of(ndt_ec *h, const std::vector<const float *> &xyz, const std::vecto
     ECK(cudaMemsetAsync(h->cell_first, 0xff, sizeof(int) * (size_t)cells, st));
     ndt::SortBuffers sb = ndt::sort_buffers(h->scratch, N);
     const unsigned blocks = (unsigned)((N + ec::kThreads - 1) / ec::kThreads);
-    ec::key_kernel<<<blocks, ec::kThreads, 0, st>>>(d_pts, N, P, sb.k0, sb.v0, parent);
-    ndt::sort_segments(sb, N, bits, (int32_t *)h->seg_start, (uint32_t *)h->seg_key, st);
+    ec::key_kernel<<<blocks, ec::kThreads, 0, st>>>(d_pts, N, P, sb.k0, parent);
+    ndt::sort_segments(sb, N, bits, (int32_t *)h->seg_start, (uint32_t *)h->seg_key, st, true);
     ec::cell_index_kernel<<<blocks, ec::kThreads, 0, st>>>((const int32_t *)h->seg_start, (const uint32_t *)h->seg_key,
                                                            sb.nseg, (int *)h->cell_first);
     ec::join_kernel<<<dim3(blocks, 27 * ec::kSplit), ec::kThreads, 0, st>>>(
@@ -306,9 +305,11 @@ int labels_of(ndt_ec *h, const std::vector<const float *> &xyz, const std::vecto
     ec::label_kernel<<<blocks, ec::kThreads, 0, st>>>(parent, N, err);
     ECK(cudaGetLastError());
     ECK(cudaMemcpyAsync(h->h_labels, parent, sizeof(int) * (size_t)N, cudaMemcpyDeviceToHost, st));
-    int e = 0;
+    int e = 0, sort_err = 0;
     ECK(cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    ECK(cudaMemcpyAsync(&sort_err, ndt::sort_error(sb, N), sizeof(int), cudaMemcpyDeviceToHost, st));
     ECK(cudaStreamSynchronize(st));
+    if (sort_err) return fail(h, NDT_E_CUDA, "a wait between the sort's tiles gave up");
     if (e) return fail(h, NDT_E_CUDA, "union-find retry limit reached");
     for (int q = 0; q < np; ++q)
         for (int i = 0; i < n[q]; ++i) labels[q][i] = h->h_labels[P.off[q] + i] - P.off[q];
@@ -345,6 +346,7 @@ int ndt_ec_create(int device, ndt_ec **out) {
     ndt_ec *h = new ndt_ec();
     h->device = device;
     cudaError_t e = cudaSetDevice(device);
+    if (e == cudaSuccess) e = (cudaError_t)ndt::prepare_sort();
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) {
         delete h;

@@ -1070,6 +1070,7 @@ int ndt_create(const ndt_params *params, int device, ndt_ctx **out) {
     if (e == cudaSuccess) e = cudaMemset(c->dev_launches.p, 0, sizeof(unsigned long long));
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess) e = (cudaError_t)prepare_derivatives();
+    if (e == cudaSuccess) e = (cudaError_t)prepare_sort();
     if (e != cudaSuccess) {
         delete c;
         return NDT_E_CUDA;

@@ -4,8 +4,8 @@
 // Pipeline (one map):
 //   bbox_partial / bbox_final   bounding box +-0.01, dims, G        (:1305-1322)
 //   cell_key                    dense cell id of every map point     (:1343, :236-244)
-//   radix_{upsweep,scan,down}   stable LSD sort of (cell, point index)
-//   seg_{count,write}           one segment per occupied cell
+//   radix_{hist,pass}           stable LSD sort of (cell, point index)
+//   segment                     one segment per occupied cell
 //   cell_finalize_{compat,corrected}
 //                               per-cell sums in point order, covariance, inverse
 //
@@ -25,10 +25,12 @@ namespace ndt {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kItems = 8;                       // items per thread in the sort / segment tiles
-constexpr int kSortTile = kThreads * kItems;    // 2048
+constexpr int kSegItems = 16;                   // items per thread in the segment tiles
+constexpr int kSegThreads = 1024, kSegWarps = kSegThreads / 32;
+constexpr int kSegTile = kSegThreads * kSegItems;
 constexpr int kWarps = kThreads / 32;
-constexpr int kMaxDigits = 1 << 10;             // radix digits of one pass, at most
+constexpr int kDigits = 256;                    // radix digits of one pass: one per thread
+constexpr int kMaxPasses = 4;
 // Scratch layout: [bounding-box partials (6 x 1024 floats) + its 2 counters,
 // which must stay zero between builds] [sort and segment buffers].
 constexpr size_t kBboxFlagsOffset = sizeof(float) * 6 * 1024;
@@ -135,7 +137,7 @@ __global__ void bbox_kernel(const float4 *__restrict__ map, int m, float *__rest
 
 // Dense cell id of each map point (linearizeCoord, kernel.cpp:236-244).
 __global__ void cell_key_kernel(const float4 *__restrict__ map, int m, const GridMeta *__restrict__ meta,
-                                uint32_t *__restrict__ keys, uint32_t *__restrict__ vals, int index_offset = 0) {
+                                uint32_t *__restrict__ keys) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m) return;
     const GridMeta g = *meta;
@@ -145,7 +147,6 @@ __global__ void cell_key_kernel(const float4 *__restrict__ map, int m, const Gri
     int iy = (int)((p.y - g.minv[1]) / g.res);
     int iz = (int)((p.z - g.minv[2]) / g.res);
     keys[i] = (uint32_t)(ix + g.dim[0] * (iy + g.dim[1] * iz));
-    vals[i] = (uint32_t)(i + index_offset);
 }
 
 // Stable merge of two key-sorted (key, value) runs, run a first on equal
@@ -154,9 +155,9 @@ __global__ void cell_key_kernel(const float4 *__restrict__ map, int m, const Gri
 // once).
 __global__ void merge_kernel(const uint32_t *__restrict__ ka, const uint32_t *__restrict__ va, int na,
                              const uint32_t *__restrict__ kb, const uint32_t *__restrict__ vb, int nb,
-                             uint32_t *__restrict__ ko, uint32_t *__restrict__ vo) {
+                             uint32_t *__restrict__ ko, uint32_t *__restrict__ vo, const int *__restrict__ sort_err) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= na + nb) return;
+    if (t >= na + nb || *sort_err) return;
     if (t < na) {
         const uint32_t key = ka[t];
         int lo = 0, hi = nb;  // first b key >= key
@@ -180,23 +181,288 @@ __global__ void merge_kernel(const uint32_t *__restrict__ ka, const uint32_t *__
 }
 
 // ---------------------------------------------------------------------------
-// Stable LSD radix sort of (key, value) pairs, `bits`-wide digit per pass.
-// hist layout: digit-major, hist[d * nblk + block].
-__global__ void radix_upsweep_kernel(const uint32_t *__restrict__ keys, int n, int shift, int bits,
-                                     int *__restrict__ hist) {
-    extern __shared__ int s_hist[];
-    const int nb = 1 << bits;
-    for (int d = threadIdx.x; d < nb; d += blockDim.x) s_hist[d] = 0;
-    __syncthreads();
-    const int base = blockIdx.x * kSortTile;
-    const uint32_t mask = (uint32_t)nb - 1u;
+// Chained prefixes: tile t of a launch publishes its own sum, then the sum of
+// all tiles up to it; a later tile walks back over the published values.
+// Tiles are numbered by an atomic ticket, so every tile that one waits for is
+// already running and never waits for a later one.  A word holds the state in
+// its two top bits and the count below them.
+template <class S>
+struct Chain {
+    static constexpr int kShift = 8 * (int)sizeof(S) - 2;
+    static constexpr S kMask = ((S)1 << kShift) - 1;
+    static __device__ __forceinline__ void publish(S *w, int flag, S count) {
+        *(volatile S *)w = ((S)flag << kShift) | count;
+    }
+    static __device__ __forceinline__ S load(const S *w) { return *(const volatile S *)w; }
+};
+constexpr int kOwnSum = 1, kUpToSum = 2;
+constexpr int kLookback = 16;                   // words read at a time
+constexpr unsigned kChainPolls = 1u << 24;      // polls before a wait gives up (no healthy launch comes near)
+
+// Sum of the counts of the tiles before `tile` in column `col` of state
+// [tiles][cols]; *bad = true when a wait gave up.
+template <class S>
+__device__ __forceinline__ S chain_before(const S *state, int tile, int cols, int col, bool &bad) {
+    S sum = 0;
+    unsigned polls = 0;
+    for (int p = tile - 1; p >= 0;) {
+        S v[kLookback];
 #pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-        int i = base + k * kThreads + threadIdx.x;
-        if (i < n) atomicAdd(&s_hist[(keys[i] >> shift) & mask], 1);
+        for (int u = 0; u < kLookback; ++u)
+            v[u] = p - u >= 0 ? Chain<S>::load(state + (size_t)(p - u) * cols + col)
+                              : (S)kUpToSum << Chain<S>::kShift;
+        int used = 0;
+        bool end = false, wait = false;
+#pragma unroll
+        for (int u = 0; u < kLookback; ++u) {
+            if (end || wait) continue;
+            const int flag = (int)(v[u] >> Chain<S>::kShift);
+            if (flag == 0) {
+                wait = true;
+                continue;
+            }
+            sum += v[u] & Chain<S>::kMask;
+            ++used;
+            end = flag == kUpToSum;
+        }
+        if (end) break;
+        p -= used;
+        if (wait) {
+            if (++polls > kChainPolls) {
+                bad = true;
+                break;
+            }
+            __nanosleep(100);
+        }
+    }
+    return sum;
+}
+
+// The same for one column by a whole warp, 32 words at a time.
+__device__ __forceinline__ uint64_t warp_chain_before(const uint64_t *state, int tile, bool &bad) {
+    using C = Chain<uint64_t>;
+    const int lane = threadIdx.x & 31;
+    uint64_t sum = 0;
+    unsigned polls = 0;
+    for (int p = tile - 1; p >= 0;) {
+        const uint64_t v = p - lane >= 0 ? C::load(state + p - lane) : (uint64_t)kUpToSum << C::kShift;
+        const int flag = (int)(v >> C::kShift);
+        const unsigned ready = __ballot_sync(0xffffffffu, flag != 0), end = __ballot_sync(0xffffffffu, flag == kUpToSum);
+        const int run = ready == 0xffffffffu ? 32 : __ffs(~ready) - 1;  // words published without a gap
+        const int last = end ? __ffs(end) - 1 : 32;
+        const int take = last < run ? last + 1 : run;
+        uint64_t mine = lane < take ? v & C::kMask : 0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+        sum += mine;
+        if (last < run) break;
+        p -= take;
+        if (take < 32 && ++polls > kChainPolls) {
+            bad = true;
+            break;
+        }
+    }
+    return sum;
+}
+
+// ---------------------------------------------------------------------------
+// Stable LSD radix sort of (key, value) pairs, at most 8 bits per pass.  One
+// histogram kernel counts every pass's digits in one read of the keys; a pass
+// is one kernel (each tile finds where its digits go from the chained counts
+// of the tiles before it), so a pass reads and writes every pair once.
+// Bound by the chain: tiles in flight at the same time look back over one
+// another, so few large tiles (two blocks of 1024 threads per SM) beat many
+// small ones (2M pairs, one pass: 29 us with 512 x 8 items, 25 us with 1024 x
+// 8), and by the ranks: peer masks from 8 ballots instead of
+// __match_any_sync, 30 -> 25 us.  Sort and segments against a histogram, a
+// scan and a scatter kernel per pass: 400k pairs of 18 bits 61 -> 41 us, 2M
+// pairs of 22 bits 155 -> 99 us; 16.7M pairs of 23 bits 582 -> 579 us.
+constexpr int kHistItems = 8;
+constexpr int kSortThreads = 1024, kSortWarps = kSortThreads / 32;
+
+struct RadixPlan {
+    int passes, width, bits;
+};
+
+__host__ __device__ inline int pass_bits(const RadixPlan &p, int pass) {
+    const int rest = p.bits - pass * p.width;
+    return rest < p.width ? rest : p.width;
+}
+
+RadixPlan radix_plan(int bits) {
+    RadixPlan p;
+    p.bits = bits;
+    p.passes = (bits + 7) / 8;
+    p.width = (bits + p.passes - 1) / p.passes;
+    return p;
+}
+
+__global__ void __launch_bounds__(kThreads) radix_hist_kernel(const uint32_t *__restrict__ keys, int n, RadixPlan P,
+                                                              unsigned *__restrict__ hist) {
+    __shared__ unsigned s_hist[kMaxPasses][kDigits];
+    for (int d = threadIdx.x; d < kMaxPasses * kDigits; d += kThreads) (&s_hist[0][0])[d] = 0;
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const long long stride = (long long)gridDim.x * kThreads * kHistItems;
+    for (long long base = (long long)blockIdx.x * kThreads * kHistItems; base < n; base += stride) {
+        uint32_t key[kHistItems];
+#pragma unroll
+        for (int k = 0; k < kHistItems; ++k) {
+            const long long i = base + k * kThreads + threadIdx.x;
+            key[k] = i < n ? keys[i] : 0u;
+        }
+#pragma unroll
+        for (int k = 0; k < kHistItems; ++k) {
+            const bool valid = base + k * kThreads + threadIdx.x < n;
+            const unsigned mask = __ballot_sync(0xffffffffu, valid);
+            if (!valid) continue;
+            for (int p = 0; p < P.passes; ++p) {
+                const uint32_t d = (key[k] >> (p * P.width)) & ((1u << pass_bits(P, p)) - 1u);
+                // neighbours often share their high digits: one add for the warp
+                if (__all_sync(mask, d == __shfl_sync(mask, d, 0))) {
+                    if (lane == 0) atomicAdd(&s_hist[p][d], __popc(mask));
+                } else {
+                    atomicAdd(&s_hist[p][d], 1u);
+                }
+            }
+        }
     }
     __syncthreads();
-    for (int d = threadIdx.x; d < nb; d += blockDim.x) hist[d * gridDim.x + blockIdx.x] = s_hist[d];
+    for (int d = threadIdx.x; d < P.passes * kDigits; d += kThreads) {
+        const unsigned c = (&s_hist[0][0])[d];
+        if (c) atomicAdd(hist + d, c);
+    }
+}
+
+// One pass.  Warp w of a tile owns ITEMS runs of 32 consecutive items; ranks
+// inside a run come from the masks of the lanes with the same digit, so equal
+// digits keep their input order.  The tile is put in digit order in shared memory first,
+// so that its writes are runs of consecutive addresses.  vin == nullptr: the
+// values are the items' indices from iota on.  *err: a wait gave up (the pairs
+// are then not written).
+template <int ITEMS, class S>
+__global__ void __launch_bounds__(kSortThreads) radix_pass_kernel(const uint32_t *__restrict__ kin,
+                                                              const uint32_t *__restrict__ vin, uint32_t iota,
+                                                              uint32_t *__restrict__ kout, uint32_t *__restrict__ vout,
+                                                              int n, int shift, int bits,
+                                                              const unsigned *__restrict__ hist, S *__restrict__ state,
+                                                              int *__restrict__ ticket, int *__restrict__ err) {
+    constexpr int kTileItems = kSortThreads * ITEMS;
+    extern __shared__ __align__(16) unsigned char s_dyn[];
+    unsigned (*s_cnt)[kDigits] = reinterpret_cast<unsigned (*)[kDigits]>(s_dyn);
+    uint32_t *s_key = reinterpret_cast<uint32_t *>(s_cnt + kSortWarps), *s_val = s_key + kTileItems;
+    __shared__ unsigned s_base[kDigits];
+    __shared__ unsigned s_warp[2][kDigits / 32];
+    __shared__ int s_tile;
+    const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+    if (t == 0) s_tile = atomicAdd(ticket, 1);
+    for (int d = t; d < kSortWarps * kDigits; d += kSortThreads) (&s_cnt[0][0])[d] = 0;
+    __syncthreads();
+    const int tile = s_tile;
+    const long long base = (long long)tile * kTileItems;
+    const int count = (int)(n - base < kTileItems ? n - base : kTileItems);
+    const uint32_t mask = (1u << bits) - 1u;
+    const int wbase = w * 32 * ITEMS;
+    uint32_t key[ITEMS], val[ITEMS];
+    unsigned short rank[ITEMS];
+    const unsigned lt = lanemask_lt();
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+        const int i = wbase + k * 32 + lane;
+        key[k] = i < count ? kin[base + i] : 0u;
+        val[k] = i < count ? (vin ? vin[base + i] : iota + (uint32_t)(base + i)) : 0u;
+    }
+    unsigned *cnt = s_cnt[w];
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+        const int i = wbase + k * 32 + lane;
+        const bool valid = i < count;
+        const uint32_t d = (key[k] >> shift) & mask;
+        unsigned peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            if (q < bits) {
+                const bool one = (d >> q) & 1u;
+                const unsigned ones = __ballot_sync(0xffffffffu, one);
+                peers &= one ? ones : ~ones;
+            }
+        const unsigned before = valid ? cnt[d] : 0u;
+        __syncwarp();
+        rank[k] = (unsigned short)(before + __popc(peers & lt));
+        if (valid && (peers & lt) == 0u) cnt[d] = before + __popc(peers);
+        __syncwarp();
+    }
+    __syncthreads();
+    // thread d < 256: digit d
+    bool bad = false;
+    unsigned total = 0, start = 0, first = 0;
+    S *mine = state + (size_t)tile * kDigits + t;
+    if (t < kDigits) {
+#pragma unroll
+        for (int ww = 0; ww < kSortWarps; ++ww) {
+            const unsigned c = s_cnt[ww][t];
+            s_cnt[ww][t] = total;
+            total += c;
+        }
+        Chain<S>::publish(mine, tile == 0 ? kUpToSum : kOwnSum, (S)total);
+        // exclusive prefixes over the digits: of the tile's items, of all items
+        const unsigned all = hist[t];
+        start = total;
+        first = all;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned u = __shfl_up_sync(0xffffffffu, start, o), v = __shfl_up_sync(0xffffffffu, first, o);
+            if (lane >= o) {
+                start += u;
+                first += v;
+            }
+        }
+        if (lane == 31) {
+            s_warp[0][w] = start;
+            s_warp[1][w] = first;
+        }
+        start -= total;
+        first -= all;
+    }
+    __syncthreads();
+    if (t < kDigits) {
+        for (int k = 0; k < w; ++k) {
+            start += s_warp[0][k];
+            first += s_warp[1][k];
+        }
+        S before = 0;
+        if (tile > 0) {
+            before = chain_before<S>(state, tile, kDigits, t, bad);
+            if (!bad) Chain<S>::publish(mine, kUpToSum, before + (S)total);
+        }
+        s_base[t] = first + (unsigned)before - start;
+#pragma unroll
+        for (int ww = 0; ww < kSortWarps; ++ww) s_cnt[ww][t] += start;
+    }
+    if (__syncthreads_or(bad)) {
+        if (t == 0) atomicOr(err, 1);
+        return;
+    }
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+        const int i = wbase + k * 32 + lane;
+        if (i < count) {
+            const unsigned at = cnt[(key[k] >> shift) & mask] + rank[k];
+            s_key[at] = key[k];
+            s_val[at] = val[k];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+        const int j = k * kSortThreads + t;
+        if (j < count) {
+            const uint32_t q = s_key[j];
+            const unsigned pos = s_base[(q >> shift) & mask] + (unsigned)j;
+            kout[pos] = q;
+            vout[pos] = s_val[j];
+        }
+    }
 }
 
 // Exclusive scan of data[begin, end) in place by one block of 1024 threads,
@@ -314,113 +580,74 @@ int scan_exclusive(int *data, int n, int *total, int *part, cudaStream_t st) {
 
 size_t scan_part_ints(size_t n) { return (n + kScanTile - 1) / kScanTile + 1; }
 
-// Stable scatter: warp w of a block owns items [base + w*256, base + w*256 + 256)
-// in 8 chunks of 32 consecutive items; ranks inside a chunk come from
-// __match_any_sync peer masks, so equal digits keep their input order.
-__global__ void radix_downsweep_kernel(const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin,
-                                       uint32_t *__restrict__ kout, uint32_t *__restrict__ vout, int n,
-                                       int shift, int bits, const int *__restrict__ hist) {
-    extern __shared__ int s_cnt[];  // [kWarps][nb]
-    const int nb = 1 << bits;
-    const uint32_t mask = (uint32_t)nb - 1u;
-    for (int d = threadIdx.x; d < kWarps * nb; d += blockDim.x) s_cnt[d] = 0;
-    __syncthreads();
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int wbase = blockIdx.x * kSortTile + w * (32 * kItems);
-    int *cnt = s_cnt + w * nb;
-    uint32_t key[kItems], val[kItems];
-    int rank[kItems];
-    const unsigned lt = lanemask_lt();
-#pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-        int i = wbase + k * 32 + lane;
-        bool valid = i < n;
-        key[k] = valid ? kin[i] : 0u;
-        val[k] = valid ? vin[i] : 0u;
-        uint32_t d = valid ? ((key[k] >> shift) & mask) : (uint32_t)nb;  // sentinel group
-        unsigned peers = __match_any_sync(0xffffffffu, d);
-        int before = valid ? cnt[d] : 0;
-        __syncwarp();
-        rank[k] = before + __popc(peers & lt);
-        int leader = __ffs(peers) - 1;
-        if (valid && lane == leader) cnt[d] = before + __popc(peers);
-        __syncwarp();
-    }
-    __syncthreads();
-    // exclusive prefix over warps, per digit
-    for (int d = threadIdx.x; d < nb; d += blockDim.x) {
-        int run = 0;
-        for (int ww = 0; ww < kWarps; ++ww) {
-            int c = s_cnt[ww * nb + d];
-            s_cnt[ww * nb + d] = run;
-            run += c;
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-        int i = wbase + k * 32 + lane;
-        if (i < n) {
-            uint32_t d = (key[k] >> shift) & mask;
-            int pos = hist[d * gridDim.x + blockIdx.x] + cnt[d] + rank[k];
-            kout[pos] = key[k];
-            vout[pos] = val[k];
-        }
-    }
-}
-
 // ---------------------------------------------------------------------------
-// Segments of equal keys in the sorted order = occupied cells.
-__device__ __forceinline__ bool is_head(const uint32_t *k, int i) { return i == 0 || k[i] != k[i - 1]; }
-
-__global__ void seg_count_kernel(const uint32_t *__restrict__ keys, int n, int *__restrict__ counts) {
-    int c = 0;
-    const int base = blockIdx.x * kSortTile;
-#pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-        int i = base + k * kThreads + threadIdx.x;
-        if (i < n && is_head(keys, i)) ++c;
-    }
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-    __shared__ int s[kWarps];
-    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = c;
+// Segments of equal keys in the sorted order = occupied cells: seg_start[s] and
+// seg_key[s] of every segment, in sorted order, and their number, in one read
+// of the keys (the tiles' counts are chained).  After a sort that gave up
+// (*err) there are none.
+__global__ void __launch_bounds__(kSegThreads) segment_kernel(const uint32_t *__restrict__ keys, int n,
+                                                           int *__restrict__ seg_start, uint32_t *__restrict__ seg_key,
+                                                           int *__restrict__ nseg, uint64_t *__restrict__ state,
+                                                           int *__restrict__ ticket, int *__restrict__ err) {
+    __shared__ unsigned s_cnt[kSegWarps];
+    __shared__ unsigned s_before;
+    __shared__ int s_tile;
+    const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+    if (t == 0) s_tile = *(volatile int *)err ? -1 : atomicAdd(ticket, 1);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int t = 0;
-        for (int k = 0; k < kWarps; ++k) t += s[k];
-        counts[blockIdx.x] = t;
+    const int tile = s_tile;
+    if (tile < 0) {
+        if (t == 0) *nseg = 0;
+        return;
     }
-}
-
-// Writes seg_start[s] and seg_cell[s] for every segment head, s in sorted order.
-__global__ void seg_write_kernel(const uint32_t *__restrict__ keys, int n, const int *__restrict__ offsets,
-                                 int *__restrict__ seg_start, uint32_t *__restrict__ seg_cell) {
-    __shared__ int s_warp[kWarps];
-    __shared__ int s_run;
-    if (threadIdx.x == 0) s_run = offsets[blockIdx.x];
-    const int base = blockIdx.x * kSortTile;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int k = 0; k < kItems; ++k) {
-        int i = base + k * kThreads + threadIdx.x;
-        bool h = i < n && is_head(keys, i);
-        unsigned b = __ballot_sync(0xffffffffu, h);
-        if (lane == 0) s_warp[w] = __popc(b);
-        __syncthreads();
-        int before = 0, total = 0;
-        for (int ww = 0; ww < kWarps; ++ww) {
-            int c = s_warp[ww];
-            if (ww < w) before += c;
-            total += c;
+    // warp w: kSegItems runs of 32 consecutive keys
+    const long long base = (long long)tile * kSegTile + w * 32 * kSegItems;
+    uint32_t key[kSegItems];
+    unsigned heads[kSegItems];
+#pragma unroll
+    for (int k = 0; k < kSegItems; ++k) key[k] = base + 32 * k + lane < n ? keys[base + 32 * k + lane] : 0u;
+    uint32_t carry = base > 0 && base < n ? keys[base - 1] : 0u;
+    unsigned mine = 0;
+#pragma unroll
+    for (int k = 0; k < kSegItems; ++k) {
+        const long long i = base + 32 * k + lane;
+        uint32_t prev = __shfl_up_sync(0xffffffffu, key[k], 1);
+        if (lane == 0) prev = carry;
+        carry = __shfl_sync(0xffffffffu, key[k], 31);
+        heads[k] = __ballot_sync(0xffffffffu, i < n && (i == 0 || key[k] != prev));
+        mine += __popc(heads[k]);
+    }
+    if (lane == 0) s_cnt[w] = mine;
+    __syncthreads();
+    unsigned total = 0, before = 0;
+#pragma unroll
+    for (int ww = 0; ww < kSegWarps; ++ww) {
+        if (ww < w) before += s_cnt[ww];
+        total += s_cnt[ww];
+    }
+    if (w == 0) {
+        bool bad = false;
+        if (lane == 0) Chain<uint64_t>::publish(state + tile, tile == 0 ? kUpToSum : kOwnSum, total);
+        const uint64_t b = warp_chain_before(state, tile, bad);
+        if (lane == 0) {
+            if (!bad) Chain<uint64_t>::publish(state + tile, kUpToSum, b + total);
+            if (bad) atomicOr(err, 1);
+            s_before = (unsigned)b;
+            s_tile = bad ? -1 : tile;
+            if (tile == (int)gridDim.x - 1) *nseg = bad ? 0 : (int)(b + total);
         }
-        int run = s_run;
-        if (h) {
-            int s = run + before + __popc(b & lanemask_lt());
-            seg_start[s] = i;
-            seg_cell[s] = keys[i];
+    }
+    __syncthreads();
+    if (s_tile < 0) return;
+    unsigned at = s_before + before;
+#pragma unroll
+    for (int k = 0; k < kSegItems; ++k) {
+        if ((heads[k] >> lane) & 1u) {
+            const unsigned s = at + __popc(heads[k] & lanemask_lt());
+            seg_start[s] = (int)(base + 32 * k + lane);
+            seg_key[s] = key[k];
         }
-        __syncthreads();
-        if (threadIdx.x == 0) s_run = run + total;
-        __syncthreads();
+        at += __popc(heads[k]);
     }
 }
 
@@ -632,10 +859,14 @@ __global__ void cell_finalize_corrected_kernel(const float4 *__restrict__ map, c
 // k_old = the slot count before the append.
 __global__ void append_mark_kernel(const uint32_t *__restrict__ new_keys, int k, const int32_t *__restrict__ slot_of,
                                    const GridMeta *__restrict__ meta, int *__restrict__ fresh,
-                                   int *__restrict__ k_old) {
+                                   int *__restrict__ k_old, const int *__restrict__ sort_err) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j == 0) *k_old = meta->occupied;
     if (j >= k) return;
+    if (*sort_err) {  // (a wait of the sort gave up: the keys are not sorted)
+        fresh[j] = 0;
+        return;
+    }
     const uint32_t key = new_keys[j];
     const bool first = j == 0 || new_keys[j - 1] != key;
     fresh[j] = (first && slot_of[key] < 0) ? 1 : 0;
@@ -649,10 +880,10 @@ __global__ void append_cells_kernel(const float4 *__restrict__ map, const uint32
                                     const uint32_t *__restrict__ keys, const uint32_t *__restrict__ order, int n,
                                     const int *__restrict__ fresh, const int *__restrict__ n_fresh,
                                     const int *__restrict__ k_old, int compat, int min_points, double eig_ratio,
-                                    GridMeta *__restrict__ meta, GridBuffers buf) {
+                                    GridMeta *__restrict__ meta, GridBuffers buf, const int *__restrict__ sort_err) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j == 0) meta->occupied = *k_old + *n_fresh;
-    if (j >= k) return;
+    if (j >= k || *sort_err) return;
     const uint32_t key = new_keys[j];
     if (j > 0 && new_keys[j - 1] == key) return;
     const int old_slot = buf.slot_of[key];
@@ -797,53 +1028,107 @@ int grid_windows(const GridMeta &meta_host, const int32_t *index, const float4 *
     return (int)cudaGetLastError();
 }
 
-int radix_sort_pairs(SortBuffers &b, int n, int bits, cudaStream_t st) {
-    const int nblk = div_up(n, kSortTile);
-    int nl = 0;
-    // digit width: passes = ceil(bits / 8), width = ceil(bits / passes).  (Wider
-    // digits save a pass but make the one-block histogram scan longer than the
-    // pass: 9-bit digits over 196 blocks were slower on a 400k-point map.)
-    int passes = (bits + 7) / 8;
-    int width = (bits + passes - 1) / passes;  // <= 8 <= log2(kMaxDigits)
-    int shift = 0;
-    for (int ps = 0; ps < passes; ++ps) {
-        int w = width;
-        if (shift + w > bits) w = bits - shift;
-        size_t smem_up = sizeof(int) << w;
-        size_t smem_dn = sizeof(int) * kWarps << w;
-        radix_upsweep_kernel<<<nblk, kThreads, smem_up, st>>>(b.k0, n, shift, w, b.hist);
-        nl += scan_exclusive(b.hist, nblk << w, nullptr, b.part, st);
-        radix_downsweep_kernel<<<nblk, kThreads, smem_dn, st>>>(b.k0, b.v0, b.k1, b.v1, n, shift, w, b.hist);
-        nl += 2;
+namespace {
+
+// Items per thread of the sort's tiles: up to 2^19 pairs small tiles spread
+// over more SMs (400k pairs: 98 tiles instead of 49), beyond that large ones
+// have fewer chained counts and longer runs to write.
+constexpr int kSmallSort = 1 << 19;
+int sort_items(int n) { return n <= kSmallSort ? 4 : 8; }
+int sort_tiles(int n) { return div_up(n, kSortThreads * sort_items(n)); }
+bool wide_state(int n) { return n >= (1 << 30); }  // counts beyond 30 bits
+
+// What must be zero before a sort, in one piece: tickets, error flag, digit
+// counts, the segment kernel's and the passes' chained counts.
+struct SortSync {
+    int *ticket;      // kMaxPasses + 1
+    int *err;
+    unsigned *hist;   // kMaxPasses x kDigits
+    uint64_t *seg;    // segment tiles
+    char *state;      // passes x tiles x kDigits words
+    size_t pass_bytes;
+};
+
+constexpr size_t kSyncHead = 256 + sizeof(unsigned) * kMaxPasses * kDigits;
+
+size_t sync_bytes(int n, int passes) {
+    return kSyncHead + sizeof(uint64_t) * (size_t)div_up(n, kSegTile) +
+           (size_t)passes * sort_tiles(n) * kDigits * (wide_state(n) ? 8 : 4);
+}
+
+SortSync sort_sync(void *sync, int n) {
+    char *p = (char *)sync;
+    SortSync s;
+    s.ticket = (int *)p;
+    s.err = s.ticket + kMaxPasses + 1;
+    s.hist = (unsigned *)(p + 256);
+    s.seg = (uint64_t *)(p + kSyncHead);
+    s.state = p + kSyncHead + sizeof(uint64_t) * (size_t)div_up(n, kSegTile);
+    s.pass_bytes = (size_t)sort_tiles(n) * kDigits * (wide_state(n) ? 8 : 4);
+    return s;
+}
+
+template <int ITEMS>
+constexpr size_t kPassSmem = sizeof(unsigned) * kSortWarps * kDigits + 2 * sizeof(uint32_t) * kSortThreads * ITEMS;
+
+template <int ITEMS, class S>
+cudaError_t prepare_pass() {
+    return cudaFuncSetAttribute(radix_pass_kernel<ITEMS, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)kPassSmem<ITEMS>);
+}
+
+template <int ITEMS, class S>
+void launch_pass(SortBuffers &b, const SortSync &y, int n, const RadixPlan &P, int pass, bool iota, uint32_t iota_base,
+                 cudaStream_t st) {
+    radix_pass_kernel<ITEMS, S><<<sort_tiles(n), kSortThreads, kPassSmem<ITEMS>, st>>>(
+        b.k0, iota ? nullptr : b.v0, iota_base, b.k1, b.v1, n, pass * P.width, pass_bits(P, pass),
+        y.hist + pass * kDigits, (S *)(y.state + (size_t)pass * y.pass_bytes), y.ticket + pass, y.err);
+}
+
+}  // namespace
+
+int prepare_sort() {
+    cudaError_t e = prepare_pass<4, uint32_t>();
+    if (e == cudaSuccess) e = prepare_pass<8, uint32_t>();
+    if (e == cudaSuccess) e = prepare_pass<8, uint64_t>();
+    return (int)e;
+}
+
+int radix_sort_pairs(SortBuffers &b, int n, int bits, cudaStream_t st, bool iota, uint32_t iota_base) {
+    const RadixPlan P = radix_plan(bits);
+    const SortSync y = sort_sync(b.sync, n);
+    cudaMemsetAsync(b.sync, 0, sync_bytes(n, P.passes), st);
+    const int blocks = div_up(n, kThreads * 8);
+    radix_hist_kernel<<<blocks < 1184 ? blocks : 1184, kThreads, 0, st>>>(b.k0, n, P, y.hist);
+    for (int ps = 0; ps < P.passes; ++ps) {
+        const bool io = iota && ps == 0;
+        if (wide_state(n))
+            launch_pass<8, uint64_t>(b, y, n, P, ps, io, iota_base, st);
+        else if (sort_items(n) == 4)
+            launch_pass<4, uint32_t>(b, y, n, P, ps, io, iota_base, st);
+        else
+            launch_pass<8, uint32_t>(b, y, n, P, ps, io, iota_base, st);
         uint32_t *t = b.k0; b.k0 = b.k1; b.k1 = t;
         t = b.v0; b.v0 = b.v1; b.v1 = t;
-        shift += w;
     }
-    return nl;
+    return 1 + P.passes;
 }
 
-int segment_sorted(const uint32_t *keys, int n, int *segc, int *nseg, int *part, int32_t *seg_start,
-                   uint32_t *seg_key, cudaStream_t st) {
-    const int nblk = div_up(n, kSortTile);
-    seg_count_kernel<<<nblk, kThreads, 0, st>>>(keys, n, segc);
-    int nl = scan_exclusive(segc, nblk, nseg, part, st);
-    seg_write_kernel<<<nblk, kThreads, 0, st>>>(keys, n, segc, seg_start, seg_key);
-    return nl + 2;
+int sort_segments(SortBuffers &b, int n, int bits, int32_t *seg_start, uint32_t *seg_key, cudaStream_t st, bool iota) {
+    const int nl = radix_sort_pairs(b, n, bits, st, iota, 0u);
+    const SortSync y = sort_sync(b.sync, n);
+    segment_kernel<<<div_up(n, kSegTile), kSegThreads, 0, st>>>(b.k0, n, seg_start, seg_key, b.nseg, y.seg,
+                                                             y.ticket + kMaxPasses, y.err);
+    return nl + 1;
 }
 
-int sort_segments(SortBuffers &b, int n, int bits, int32_t *seg_start, uint32_t *seg_key, cudaStream_t st) {
-    int nl = radix_sort_pairs(b, n, bits, st);
-    return nl + segment_sorted(b.k0, n, b.segc, b.nseg, b.part, seg_start, seg_key, st);
-}
+int *sort_error(const SortBuffers &b, int n) { return sort_sync(b.sync, n).err; }
 
 size_t sort_scratch_bytes(int n) {
-    const size_t nblk = (size_t)div_up(n, kSortTile);
-    return 4 * sizeof(uint32_t) * (size_t)n + sizeof(int) * kMaxDigits * nblk + sizeof(int) * (nblk + 1) +
-           sizeof(int) * scan_part_ints((size_t)kMaxDigits * nblk) + 8 * 256;
+    return 4 * sizeof(uint32_t) * (size_t)n + sync_bytes(n, kMaxPasses) + 8 * 256;
 }
 
 SortBuffers sort_buffers(void *scratch, int n) {
-    const size_t nblk = (size_t)div_up(n, kSortTile);
     char *p = (char *)scratch;
     auto take = [&](size_t bytes) {
         char *r = p;
@@ -855,10 +1140,8 @@ SortBuffers sort_buffers(void *scratch, int n) {
     b.v0 = (uint32_t *)take(sizeof(uint32_t) * (size_t)n);
     b.k1 = (uint32_t *)take(sizeof(uint32_t) * (size_t)n);
     b.v1 = (uint32_t *)take(sizeof(uint32_t) * (size_t)n);
-    b.hist = (int *)take(sizeof(int) * (size_t)kMaxDigits * nblk);
-    b.segc = (int *)take(sizeof(int) * (nblk + 1));
     b.nseg = (int *)take(sizeof(int));
-    b.part = (int *)take(sizeof(int) * scan_part_ints((size_t)kMaxDigits * nblk));
+    b.sync = take(sync_bytes(n, kMaxPasses));
     return b;
 }
 
@@ -891,9 +1174,9 @@ int grid_build(const float4 *d_map, int m, const GridMeta &meta_host, GridMeta *
 
     cudaMemsetAsync(buf.index, 0xff, sizeof(int32_t) * (size_t)meta_host.G, st);
     cudaMemsetAsync(buf.slot_of, 0xff, sizeof(int32_t) * (size_t)meta_host.G, st);
-    cell_key_kernel<<<div_up(m, kThreads), kThreads, 0, st>>>(d_map, m, d_meta, sb.k0, sb.v0);
+    cell_key_kernel<<<div_up(m, kThreads), kThreads, 0, st>>>(d_map, m, d_meta, sb.k0);
     ++nl;
-    nl += sort_segments(sb, m, key_bits(meta_host), buf.seg_start, buf.seg_cell, st);
+    nl += sort_segments(sb, m, key_bits(meta_host), buf.seg_start, buf.seg_cell, st, true);
     nl += grid_finalize(d_map, sb.v0, m, sb.nseg, d_meta, opt, buf, st);
     if (sorted) {
         sorted->keys = sb.k0;
@@ -923,18 +1206,20 @@ int grid_append(const float4 *d_map, int m_old, int k, const GridMeta &meta_host
     int *part = (int *)take(sizeof(int) * scan_part_ints((size_t)k));
     int nl = 0;
     // the new points' keys (point indices m_old ...), stably sorted
-    cell_key_kernel<<<div_up(k, kThreads), kThreads, 0, st>>>(d_map + m_old, k, d_meta, sb.k0, sb.v0, m_old);
+    cell_key_kernel<<<div_up(k, kThreads), kThreads, 0, st>>>(d_map + m_old, k, d_meta, sb.k0);
     ++nl;
-    nl += radix_sort_pairs(sb, k, key_bits(meta_host), st);
+    nl += radix_sort_pairs(sb, k, key_bits(meta_host), st, true, (uint32_t)m_old);
     // merged with the map's sorted pairs: the stable sort of all n points
     merge_kernel<<<div_up(n, kThreads), kThreads, 0, st>>>(old_sorted.keys, old_sorted.order, m_old, sb.k0, sb.v0,
-                                                           k, keys_out, order_out);
+                                                           k, keys_out, order_out, sort_error(sb, k));
     // the touched cells: new slots in key order, records from all their points
-    append_mark_kernel<<<div_up(k, kThreads), kThreads, 0, st>>>(sb.k0, k, buf.slot_of, d_meta, fresh, small + 1);
+    append_mark_kernel<<<div_up(k, kThreads), kThreads, 0, st>>>(sb.k0, k, buf.slot_of, d_meta, fresh, small + 1,
+                                                             sort_error(sb, k));
     nl += 2;
     nl += scan_exclusive(fresh, k, small, part, st);
     append_cells_kernel<<<div_up(k, 128), 128, 0, st>>>(d_map, sb.k0, k, keys_out, order_out, n, fresh, small, small + 1,
-                                                        opt.compat, opt.min_points, opt.eigen_ratio, d_meta, buf);
+                                                        opt.compat, opt.min_points, opt.eigen_ratio, d_meta, buf,
+                                                        sort_error(sb, k));
     ++nl;
     if (launches) *launches += nl;
     return (int)cudaGetLastError();

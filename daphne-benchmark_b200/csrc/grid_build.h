@@ -47,24 +47,26 @@ int64_t window_count(const GridMeta &g);  // W = (dim_x + 2)(dim_y + 2)(dim_z + 
 int grid_windows(const GridMeta &meta_host, const int32_t *index, const float4 *vox32, WindowBuffers wb,
                  cudaStream_t st, int *launches);
 
-// Stable LSD radix sort of n (key, value) pairs on the low `bits` key bits,
-// then the segments of equal keys: seg_start[s] = first sorted position of
-// segment s, seg_key[s] = its key, *b.nseg = segment count (device).  After
-// the call b.k0 / b.v0 hold the sorted keys and values.  Returns the number of
-// kernel launches.
+// Stable LSD radix sort of n > 0 (key, value) pairs on the low `bits` key
+// bits (iota: the values are iota_base, iota_base + 1, ... and b.v0 need not be
+// filled), then the segments of equal keys: seg_start[s] = first sorted
+// position of segment s, seg_key[s] = its key, *b.nseg = segment count
+// (device).  After the call b.k0 / b.v0 hold the sorted keys and values.
+// Returns the number of kernel launches.  *sort_error (device) is set when a
+// wait between tiles gave up; there are then no segments.
 struct SortBuffers {
     uint32_t *k0, *v0, *k1, *v1;
-    int *hist, *segc, *nseg, *part;
+    int *nseg;
+    void *sync;
 };
+// Per-device set-up (dynamic shared memory opt-in); call with the device current.
+int prepare_sort();
 size_t sort_scratch_bytes(int n);
 SortBuffers sort_buffers(void *scratch, int n);
-int sort_segments(SortBuffers &b, int n, int bits, int32_t *seg_start, uint32_t *seg_key, cudaStream_t st);
-// The two halves: the radix passes alone (b.k0 / b.v0 sorted afterwards), and
-// the segments of sorted keys (segc: ceil(n / 2048) + 1 ints, part: the
-// multi-block scan's tile sums).
-int radix_sort_pairs(SortBuffers &b, int n, int bits, cudaStream_t st);
-int segment_sorted(const uint32_t *keys, int n, int *segc, int *nseg, int *part, int32_t *seg_start,
-                   uint32_t *seg_key, cudaStream_t st);
+int sort_segments(SortBuffers &b, int n, int bits, int32_t *seg_start, uint32_t *seg_key, cudaStream_t st,
+                  bool iota = false);
+int radix_sort_pairs(SortBuffers &b, int n, int bits, cudaStream_t st, bool iota = false, uint32_t iota_base = 0);
+int *sort_error(const SortBuffers &b, int n);
 
 // The map's points sorted by dense cell (key) and, within a cell, by point
 // index: what the last build or append left, the input of the next append.

@@ -219,10 +219,10 @@ __global__ void __launch_bounds__(kRangeThreads) range_kernel(long long *__restr
 }
 
 // key = base[scan] + local leaf key (x fastest); non-finite points get the
-// key of the batch's end (sorted last, dropped); val = point index.
+// key of the batch's end (sorted last, dropped).
 __global__ void key_kernel(const float4 *__restrict__ pts, const int *__restrict__ offsets, int B, float r,
                            const ScanGeom *__restrict__ geom, const int *__restrict__ base, int total_keys, int n,
-                           uint32_t *__restrict__ keys, uint32_t *__restrict__ vals) {
+                           uint32_t *__restrict__ keys) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 p = pts[i];
@@ -234,15 +234,14 @@ __global__ void key_kernel(const float4 *__restrict__ pts, const int *__restrict
         k = (uint32_t)(base[b] + (int)(qx + g.d[0] * (qy + g.d[1] * qz)));
     }
     keys[i] = k;
-    vals[i] = (uint32_t)i;
 }
 
 // sorted[j] = pts[order[j]]: the points in key order (one thread per point,
 // so the random reads are all in flight at once; writes coalesced).
 __global__ void gather_kernel(const float4 *__restrict__ pts, const uint32_t *__restrict__ order, int n,
-                              float4 *__restrict__ sorted) {
+                              float4 *__restrict__ sorted, const int *__restrict__ sort_err) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < n) sorted[j] = pts[__ldg(order + j)];
+    if (j < n && !*sort_err) sorted[j] = pts[__ldg(order + j)];
 }
 
 // One thread per segment: the FP64 mean of its points in input order (the
@@ -327,6 +326,7 @@ int ndt_filter_create(int device, ndt_filter **out) {
     cudaError_t e = cudaSetDevice(device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&f->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMallocHost((void **)&f->h_flags, sizeof(int) * 4);
+    if (e == cudaSuccess) e = (cudaError_t)ndt::prepare_sort();
     if (e != cudaSuccess) {
         ndt_filter_destroy(f);
         return NDT_E_CUDA;
@@ -414,11 +414,12 @@ int ndt_voxel_filter_device(ndt_filter *f, int B, const float *d_points, const i
     ndt::SortBuffers sb = ndt::sort_buffers(f->sort_scratch.p, n);
     const unsigned pblk = (unsigned)((n + vf::kThreads - 1) / vf::kThreads);
     vf::key_kernel<<<pblk, vf::kThreads, 0, st>>>((const float4 *)d_points, d_offsets, B, r,
-                                                  (const vf::ScanGeom *)f->geom.p, base, total_keys, n, sb.k0, sb.v0);
+                                                  (const vf::ScanGeom *)f->geom.p, base, total_keys, n, sb.k0);
     FCK(cudaGetLastError());
-    ndt::sort_segments(sb, n, bits, (int32_t *)f->seg_start.p, (uint32_t *)f->seg_key.p, st);
+    ndt::sort_segments(sb, n, bits, (int32_t *)f->seg_start.p, (uint32_t *)f->seg_key.p, st, true);
     FCK(cudaGetLastError());
-    vf::gather_kernel<<<pblk, vf::kThreads, 0, st>>>((const float4 *)d_points, sb.v0, n, (float4 *)f->sorted.p);
+    vf::gather_kernel<<<pblk, vf::kThreads, 0, st>>>((const float4 *)d_points, sb.v0, n, (float4 *)f->sorted.p,
+                                                     ndt::sort_error(sb, n));
     vf::mean_kernel<<<pblk, vf::kThreads, 0, st>>>((const float4 *)f->sorted.p, (const int32_t *)f->seg_start.p,
                                                    (const uint32_t *)f->seg_key.p, sb.nseg, n, (uint32_t)total_keys,
                                                    (float4 *)d_out);
@@ -426,7 +427,12 @@ int ndt_voxel_filter_device(ndt_filter *f, int B, const float *d_points, const i
         (const uint32_t *)f->seg_key.p, sb.nseg, base, B, d_out_offsets);
     FCK(cudaGetLastError());
     FCK(cudaMemcpyAsync(f->h_flags + 2, d_out_offsets + B, sizeof(int), cudaMemcpyDeviceToHost, st));
+    FCK(cudaMemcpyAsync(f->h_flags + 3, ndt::sort_error(sb, n), sizeof(int), cudaMemcpyDeviceToHost, st));
     FCK(cudaStreamSynchronize(st));
+    if (f->h_flags[3]) {
+        f->msg = "a wait between the sort's tiles gave up";
+        return NDT_E_CUDA;
+    }
     *out_total = f->h_flags[2];
     return NDT_OK;
 }
