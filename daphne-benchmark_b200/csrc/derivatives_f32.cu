@@ -437,7 +437,7 @@ cudaError_t prepare_one() {
 template <int TILE, int MINB>
 void launch_one(const EvalArgs &args, int blocks, cudaStream_t st) {
     const size_t smem = sizeof(F32Smem<TILE / 32>);
-    const bool win = args.grid.win_off != nullptr;
+    const bool win = args.grid.win != nullptr;
     if (args.compat) {
         if (win)
             derivative_f32_kernel<TILE, MINB, true, true><<<blocks, TILE, smem, st>>>(args);

@@ -398,7 +398,7 @@ void launch_one(const EvalArgs &args, int sms, cudaStream_t st) {
     const size_t smem = sizeof(WideSmem);
     const long long want = (long long)(args.max_tiles < args.wide_chunks ? args.max_tiles : args.wide_chunks) * W;
     const int blocks = (int)(want < sms * kWideResident ? want : sms * kWideResident);
-    const bool win = args.grid.win_off != nullptr;
+    const bool win = args.grid.win != nullptr;
     if (args.compat) {
         if (win)
             derivative_wide_kernel<W, true, true><<<blocks, kBlock, smem, st>>>(args);

@@ -139,7 +139,7 @@ struct ndt_ctx {
     double d1 = 0, d2 = 0;
     // grid
     DevBuf map, index, slot_of, mean, vox32, icov64, count, cell, seg_start, seg_cell, scratch, meta;
-    DevBuf win_off, win_ent, win_ctot;
+    DevBuf win, win_ent, win_cursor;
     GridMeta meta_host{};
     bool have_map = false;
     bool have_windows = false;
@@ -271,7 +271,7 @@ GridDev grid_dev(ndt_ctx *c) {
     g.inv_res = c->inv_res;
     g.radius_final = (float)((double)c->prm.resolution + (double)0.001f);
     g.icov64 = c->icov64.as<double>();
-    g.win_off = c->have_windows ? c->win_off.as<int32_t>() : nullptr;
+    g.win = c->have_windows ? c->win.as<int2>() : nullptr;
     g.win_ent = c->have_windows ? c->win_ent.as<float4>() : nullptr;
     g.win_dim[0] = c->meta_host.dim[0] + 2;
     g.win_dim[1] = c->meta_host.dim[1] + 2;
@@ -292,12 +292,12 @@ int set_device(ndt_ctx *c) {
     return NDT_OK;
 }
 
-constexpr long long kMaxWindows = 1LL << 28;        // probe windows (4 B offset each)
+constexpr long long kMaxWindows = 1LL << 28;        // probe windows (8 B offset and count each)
 constexpr long long kMaxWindowEntries = 1LL << 28;  // window entries (16 B each)
 
 // Grid build from a device-resident map (any device pointer valid on the
 // context's stream for the duration of the call).
-// Probe-window table of the finished dense index: W + 1 offsets and at most
+// Probe-window table of the finished dense index: W offsets and counts and at most
 // 27 entries per usable voxel (skipped when it would not fit, or with
 // dense_probe set).  prepare_windows sizes the buffers (false: no table);
 // enqueue_windows launches the build.
@@ -308,12 +308,12 @@ int prepare_windows(ndt_ctx *c, int m, bool &use, WindowBuffers &wb) {
     use = !c->prm.dense_probe && W < kMaxWindows && ent_cap < kMaxWindowEntries;
     std::memset(&wb, 0, sizeof(wb));
     if (!use) return NDT_OK;
-    CK(c->win_off.ensure(sizeof(int32_t) * (size_t)(W + 1)));
+    CK(c->win.ensure(sizeof(int2) * (size_t)W));
     CK(c->win_ent.ensure(sizeof(float4) * (size_t)ent_cap));
-    CK(c->win_ctot.ensure(sizeof(int32_t) * (size_t)(W / 256 + 2)));
-    wb.off = c->win_off.as<int32_t>();
+    CK(c->win_cursor.ensure(sizeof(int32_t)));
+    wb.win = c->win.as<int2>();
     wb.ent = c->win_ent.as<float4>();
-    wb.ctot = c->win_ctot.as<int32_t>();
+    wb.cursor = c->win_cursor.as<int32_t>();
     return NDT_OK;
 }
 
@@ -1084,7 +1084,7 @@ void ndt_destroy(ndt_ctx *c) {
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     if (c->copy_stream) cudaStreamSynchronize(c->copy_stream);
-    DevBuf *bufs[] = {&c->win_off, &c->win_ent, &c->win_ctot, &c->map, &c->index, &c->mean, &c->vox32,
+    DevBuf *bufs[] = {&c->win, &c->win_ent, &c->win_cursor, &c->map, &c->index, &c->mean, &c->vox32,
                       &c->icov64, &c->count, &c->cell, &c->seg_start, &c->seg_cell,
                       &c->scratch, &c->meta, &c->points, &c->offsets, &c->guesses, &c->states,
                       &c->tiles, &c->tile_begin, &c->num_tiles, &c->chunks, &c->chunk_begin, &c->num_chunks,
@@ -1480,7 +1480,7 @@ int ndt_window_info(ndt_ctx *c, long long *windows, long long *entries) {
     if (c->have_windows) {
         W = (long long)window_count(c->meta_host);
         int32_t e = 0;
-        CK(cudaMemcpyAsync(&e, c->win_off.as<int32_t>() + W, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaMemcpyAsync(&e, c->win_cursor.p, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
         E = e;
     }

@@ -33,12 +33,12 @@ struct NdtGridOptions {
 // consecutive cells).  Window w of base cell b, each component in
 // [-2, dim - 1], lists the usable voxels of those 27 cells in the reference's
 // probe order (z outer, x inner) as float4 {float(mean) xyz, code}, code =
-// slot << 6 | flag << 5 | 9 dz + 3 dy + dx, so a point reads 2 offsets and one
-// record per occupied cell instead of 27 dense-index entries.
+// slot << 6 | flag << 5 | 9 dz + 3 dy + dx, so a point reads its window's offset
+// and count and one record per occupied cell instead of 27 dense-index entries.
 struct WindowBuffers {
-    int32_t *off;   // W + 1 entry offsets
-    float4 *ent;    // entries (capacity 27 * min(m, G))
-    int32_t *ctot;  // per-block totals (ceil(W / 256) + 1)
+    int2 *win;      // W: first entry and number of entries of each window
+    float4 *ent;    // entries (capacity 27 * min(m, G)), in any order of the windows
+    int32_t *cursor;  // entries in the table
 };
 
 int64_t window_count(const GridMeta &g);  // W = (dim_x + 2)(dim_y + 2)(dim_z + 2)

@@ -71,7 +71,7 @@ struct GridDev {
     float radius_final;      // (float)(res + 0.001f): the probe loop bound of kernel.cpp:254
     const double *icov64;    // 9K: inverse covariance as the reference stores it (row major)
     // probe-window table (grid_build.h), nullptr when not built
-    const int32_t *win_off;  // W + 1
+    const int2 *win;         // W: first entry, number of entries
     const float4 *win_ent;   // {float(mean) xyz, slot << 6 | flag << 5 | cell offset}
     int32_t win_dim[2];      // dim_x + 2, dim_y + 2
 };

@@ -182,7 +182,7 @@ constexpr int kProbeAll = kProbeWindows | kProbeDenseIndex;
 // probes are done, or, on the generic path (trip counts up to 4: coordinates
 // beyond ~1e6 m or inf), the probe position to continue from once the caller
 // has emptied the sink.  Three paths, chosen per warp:
-//   windows  the probe-window table (2 offsets + 1 record per occupied cell),
+//   windows  the probe-window table (1 offset and count + 1 record per occupied cell),
 //            when the table exists and every lane's cells are consecutive;
 //   dense    the 27 dense-index entries in 3 layers of 9 loads, skipping with
 //            warp-uniform branches the layers and rows no lane has in bounds
@@ -211,7 +211,7 @@ __device__ __forceinline__ void collect_pairs(const GridDev &grid, float px, flo
               mz = __reduce_max_sync(kFull, az.n);
     const float tol = radius_margin(px, py, pz, res);
     const bool small = mx <= 3 && my <= 3 && mz <= 3;
-    if ((kPaths & kProbeWindows) && small && grid.win_off) {
+    if ((kPaths & kProbeWindows) && small && grid.win) {
         bool ok = true;
         const int bx = window_base(ax, g.dim[0], ok);
         const int by = window_base(ay, g.dim[1], ok);
@@ -226,8 +226,9 @@ __device__ __forceinline__ void collect_pairs(const GridDev &grid, float px, flo
                     for (int dy = 0; dy < 3; ++dy)
                         if ((az.in >> dz) & (ay.in >> dy) & 1u) allowed |= ax.in << (9 * dz + 3 * dy);
                 const int w = (bx + 2) + grid.win_dim[0] * ((by + 2) + grid.win_dim[1] * (bz + 2));
-                beg = __ldg(grid.win_off + w);
-                cnt = __ldg(grid.win_off + w + 1) - beg;
+                const int2 o = __ldg(grid.win + w);
+                beg = o.x;
+                cnt = o.y;
                 n_probe += __popc(allowed);
             }
             const int maxc = __reduce_max_sync(kFull, cnt);
