@@ -62,11 +62,14 @@ struct ndt_mlp {
     int device = 0;
     cudaStream_t stream = nullptr;
     cudaStream_t own_stream = nullptr;  // created with the network; `stream` may be a caller's
-    float *w = nullptr, *m = nullptr, *v = nullptr, *grad = nullptr, *loss = nullptr;
+    float *w = nullptr, *m = nullptr, *v = nullptr, *grad = nullptr;  // grad: the gradient, then the loss
+    float *h_grad = nullptr;     // pinned: what a training step returns
+    float *w1 = nullptr;         // W1 and b1 as the last backward used them
     uint8_t *w2op = nullptr;
     int *err = nullptr;
     unsigned long long *gmax = nullptr;
     float *grad_scan = nullptr, *loss_scan = nullptr;
+    float4 *feat = nullptr;      // B x 128: the features of the points the max-pool routes gradients to
     float *dg = nullptr;         // B x 128: the head's gradient at the max-pooled features
     float *head_part = nullptr;  // per 128-scan tile: the head's weight and bias gradient sums
     size_t cap_b = 0;

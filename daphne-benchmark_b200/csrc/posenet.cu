@@ -21,7 +21,7 @@
 // max-pool routes the gradient of channel c of scan b to one point (its
 // argmax), so the shared layers' gradient touches at most 128 points per scan
 // with a different point per channel: a gather, not a GEMM, computed on CUDA
-// cores per scan (shared_bwd_kernel) with the same BF16 operands the forward
+// cores per scan (shared_bwd_kernel and reduce_adam_kernel) with the same BF16 operands the forward
 // used (h1 and W2 rounded to BF16).  Gradients are summed over the batch in a
 // fixed order (deterministic) and applied with Adam to FP32 master weights; W2
 // is then re-packed to BF16.
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(128, 1) point_kernel(const __grid_constant__ P
 // D4 192, D5 320, D6 448), one elected thread issues the MMAs.  Bias
 // gradients are summed over the tile's rows in a fixed order.
 constexpr int kOutPad = 16;
-constexpr int kHeadPart = kNumW;  // per-CTA partial: the head's weights and biases at their blob offsets
+constexpr int kHeadPart = (kNumW + 3) & ~3;  // per-CTA partial: the head's weights and biases at their blob offsets
 
 // Byte offset of element (r, k) in a K-major interleaved operand with K columns.
 __host__ __device__ __forceinline__ uint32_t opk(int r, int k, int K) {
@@ -316,10 +316,18 @@ struct HeadTcArgs {
 constexpr uint32_t hG = 0, hGt = hG + 32768, hW3 = hGt + 32768, hW3t = hW3 + 16384, hH3 = hW3t + 16384,
                    hH3t = hH3 + 16384, hW4 = hH3t + 16384, hW4t = hW4 + 2048, hDY = hW4t + 2048, hDYt = hDY + 4096,
                    hDH3 = hDYt + 32768, hDH3t = hDH3 + 16384, hBar = hDH3t + 32768, hTmem = hBar + 8,
-                   kHeadSmem = hTmem + 8;
+                   hMask = hTmem + 8, kHeadSmem = hMask + 128 * 4 * 4;
 
 __device__ __forceinline__ void st_bf16(uint8_t *base, uint32_t off, float v) {
     *reinterpret_cast<__nv_bfloat16 *>(base + off) = __float2bfloat16_rn(v);
+}
+
+// Eight values as one 16-byte row piece of an operand.
+__device__ __forceinline__ void st_bf16x8(uint8_t *base, uint32_t off, const float *v) {
+    __align__(16) __nv_bfloat16 h[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) h[e] = __float2bfloat16_rn(v[e]);
+    *reinterpret_cast<uint4 *>(base + off) = *reinterpret_cast<const uint4 *>(h);
 }
 
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint32_t a_smem, uint32_t b_smem, int K_a, int K_b,
@@ -413,26 +421,45 @@ __global__ void __launch_bounds__(128, 1) head_tc_kernel(const __grid_constant__
             *reinterpret_cast<uint4 *>(sm + o) = make_uint4(0, 0, 0, 0);
         }
     }
-    for (int i = tid; i < kH3 * kH2; i += 128) {  // W3 (64 x 128) and its transpose
-        const int j = i / kH2, c = i % kH2;
-        const float v = w[oW3 + i];
-        st_bf16(sm, hW3 + opk(j, c, kH2), v);
-        st_bf16(sm, hW3t + opk(c, j, kH3), v);
+    // Global reads are coalesced, thread tid taking channel tid of 8 rows at a
+    // time (a thread reading its own row of G, 128 dependent 8-byte reads, was
+    // most of the kernel's time); 8 rows of a channel are one 16-byte piece of
+    // the transposed operand.
+#pragma unroll 2
+    for (int j0 = 0; j0 < kH3; j0 += 8) {  // W3 (64 x 128) and its transpose
+        float v[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = w[oW3 + (j0 + e) * kH2 + tid];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) st_bf16(sm, hW3 + opk(j0 + e, tid, kH2), v[e]);
+        if (train) st_bf16x8(sm, hW3t + opk(tid, j0, kH3), v);
     }
     for (int i = tid; i < kOutPad * kH3; i += 128) {  // W4 (6 x 64) padded to 16 rows, and its transpose
         const int o = i / kH3, j = i % kH3;
         const float v = o < kOut ? w[oW4 + o * kH3 + j] : 0.0f;
         st_bf16(sm, hW4 + opk(o, j, kH3), v);
-        st_bf16(sm, hW4t + opk(j, o, kOutPad), v);
+        if (train) st_bf16(sm, hW4t + opk(j, o, kOutPad), v);
     }
-    float g[kH2];
+    uint32_t *mask = reinterpret_cast<uint32_t *>(sm + hMask);  // [row][channel / 32]: G > 0
     {
-        const unsigned long long *gm = a.gmax + (size_t)(valid ? b : 0) * kH2;
-#pragma unroll 4
-        for (int c = 0; c < kH2; ++c) {
-            g[c] = valid ? __uint_as_float((unsigned)(gm[c] >> 32)) : 0.0f;
-            st_bf16(sm, hG + opk(tid, c, kH2), g[c]);
-            st_bf16(sm, hGt + opk(c, tid, 128), g[c]);
+        const int rows = min(128, a.B - (int)blockIdx.x * 128);
+        const unsigned long long *gm = a.gmax + (size_t)blockIdx.x * 128 * kH2 + tid;
+#pragma unroll 2
+        for (int r0 = 0; r0 < 128; r0 += 8) {
+            float g[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                g[e] = r0 + e < rows ? __uint_as_float((unsigned)(gm[(size_t)(r0 + e) * kH2] >> 32)) : 0.0f;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) st_bf16(sm, hG + opk(r0 + e, tid, kH2), g[e]);
+            if (train) {
+                st_bf16x8(sm, hGt + opk(tid, r0, 128), g);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const unsigned m = __ballot_sync(0xffffffffu, g[e] > 0.0f);
+                    if ((tid & 31) == 0) mask[(r0 + e) * 4 + warp] = m;
+                }
+            }
         }
     }
     if (tid == 0) {
@@ -463,9 +490,10 @@ __global__ void __launch_bounds__(128, 1) head_tc_kernel(const __grid_constant__
 #pragma unroll
         for (int j = 0; j < kH3; ++j) {
             h3[j] = valid ? fmaxf(h3[j] + w[oB3 + j], 0.0f) : 0.0f;
-            st_bf16(sm, hH3 + opk(tid, j, kH3), h3[j]);
-            st_bf16(sm, hH3t + opk(j, tid, 128), h3[j]);
+            if (train) st_bf16(sm, hH3t + opk(j, tid, 128), h3[j]);
         }
+#pragma unroll
+        for (int j0 = 0; j0 < kH3; j0 += 8) st_bf16x8(sm, hH3 + opk(tid, j0, kH3), h3 + j0);
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -526,9 +554,10 @@ __global__ void __launch_bounds__(128, 1) head_tc_kernel(const __grid_constant__
 #pragma unroll
         for (int j = 0; j < kH3; ++j) {
             dh3[j] = h3[j] > 0.0f ? dh3[j] : 0.0f;
-            st_bf16(sm, hDH3 + opk(tid, j, kH3), dh3[j]);
             st_bf16(sm, hDH3t + opk(j, tid, 128), dh3[j]);
         }
+#pragma unroll
+        for (int j0 = 0; j0 < kH3; j0 += 8) st_bf16x8(sm, hDH3 + opk(tid, j0, kH3), dh3 + j0);
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -548,13 +577,23 @@ __global__ void __launch_bounds__(128, 1) head_tc_kernel(const __grid_constant__
     if (!failed) {
         float d4[kH2];
         tmem_row<kH2>(tmem, warp, 192, d4);
-        if (valid)
-            for (int c = 0; c < kH2; ++c) a.dg[(size_t)b * kH2 + c] = g[c] > 0.0f ? d4[c] : 0.0f;
+        if (valid) {
+            const uint32_t m[4] = {mask[tid * 4], mask[tid * 4 + 1], mask[tid * 4 + 2], mask[tid * 4 + 3]};
+            float4 *dg = reinterpret_cast<float4 *>(a.dg + (size_t)b * kH2);
+#pragma unroll
+            for (int c = 0; c < kH2; c += 4) {
+                const uint32_t q = m[c >> 5] >> (c & 31);
+                dg[c / 4] = make_float4(q & 1u ? d4[c] : 0.0f, q & 2u ? d4[c + 1] : 0.0f, q & 4u ? d4[c + 2] : 0.0f,
+                                        q & 8u ? d4[c + 3] : 0.0f);
+            }
+        }
         float *part = a.head_part + (size_t)blockIdx.x * kHeadPart;
         if (warp < 2) {  // rows 0..63 of D5: dW3
             float r[kH2];
             tmem_row<kH2>(tmem, warp, 320, r);
-            for (int c = 0; c < kH2; ++c) part[oW3 + tid * kH2 + c] = r[c];
+            float4 *out = reinterpret_cast<float4 *>(part + oW3 + tid * kH2);
+#pragma unroll
+            for (int c = 0; c < kH2; c += 4) out[c / 4] = make_float4(r[c], r[c + 1], r[c + 2], r[c + 3]);
         }
         if (warp == 0) {  // rows 0..5 of D6: dW4
             float r[kH3];
@@ -582,12 +621,18 @@ __global__ void __launch_bounds__(128, 1) head_tc_kernel(const __grid_constant__
     }
 }
 
-// The shared layers' gradient of one scan (one CTA of 128 threads): the
-// max-pool routes channel c's gradient dg[c] to one point (its argmax), so
-// this is a gather over at most 128 points, with the BF16 operands of the
-// forward (h1 and W2 rounded to BF16):
+// The shared layers' gradient: the max-pool routes channel c's gradient dg[c]
+// of scan b to one point (its argmax), so this is a gather over at most 128
+// points per scan, with the BF16 operands of the forward (h1 and W2 rounded to
+// BF16):
 //   dW2[c][k] = dg[c] bf16(h1[p_c][k]),  db2[c] = dg[c],
 //   dz1[c][k] = dg[c] bf16(W2[c][k]) [z1[p_c][k] > 0],  dW1[k] = sum_c dz1[c][k] u[p_c],  db1[k] = sum_c dz1[c][k].
+// One CTA of 128 threads per scan gathers the points' features once (u and dg
+// of every channel, 2 KB per scan) and sums up dW1 and db1; dW2 is summed over
+// the scans from the same features in reduce_adam_kernel, so the scans' dW2
+// (33 KB each) never exist.
+constexpr int kScanPart = oW2;  // dW1 and db1 of one scan, at their blob offsets
+
 struct SharedBwdArgs {
     const float4 *points;
     const int *offsets;
@@ -595,7 +640,9 @@ struct SharedBwdArgs {
     const float *w;
     const unsigned long long *gmax;
     const float *dg;     // B x 128
-    float *grad_scan;    // B x kNumW (the shared layers' entries)
+    float4 *feat;        // B x 128 out: the routed point's features and the channel's gradient
+    float *grad_scan;    // B x kScanPart out
+    float *w1;           // kScanPart out: W1 and b1 as the backward used them
     Norm nm;
     int B;
     int max_points;
@@ -604,87 +651,145 @@ struct SharedBwdArgs {
 __device__ __forceinline__ float bf16r(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
 __global__ void __launch_bounds__(128) shared_bwd_kernel(const __grid_constant__ SharedBwdArgs a) {
-    __shared__ float dgs[kH2];
-    __shared__ int arg[kH2];
+    __shared__ float4 s_f[kH2];
     __shared__ float sT[12];
     const int tid = threadIdx.x, b = blockIdx.x;
     if (b >= a.B) return;
     const float *w = a.w;
-    {
-        const unsigned long long m = a.gmax[(size_t)b * kH2 + tid];
-        arg[tid] = (int)(0xffffffffu - (unsigned)(m & 0xffffffffu));
-        dgs[tid] = a.dg[(size_t)b * kH2 + tid];
-    }
     if (tid < 12) sT[tid] = a.guesses[16 * (size_t)b + tid];
+    const unsigned long long m = a.gmax[(size_t)b * kH2 + tid];
+    const float d = a.dg[(size_t)b * kH2 + tid];
+    if (b == 0)
+        for (int i = tid; i < kScanPart; i += 128) a.w1[i] = w[oW1 + i];
     __syncthreads();
-    float *G = a.grad_scan + (size_t)b * kNumW;
     const int start = a.offsets[b], n = a.offsets[b + 1] - start;
     const int P = n < a.max_points ? n : a.max_points;
     {
-        const int c = tid;
-        const float d = dgs[c];
         float u[3] = {0.f, 0.f, 0.f};
-        if (d != 0.0f && P > 0) point_feature(sT, a.points[start + sample_index(arg[c], P, n)], a.nm, u);
-        for (int k = 0; k < kH1; ++k) {
-            const float v = fmaf(w[oW1 + 3 * k], u[0], fmaf(w[oW1 + 3 * k + 1], u[1], fmaf(w[oW1 + 3 * k + 2], u[2],
-                                                                                            w[oB1 + k])));
-            G[oW2 + c * kH1 + k] = d * bf16r(fmaxf(v, 0.0f));
-        }
-        G[oB2 + c] = d;
+        const int arg = (int)(0xffffffffu - (unsigned)(m & 0xffffffffu));
+        if (d != 0.0f && P > 0) point_feature(sT, a.points[start + sample_index(arg, P, n)], a.nm, u);
+        s_f[tid] = a.feat[(size_t)b * kH2 + tid] = make_float4(u[0], u[1], u[2], d);
     }
-    if (tid < kH1) {
-        const int k = tid;
-        float gw0 = 0.f, gw1 = 0.f, gw2 = 0.f, gb = 0.f;
-        for (int c = 0; c < kH2; ++c) {
-            const float d = dgs[c];
-            if (d == 0.0f) continue;
-            float u[3];
-            point_feature(sT, a.points[start + sample_index(arg[c], P, n)], a.nm, u);
-            const float z = fmaf(w[oW1 + 3 * k], u[0], fmaf(w[oW1 + 3 * k + 1], u[1], fmaf(w[oW1 + 3 * k + 2], u[2],
-                                                                                            w[oB1 + k])));
-            if (!(z > 0.0f)) continue;
-            const float dz = bf16r(w[oW2 + c * kH1 + k]) * d;
-            gw0 = fmaf(dz, u[0], gw0);
-            gw1 = fmaf(dz, u[1], gw1);
-            gw2 = fmaf(dz, u[2], gw2);
-            gb += dz;
+    __syncthreads();
+    // thread (k, h): unit k of layer 1; h = 0 sums dW1[k][0..1], h = 1 dW1[k][2] and db1[k]
+    const int k = tid & (kH1 - 1), h = tid / kH1;
+    const float w0 = w[oW1 + 3 * k], w1 = w[oW1 + 3 * k + 1], w2 = w[oW1 + 3 * k + 2], b1 = w[oB1 + k];
+    float g0 = 0.f, g1 = 0.f;
+    for (int c0 = 0; c0 < kH2; c0 += 32) {
+        float wc[32];  // (32 loads in flight)
+#pragma unroll
+        for (int u = 0; u < 32; ++u) wc[u] = w[oW2 + (c0 + u) * kH1 + k];
+#pragma unroll
+        for (int u = 0; u < 32; ++u) {
+            const float4 f = s_f[c0 + u];
+            const float z = fmaf(w0, f.x, fmaf(w1, f.y, fmaf(w2, f.z, b1)));
+            // (selects, not branches: the channels' chains overlap)
+            const bool on = f.w != 0.0f && z > 0.0f;
+            const float dz = on ? bf16r(wc[u]) * f.w : 0.0f;
+            const float p = on ? (h == 0 ? f.x : f.z) : 0.0f, q = on ? (h == 0 ? f.y : 1.0f) : 0.0f;
+            g0 = fmaf(dz, p, g0);
+            g1 = fmaf(dz, q, g1);
         }
-        G[oW1 + 3 * k] = gw0;
-        G[oW1 + 3 * k + 1] = gw1;
-        G[oW1 + 3 * k + 2] = gw2;
-        G[oB1 + k] = gb;
+    }
+    float *G = a.grad_scan + (size_t)b * kScanPart;
+    if (h == 0) {
+        G[oW1 + 3 * k] = g0;
+        G[oW1 + 3 * k + 1] = g1;
+    } else {
+        G[oW1 + 3 * k + 2] = g0;
+        G[oB1 + k] = g1;
     }
 }
 
-// Batch gradient (mean over the scans: the shared layers' per-scan gradients
-// in scan order, the head's per-tile sums in tile order) and loss; optionally
-// an Adam step on the FP32 weights.
+// Batch gradient (mean over the scans: the shared layers' gradients summed in
+// scan order, the head's per-tile sums in tile order) and loss; optionally an
+// Adam step on the FP32 weights, W2's BF16 operand with it.  Blocks of 64
+// weights, so that a block of W2 is one channel's row; the last block sums the
+// loss.
 struct AdamArgs {
     float *w, *m, *v;
-    const float *grad_scan;  // B x kNumW: the shared layers' entries (W1, b1, W2, b2)
-    const float *head_part;  // parts x kNumW: the head's entries (W3, b3, W4, b4), summed over 128 scans each
+    const float *grad_scan;  // B x kScanPart
+    const float4 *feat;      // B x 128
+    const float *w1;         // W1 and b1 as the backward used them (this kernel updates them)
+    const float *head_part;  // parts x kHeadPart: the head's entries (W3, b3, W4, b4), summed over 128 scans each
     int parts;
     const float *loss_scan;
-    float *grad;   // kNumW out (batch gradient)
-    float *loss;   // 1 out
+    float *grad;   // kNumW out (batch gradient), then the loss
+    uint8_t *w2op;
     int B;
     float lr, beta1, beta2, eps, bc1, bc2;  // bc = 1 - beta^t
     int update;
 };
 
-__global__ void reduce_adam_kernel(const __grid_constant__ AdamArgs a) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) {
-        float l = 0.f;
-        for (int b = 0; b < a.B; ++b) l += a.loss_scan[b];
-        *a.loss = l / a.B;
+constexpr int kAdamBlock = 64, kAdamBlocks = (kNumW + kAdamBlock - 1) / kAdamBlock;
+static_assert(oW2 % kAdamBlock == 0 && oB2 % kAdamBlock == 0 && oW3 % kAdamBlock == 0 && kH1 == kAdamBlock,
+              "a block of W2 is one channel's row, and no block straddles two layers");
+
+// Sum over b < n, in order, of f(row b): the rows come through shared memory,
+// kRows at a time (their latency is the sum's time otherwise: 21 us for 256
+// scans with the loads in the loop, XXX us as here).
+template <class T, class Load, class F>
+__device__ __forceinline__ float ordered_sum(int n, T *s_row, Load load, F f) {
+    constexpr int kRows = 256;
+    float s = 0.f;
+    for (int b0 = 0; b0 < n; b0 += kRows) {
+        const int m = min(kRows, n - b0);
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kRows / kAdamBlock; ++k) {
+            const int r = k * kAdamBlock + threadIdx.x;
+            if (r < m) s_row[r] = load(b0 + r);
+        }
+        __syncthreads();
+#pragma unroll 8
+        for (int r = 0; r < m; ++r) s += f(s_row[r]);
+    }
+    return s;
+}
+
+__global__ void __launch_bounds__(kAdamBlock) reduce_adam_kernel(const __grid_constant__ AdamArgs a) {
+    __shared__ float4 s_row[256];
+    float *s_val = reinterpret_cast<float *>(s_row);
+    if (blockIdx.x == kAdamBlocks) {
+        const float l = ordered_sum(a.B, s_val, [&](int b) { return a.loss_scan[b]; }, [](float x) { return x; });
+        if (threadIdx.x == 0) a.grad[kNumW] = l / a.B;
+        return;
+    }
+    const int i = blockIdx.x * kAdamBlock + threadIdx.x;
+    float s = 0.f;
+    if (blockIdx.x < oW2 / kAdamBlock) {
+        int b = 0;
+        for (; b + 32 <= a.B; b += 32) {  // (32 loads in flight)
+            float t[32];
+#pragma unroll
+            for (int u = 0; u < 32; ++u) t[u] = a.grad_scan[(size_t)(b + u) * kScanPart + i];
+#pragma unroll
+            for (int u = 0; u < 32; ++u) s += t[u];
+        }
+        for (; b < a.B; ++b) s += a.grad_scan[(size_t)b * kScanPart + i];
+    } else if (blockIdx.x < oB2 / kAdamBlock) {  // (every thread of the block: channel c)
+        const int c = (i - oW2) / kH1, k = (i - oW2) % kH1;
+        const float w0 = a.w1[oW1 + 3 * k], w1 = a.w1[oW1 + 3 * k + 1], w2 = a.w1[oW1 + 3 * k + 2], b1 = a.w1[oB1 + k];
+        s = ordered_sum(
+            a.B, s_row, [&](int b) { return a.feat[(size_t)b * kH2 + c]; },
+            [&](float4 f) {
+                const float v = fmaf(w0, f.x, fmaf(w1, f.y, fmaf(w2, f.z, b1)));
+                return f.w * bf16r(fmaxf(v, 0.0f));
+            });
+    } else if (blockIdx.x < oW3 / kAdamBlock) {
+        int b = 0;
+        for (; b + 32 <= a.B; b += 32) {
+            float t[32];
+#pragma unroll
+            for (int u = 0; u < 32; ++u) t[u] = a.feat[(size_t)(b + u) * kH2 + (i - oB2)].w;
+#pragma unroll
+            for (int u = 0; u < 32; ++u) s += t[u];
+        }
+        for (; b < a.B; ++b) s += a.feat[(size_t)b * kH2 + (i - oB2)].w;
+    } else if (i < kNumW) {
+        for (int t = 0; t < a.parts; ++t) s += a.head_part[(size_t)t * kHeadPart + i];
     }
     if (i >= kNumW) return;
-    float s = 0.f;
-    if (i < oW3)
-        for (int b = 0; b < a.B; ++b) s += a.grad_scan[(size_t)b * kNumW + i];
-    else
-        for (int t = 0; t < a.parts; ++t) s += a.head_part[(size_t)t * kNumW + i];
     const float gi = s / a.B;
     a.grad[i] = gi;
     if (!a.update) return;
@@ -692,7 +797,11 @@ __global__ void reduce_adam_kernel(const __grid_constant__ AdamArgs a) {
     const float v = a.beta2 * a.v[i] + (1.0f - a.beta2) * gi * gi;
     a.m[i] = m;
     a.v[i] = v;
-    a.w[i] -= a.lr * (m / a.bc1) / (sqrtf(v / a.bc2) + a.eps);
+    const float x = a.w[i] - a.lr * (m / a.bc1) / (sqrtf(v / a.bc2) + a.eps);
+    a.w[i] = x;
+    if (i >= oW2 && i < oB2)
+        *reinterpret_cast<__nv_bfloat16 *>(a.w2op + op_offset((i - oW2) / kH1, (i - oW2) % kH1)) =
+            __float2bfloat16_rn(x);
 }
 
 // proposal = T(pose(guess) + y * dscale)
@@ -747,11 +856,14 @@ int ensure_batch(ndt_mlp *c, int B) {
     cudaFree(c->loss_scan);
     cudaFree(c->dg);
     cudaFree(c->head_part);
+    cudaFree(c->feat);
+    c->feat = nullptr;
     c->gmax = nullptr;
     c->grad_scan = c->loss_scan = c->dg = c->head_part = nullptr;
     c->cap_b = 0;
     MCK(cudaMalloc(&c->gmax, sizeof(unsigned long long) * pn::kH2 * (size_t)B));
-    MCK(cudaMalloc(&c->grad_scan, sizeof(float) * pn::kNumW * (size_t)B));
+    MCK(cudaMalloc(&c->grad_scan, sizeof(float) * pn::kScanPart * (size_t)B));
+    MCK(cudaMalloc(&c->feat, sizeof(float4) * pn::kH2 * (size_t)B));
     MCK(cudaMalloc(&c->loss_scan, sizeof(float) * (size_t)B));
     MCK(cudaMalloc(&c->dg, sizeof(float) * pn::kH2 * (size_t)B));
     MCK(cudaMalloc(&c->head_part, sizeof(float) * pn::kHeadPart * (size_t)((B + 127) / 128)));
@@ -816,8 +928,9 @@ int ndt_mlp_create(int device, ndt_mlp **out) {
     if (e == cudaSuccess) e = cudaMalloc(&c->w, sizeof(float) * pn::kNumW);
     if (e == cudaSuccess) e = cudaMalloc(&c->m, sizeof(float) * pn::kNumW);
     if (e == cudaSuccess) e = cudaMalloc(&c->v, sizeof(float) * pn::kNumW);
-    if (e == cudaSuccess) e = cudaMalloc(&c->grad, sizeof(float) * pn::kNumW);
-    if (e == cudaSuccess) e = cudaMalloc(&c->loss, sizeof(float));
+    if (e == cudaSuccess) e = cudaMalloc(&c->grad, sizeof(float) * (pn::kNumW + 1));
+    if (e == cudaSuccess) e = cudaMalloc(&c->w1, sizeof(float) * pn::kScanPart);
+    if (e == cudaSuccess) e = cudaMallocHost(&c->h_grad, sizeof(float) * (pn::kNumW + 1));
     if (e == cudaSuccess) e = cudaMalloc(&c->w2op, pn::kOperandBytes);
     if (e == cudaSuccess) e = cudaMalloc(&c->err, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(c->err, 0, sizeof(int));
@@ -841,10 +954,11 @@ void ndt_mlp_destroy(ndt_mlp *c) {
     if (!c) return;
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
-    void *bufs[] = {c->w, c->m, c->v, c->grad, c->loss, c->w2op, c->err, c->gmax, c->grad_scan, c->loss_scan,
-                    c->dg, c->head_part};
+    void *bufs[] = {c->w, c->m, c->v, c->grad, c->w1, c->w2op, c->err, c->gmax, c->grad_scan, c->loss_scan,
+                    c->dg, c->head_part, c->feat};
     for (void *p : bufs)
         if (p) cudaFree(p);
+    if (c->h_grad) cudaFreeHost(c->h_grad);
     learned_buffers_free(c->lb);
     for (cudaEvent_t e : c->ev)
         if (e) cudaEventDestroy(e);
@@ -929,6 +1043,8 @@ int ndt_mlp_train_step_device(ndt_mlp *c, int B, const float *d_points, const in
     sb.gmax = c->gmax;
     sb.dg = c->dg;
     sb.grad_scan = c->grad_scan;
+    sb.feat = c->feat;
+    sb.w1 = c->w1;
     sb.nm = c->nm;
     sb.B = B;
     sb.max_points = max_points;
@@ -944,7 +1060,9 @@ int ndt_mlp_train_step_device(ndt_mlp *c, int B, const float *d_points, const in
     a.parts = (B + 127) / 128;
     a.loss_scan = c->loss_scan;
     a.grad = c->grad;
-    a.loss = c->loss;
+    a.feat = c->feat;
+    a.w1 = c->w1;
+    a.w2op = c->w2op;
     a.B = B;
     a.lr = lr;
     a.beta1 = 0.9f;
@@ -953,15 +1071,16 @@ int ndt_mlp_train_step_device(ndt_mlp *c, int B, const float *d_points, const in
     a.bc1 = 1.0f - std::pow(0.9f, (float)(c->step > 0 ? c->step : 1));
     a.bc2 = 1.0f - std::pow(0.999f, (float)(c->step > 0 ? c->step : 1));
     a.update = update;
-    pn::reduce_adam_kernel<<<(pn::kNumW + 255) / 256, 256, 0, c->stream>>>(a);
+    pn::reduce_adam_kernel<<<pn::kAdamBlocks + 1, pn::kAdamBlock, 0, c->stream>>>(a);
     MCK(cudaGetLastError());
-    if (update) {
-        pn::pack_w2_kernel<<<(pn::kH2 * pn::kH1 + 255) / 256, 256, 0, c->stream>>>(c->w, c->w2op);
-        MCK(cudaGetLastError());
-    }
-    if (h_loss) MCK(cudaMemcpyAsync(h_loss, c->loss, sizeof(float), cudaMemcpyDeviceToHost, c->stream));
-    if (h_grad) MCK(cudaMemcpyAsync(h_grad, c->grad, sizeof(float) * pn::kNumW, cudaMemcpyDeviceToHost, c->stream));
-    if (h_loss || h_grad) MCK(cudaStreamSynchronize(c->stream));
+    if (!h_loss && !h_grad) return NDT_OK;
+    // one copy through pinned memory: the loss follows the gradient
+    const size_t from = h_grad ? 0 : pn::kNumW, to = h_loss ? pn::kNumW + 1 : pn::kNumW;
+    MCK(cudaMemcpyAsync(c->h_grad + from, c->grad + from, sizeof(float) * (to - from), cudaMemcpyDeviceToHost,
+                        c->stream));
+    MCK(cudaStreamSynchronize(c->stream));
+    if (h_loss) *h_loss = c->h_grad[pn::kNumW];
+    if (h_grad) std::memcpy(h_grad, c->h_grad, sizeof(float) * pn::kNumW);
     return NDT_OK;
 }
 
