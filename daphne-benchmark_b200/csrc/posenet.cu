@@ -114,9 +114,8 @@ __global__ void __launch_bounds__(128, 1) point_kernel(const __grid_constant__ P
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t *sA = smem;                                  // 16 KB
     uint8_t *sB = smem + kOperandBytes;                  // 16 KB
-    float *sW1 = reinterpret_cast<float *>(smem + 2 * kOperandBytes);  // 192 + 64 (b1) + 128 (b2)
-    float *sB1 = sW1 + kH1 * 3;
-    float *sB2 = sB1 + kH1;
+    float4 *sW1 = reinterpret_cast<float4 *>(smem + 2 * kOperandBytes);  // 64 rows (W1, b1), then 128 b2
+    float *sB2 = reinterpret_cast<float *>(sW1 + kH1);
     uint64_t *sBar = reinterpret_cast<uint64_t *>(sB2 + kH2);  // 8-byte aligned (offset 32768 + 1536)
     uint32_t *sTmem = reinterpret_cast<uint32_t *>(sBar + 1);
     __shared__ float sT[12];
@@ -131,8 +130,8 @@ __global__ void __launch_bounds__(128, 1) point_kernel(const __grid_constant__ P
     // operands and small weights into shared memory
     for (int i = tid; i < kOperandBytes / 16; i += 128)
         reinterpret_cast<uint4 *>(sB)[i] = reinterpret_cast<const uint4 *>(a.w2op)[i];
-    for (int i = tid; i < kH1 * 3; i += 128) sW1[i] = a.w[oW1 + i];
-    for (int i = tid; i < kH1; i += 128) sB1[i] = a.w[oB1 + i];
+    if (tid < kH1)
+        sW1[tid] = make_float4(a.w[oW1 + 3 * tid], a.w[oW1 + 3 * tid + 1], a.w[oW1 + 3 * tid + 2], a.w[oB1 + tid]);
     for (int i = tid; i < kH2; i += 128) sB2[i] = a.w[oB2 + i];
     if (tid < 12) sT[tid] = a.guesses[16 * (size_t)b + tid];
     if (tid == 0) {
@@ -174,12 +173,13 @@ __global__ void __launch_bounds__(128, 1) point_kernel(const __grid_constant__ P
             __align__(16) __nv_bfloat16 h[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-                const int k = kc * 8 + e;
-                float v = fmaf(sW1[3 * k], u[0], fmaf(sW1[3 * k + 1], u[1], fmaf(sW1[3 * k + 2], u[2], sB1[k])));
-                v = valid ? fmaxf(v, 0.0f) : 0.0f;
-                h[e] = __float2bfloat16_rn(v);
+                const float4 q = sW1[kc * 8 + e];
+                const float v = fmaf(q.x, u[0], fmaf(q.y, u[1], fmaf(q.z, u[2], q.w)));
+                h[e] = __float2bfloat16_rn(fmaxf(v, 0.0f));
             }
-            *reinterpret_cast<uint4 *>(sA + op_offset(tid, kc * 8)) = *reinterpret_cast<const uint4 *>(h);
+            // (rows beyond the samples are zero: their columns are not read back)
+            *reinterpret_cast<uint4 *>(sA + op_offset(tid, kc * 8)) =
+                valid ? *reinterpret_cast<const uint4 *>(h) : make_uint4(0, 0, 0, 0);
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -254,13 +254,23 @@ __global__ void __launch_bounds__(128, 1) point_kernel(const __grid_constant__ P
                   "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
                 : "r"(addr));
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            if (nvalid == kTileRows) {
 #pragma unroll
-            for (int e = 0; e < 32; ++e) {
-                const int col = 32 * q + e;
-                const float z = __uint_as_float(r[e]);
-                if (col < nvalid && z > best) {  // strict: the smallest index among equal maxima
-                    best = z;
-                    best_j = t * kTileRows + col;
+                for (int e = 0; e < 32; ++e) {
+                    const float z = __uint_as_float(r[e]);
+                    if (z > best) {  // strict: the smallest index among equal maxima
+                        best = z;
+                        best_j = t * kTileRows + 32 * q + e;
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int e = 0; e < 32; ++e) {
+                    const float z = __uint_as_float(r[e]);
+                    if (32 * q + e < nvalid && z > best) {
+                        best = z;
+                        best_j = t * kTileRows + 32 * q + e;
+                    }
                 }
             }
         }
@@ -727,7 +737,7 @@ static_assert(oW2 % kAdamBlock == 0 && oB2 % kAdamBlock == 0 && oW3 % kAdamBlock
 
 // Sum over b < n, in order, of f(row b): the rows come through shared memory,
 // kRows at a time (their latency is the sum's time otherwise: 21 us for 256
-// scans with the loads in the loop, XXX us as here).
+// scans with the loads in the loop, 8 us as here).
 template <class T, class Load, class F>
 __device__ __forceinline__ float ordered_sum(int n, T *s_row, Load load, F f) {
     constexpr int kRows = 256;
@@ -845,7 +855,7 @@ int mlp_fail(ndt_mlp *c, cudaError_t e, const char *what) {
         if (e_ != cudaSuccess) return mlp_fail(c, e_, #call);   \
     } while (0)
 
-constexpr size_t kPointSmem = 2 * pn::kOperandBytes + (pn::kH1 * 3 + pn::kH1 + pn::kH2) * 4 + 64;
+constexpr size_t kPointSmem = 2 * pn::kOperandBytes + (pn::kH1 * 4 + pn::kH2) * 4 + 64;
 // keep at most 4 CTAs per SM, so that 4 x 128 TMEM columns fit
 constexpr size_t kPointSmemAlloc = kPointSmem < 48 * 1024 ? 48 * 1024 : kPointSmem;
 
