@@ -15,11 +15,11 @@
 // Here: points are sorted into cells of edge r * (1 + 1e-4) (cell indices in
 // FP64, so an accepted pair is never more than one cell apart on any axis;
 // at most 2^28 cells per cloud) with the voxel-grid
-// build's stable radix sort; one thread per point and neighbour cell tests
-// that cell's points with the same float operations and joins accepted pairs
-// in a lock-free union-find whose roots are always the component's smallest
-// index (the larger root is linked under the smaller by atomicCAS); after a
-// final compression every label is its component's smallest index.  The host
+// build's stable radix sort; a warp per point tests the earlier points of its
+// own and the neighbour cells with the same float operations.  A first pass
+// hangs every point under the first one it is joined to, a second joins the
+// trees in a lock-free union-find (the larger root is linked under the smaller
+// by atomicCAS); every label is its tree's smallest point index.  The host
 // groups the indices by label (ascending, so clusters come out in the
 // reference's order), filters by size and applies the same std::sort.
 #include <cuda_runtime.h>
@@ -40,7 +40,6 @@
 namespace ec {
 
 constexpr int kThreads = 256;
-constexpr int kSplit = 4;  // threads per (point, neighbour cell): dense cells are shared out
 constexpr int kUnionLimit = 1 << 20;  // CAS retries of one union (never reached in practice; flags an error)
 
 constexpr int kMaxParts = 40;  // clouds clustered in one pass (segmentByDistance: 5 rings of up to 8 clouds)
@@ -78,7 +77,7 @@ __device__ __forceinline__ int part_of(const T *first, int np, long long t) {
 }
 
 __global__ void key_kernel(const float4 *__restrict__ pts, int n, const __grid_constant__ Parts P,
-                           uint32_t *__restrict__ keys, int *__restrict__ parent) {
+                           uint32_t *__restrict__ keys, int *__restrict__ least) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int q = part_of(P.off, P.np, i);
@@ -87,20 +86,24 @@ __global__ void key_kernel(const float4 *__restrict__ pts, int n, const __grid_c
     const int cy = cell_of(p.y, P.minv[q][1], P.cell[q], P.dim[q][1]);
     const int cz = cell_of(p.z, P.minv[q][2], P.cell[q], P.dim[q][2]);
     keys[i] = (uint32_t)(P.base[q] + cx + (long long)P.dim[q][0] * (cy + (long long)P.dim[q][1] * cz));
-    parent[i] = i;
+    least[i] = 0x7fffffff;
 }
 
-// cell -> first sorted position of its points (segment s), or -1
-__global__ void cell_index_kernel(const int32_t *__restrict__ seg_start, const uint32_t *__restrict__ seg_key,
-                                  const int *__restrict__ nseg, int *__restrict__ cell_first) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < *nseg) cell_first[seg_key[s]] = s;
+// The points in sorted order and cell -> its segment s of the sorted order
+// (-1 where there are no points).
+__global__ void gather_kernel(const float4 *__restrict__ pts, const uint32_t *__restrict__ order, int n,
+                              const uint32_t *__restrict__ seg_key, const int *__restrict__ nseg,
+                              float4 *__restrict__ sorted, int *__restrict__ cell_first) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    sorted[t] = pts[order[t]];
+    if (t < *nseg) cell_first[seg_key[t]] = t;
 }
 
-// Union-find over parent[] with parent[v] <= v for every v (a root links
-// under a smaller one only), so every chain strictly decreases and a root is
-// its component's smallest index.  Reads are volatile (other threads link and
-// shorten concurrently); path halving stores a valid ancestor, so any
+// Union-find over the sorted positions, parent[v] <= v for every v (a root
+// links under a smaller one only), so every chain strictly decreases and a
+// root is its component's first position.  Reads are volatile (other threads
+// link and shorten concurrently); path halving stores a valid ancestor, so any
 // interleaving keeps the invariant.
 __device__ __forceinline__ int find_root(int *parent, int x) {
     volatile int *p = parent;
@@ -114,68 +117,162 @@ __device__ __forceinline__ int find_root(int *parent, int x) {
     return -1;
 }
 
-// kSplit threads per (point i, neighbour cell): blockIdx.y picks the cell
-// offset (27 of them) and the thread's share of the cell's points (every
-// kSplit-th), x walks the points in sorted order, so a warp's points share
-// cells and read the same neighbours.  The thread tests the points j > i of
-// its cell (cells never cross parts); i's root is found at the first accepted
-// pair and kept; a pair whose roots already agree costs the reads of j's
-// chain, a merge one atomicCAS (the larger root under the smaller).
-__global__ void join_kernel(const float4 *__restrict__ pts, const uint32_t *__restrict__ order,
-                            const uint32_t *__restrict__ keys, int n, const int32_t *__restrict__ seg_start,
-                            const int *__restrict__ nseg, const int *__restrict__ cell_first,
-                            const __grid_constant__ Parts P, int *__restrict__ parent, int *__restrict__ err) {
+// The earlier points that position t has to be tested against: those before it
+// in its own cell and in the cell before that, the row of three cells at y - 1
+// and the three rows at z - 1 (cells never cross parts; a pair is accepted or
+// not whichever of its points comes first).  The cells of a row have
+// consecutive keys, so a row's points are one stretch of the sorted order;
+// lanes 0..14 of the warp look the 5 x 3 cells up at once.
+constexpr unsigned kAll = 0xffffffffu;
+constexpr int kRows = 5;
+struct Rows {
+    int from[kRows], to[kRows];  // in ascending order
+    float r2;
+    __device__ __forceinline__ Rows(int t, uint32_t key, int lane, const int32_t *__restrict__ seg_start, int n,
+                                    int nseg, const int *__restrict__ cell_first, const Parts &P) {
+        const int q = part_of(P.base, P.np, key);
+        r2 = P.r2[q];
+        const unsigned local = key - (uint32_t)P.base[q];
+        const unsigned dx0 = P.dim[q][0], dy0 = P.dim[q][1];
+        const unsigned row = local / dx0, z0 = row / dy0;
+        int first = n, last = 0;
+        if (lane < 3 * kRows - 1) {
+            const int r = lane / 3;  // (dy, dz) = (-1, -1), (0, -1), (1, -1), (-1, 0), (0, 0)
+            const int dx = lane % 3 - 1, dz = r < 3 ? -1 : 0, dy = r < 3 ? r - 1 : r - 4;
+            const int x = (int)(local - row * dx0) + dx, y = (int)(row - z0 * dy0) + dy, z = (int)z0 + dz;
+            if (x >= 0 && x < (int)dx0 && y >= 0 && y < (int)dy0 && z >= 0) {
+                const int s = cell_first[P.base[q] + x + (long long)dx0 * (y + (long long)dy0 * z)];
+                if (s >= 0) {
+                    first = seg_start[s];
+                    last = lane == 3 * kRows - 2 ? t : (s + 1 < nseg ? seg_start[s + 1] : n);
+                }
+            }
+        }
+        first = min(first, min(__shfl_down_sync(kAll, first, 1), __shfl_down_sync(kAll, first, 2)));
+        last = max(last, max(__shfl_down_sync(kAll, last, 1), __shfl_down_sync(kAll, last, 2)));
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+            from[r] = __shfl_sync(kAll, first, 3 * r);
+            to[r] = __shfl_sync(kAll, last, 3 * r);
+        }
+    }
+};
+
+__device__ __forceinline__ bool accepted(float4 a, float4 b, float r2) {
+    const float ex = __fsub_rn(a.x, b.x), ey = __fsub_rn(a.y, b.y), ez = __fsub_rn(a.z, b.z);
+    return __fadd_rn(__fadd_rn(__fmul_rn(ex, ex), __fmul_rn(ey, ey)), __fmul_rn(ez, ez)) <= r2;
+}
+
+// First pass, a warp per position t: t hangs under the first earlier point
+// that it is joined to.  Nothing but t's warp writes parent[t], and what is left to the
+// second pass are the few trees of a component whose roots have no earlier
+// neighbour.  With every point its own tree at the start of that pass, all the
+// warps of a component contended for the same few roots: 595 us, against 21 for
+// this pass, 12 for root_kernel and 91 for what is then left of the second
+// (five clouds of 9600 points).  A thread per (point, one of 27 cells, quarter
+// of that cell), which tested both orders of every pair and divided 64-bit
+// keys for each, took 278 us.
+__global__ void __launch_bounds__(kThreads) hook_kernel(
+    const float4 *__restrict__ sorted, const uint32_t *__restrict__ keys, int n,
+    const int32_t *__restrict__ seg_start, const int *__restrict__ nseg, const int *__restrict__ cell_first,
+    const __grid_constant__ Parts P, int *__restrict__ parent) {
+    const int t = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (t >= n) return;
+    const Rows R(t, keys[t], lane, seg_start, n, *nseg, cell_first, P);
+    const float4 p = sorted[t];
+    int up = t;
+#pragma unroll
+    for (int r = 0; r < kRows; ++r)
+        for (int u0 = R.from[r]; u0 < R.to[r] && up == t; u0 += 32) {
+            const int u = u0 + lane;
+            const unsigned in = __ballot_sync(kAll, u < R.to[r] && accepted(sorted[min(u, n - 1)], p, R.r2));
+            if (in) up = u0 + __ffs(in) - 1;
+        }
+    if (lane == 0) parent[t] = up;
+}
+
+__global__ void root_kernel(int *__restrict__ parent, int n, int *__restrict__ err) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
-    const int off = blockIdx.y / kSplit;  // 9 dz + 3 dy + dx, each in {0, 1, 2}
-    const int part = blockIdx.y % kSplit;  // this thread's share of the cell: every kSplit-th point
-    const long long key = keys[t];
-    const int q = part_of(P.base, P.np, key);
-    const long long local = key - P.base[q];
-    const int dx0 = P.dim[q][0], dy0 = P.dim[q][1], dz0 = P.dim[q][2];
-    const int x = (int)(local % dx0) + off % 3 - 1;
-    const int y = (int)((local / dx0) % dy0) + (off / 3) % 3 - 1;
-    const int z = (int)(local / ((long long)dx0 * dy0)) + off / 9 - 1;
-    if (x < 0 || x >= dx0 || y < 0 || y >= dy0 || z < 0 || z >= dz0) return;
-    const int s = cell_first[P.base[q] + x + (long long)dx0 * (y + (long long)dy0 * z)];
-    if (s < 0) return;
-    const int i = (int)order[t];
-    const float4 p = pts[i];
-    const float r2 = P.r2[q];
-    const int e = s + 1 < *nseg ? seg_start[s + 1] : n;
-    int ri = -2;  // not looked up yet
-    for (int u = seg_start[s] + part; u < e; u += kSplit) {
-        const int j = (int)order[u];
-        if (j <= i) continue;
-        const float4 qj = pts[j];
-        const float ex = __fsub_rn(qj.x, p.x), ey = __fsub_rn(qj.y, p.y), ez = __fsub_rn(qj.z, p.z);
-        const float d2 = __fadd_rn(__fadd_rn(__fmul_rn(ex, ex), __fmul_rn(ey, ey)), __fmul_rn(ez, ez));
-        if (!(d2 <= r2)) continue;
-        if (ri == -2) ri = find_root(parent, i);
-        int rj = find_root(parent, j);
-        int it = 0;
-        for (; it < kUnionLimit && ri >= 0 && rj >= 0 && ri != rj; ++it) {
-            const int lo = ri < rj ? ri : rj, hi = ri < rj ? rj : ri;
-            if (atomicCAS(parent + hi, hi, lo) == hi) {
-                ri = lo;
-                break;
+    const int r = find_root(parent, t);
+    if (r < 0) atomicOr(err, 2);
+    else parent[t] = r;
+}
+
+// Second pass, a warp per position t: the trees of t and of every earlier
+// point that it is joined to become one.  A candidate that hangs under t's
+// root already costs one read, next to its neighbours'; for the others the warp
+// links all roots that it sees under the smallest of them, one atomicCAS each.
+// Bound by the latency of its chains (cells, points, parents, roots) at 5 waves
+// of warps: its rows read ahead (99 us), rows skipped by their parents before
+// the coordinates are read (109 us) and a pass of atomicMin in between (35 us
+// for it and 56 for this one) did not help.
+__global__ void __launch_bounds__(kThreads) join_kernel(
+    const float4 *__restrict__ sorted, const uint32_t *__restrict__ keys, int n,
+    const int32_t *__restrict__ seg_start, const int *__restrict__ nseg, const int *__restrict__ cell_first,
+    const __grid_constant__ Parts P, int *__restrict__ parent, int *__restrict__ err) {
+    const int t = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (t >= n) return;
+    const Rows R(t, keys[t], lane, seg_start, n, *nseg, cell_first, P);
+    const float4 p = sorted[t];
+    volatile int *up = parent;
+    int ri = find_root(parent, t);
+    bool bad = ri < 0;
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+        for (int u0 = R.from[r]; u0 < R.to[r]; u0 += 32) {
+            const int u = u0 + lane;
+            const float4 c = sorted[min(u, n - 1)];
+            int rj = up[min(u, n - 1)];  // of the lanes with an accepted point: a node of its tree, in the end its root
+            if (u >= R.to[r] || !accepted(c, p, R.r2)) rj = ri;
+            if (rj != ri) rj = find_root(parent, rj);
+            for (int it = 0; !__all_sync(kAll, rj == ri); ++it) {
+                bad = bad || rj < 0 || it == kUnionLimit;
+                if (__any_sync(kAll, bad)) break;
+                const int m = min(ri, __reduce_min_sync(kAll, rj));
+                if (rj != ri && rj != m) rj = atomicCAS(parent + rj, rj, m) == rj ? m : find_root(parent, rj);
+                int rn = ri;
+                if (ri != m && lane == 0) rn = atomicCAS(parent + ri, ri, m) == ri ? m : find_root(parent, ri);
+                rn = __shfl_sync(kAll, rn, 0);
+                if (rj == ri) rj = rn;
+                bad = bad || rn < 0;
+                ri = rn;
             }
-            ri = find_root(parent, ri);  // hi was linked meanwhile
-            rj = find_root(parent, rj);
-        }
-        if (ri < 0 || rj < 0 || it == kUnionLimit) {
-            atomicOr(err, 1);
-            return;
+            if (__any_sync(kAll, bad)) {
+                if (lane == 0) atomicOr(err, 1);
+                return;
+            }
         }
     }
 }
 
-__global__ void label_kernel(int *__restrict__ parent, int n, int *__restrict__ err) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int r = find_root(parent, i);
-    if (r < 0) atomicOr(err, 2);
-    parent[i] = r;
+// The smallest point index of every tree, at its root (least[] starts at INT_MAX).
+__global__ void least_kernel(int *__restrict__ parent, const uint32_t *__restrict__ order, int n,
+                             int *__restrict__ least, int *__restrict__ err) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int r = t < n ? find_root(parent, t) : -1;
+    if (t < n) {
+        if (r < 0) atomicOr(err, 2);
+        else parent[t] = r;
+    }
+    const int r0 = __shfl_sync(kAll, r, 0);
+    const int i = t < n ? (int)order[t] : 0x7fffffff;
+    if (__all_sync(kAll, r == r0 || t >= n)) {  // one tree in the whole warp, as nearly always
+        const int m = __reduce_min_sync(kAll, i);
+        if ((threadIdx.x & 31) == 0 && r0 >= 0) atomicMin(least + r0, m);
+    } else if (r >= 0) {
+        atomicMin(least + r, i);
+    }
+}
+
+__global__ void label_kernel(const int *__restrict__ parent, const uint32_t *__restrict__ order, int n,
+                             const int *__restrict__ least, int *__restrict__ label) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const int r = parent[t];
+    label[order[t]] = least[r];
 }
 
 }  // namespace ec
@@ -184,9 +281,9 @@ struct ndt_ec {
     int device = 0;
     cudaStream_t stream = nullptr;
     std::string err;
-    void *pts = nullptr, *scratch = nullptr, *parent = nullptr, *seg_start = nullptr, *seg_key = nullptr,
+    void *pts = nullptr, *sorted = nullptr, *scratch = nullptr, *parent = nullptr, *seg_start = nullptr, *seg_key = nullptr,
          *cell_first = nullptr, *flags = nullptr;
-    size_t pts_cap = 0, scratch_cap = 0, parent_cap = 0, seg_start_cap = 0, seg_key_cap = 0, cell_cap = 0;
+    size_t pts_cap = 0, sorted_cap = 0, scratch_cap = 0, parent_cap = 0, seg_start_cap = 0, seg_key_cap = 0, cell_cap = 0;
     float4 *h_pts = nullptr;  // pinned staging
     int *h_labels = nullptr;
     size_t h_cap = 0;
@@ -282,29 +379,36 @@ int labels_of(ndt_ec *h, const std::vector<const float *> &xyz, const std::vecto
     int bits = 1;
     while (bits < 31 && (1LL << bits) < cells) ++bits;
     ECK(ensure(&h->pts, &h->pts_cap, sizeof(float4) * (size_t)N));
+    ECK(ensure(&h->sorted, &h->sorted_cap, sizeof(float4) * (size_t)N));
     ECK(ensure(&h->scratch, &h->scratch_cap, ndt::sort_scratch_bytes(N)));
-    ECK(ensure(&h->parent, &h->parent_cap, sizeof(int) * (size_t)N));
+    ECK(ensure(&h->parent, &h->parent_cap, 3 * sizeof(int) * (size_t)N));
     ECK(ensure(&h->seg_start, &h->seg_start_cap, sizeof(int) * (size_t)N));
     ECK(ensure(&h->seg_key, &h->seg_key_cap, sizeof(int) * (size_t)N));
     ECK(ensure(&h->cell_first, &h->cell_cap, sizeof(int) * (size_t)cells));
     size_t fcap = 0;
     if (!h->flags) ECK(ensure(&h->flags, &fcap, 256));
     float4 *d_pts = (float4 *)h->pts;
-    int *parent = (int *)h->parent, *err = (int *)h->flags;
+    int *parent = (int *)h->parent, *least = parent + N, *label = least + N, *err = (int *)h->flags;
     ECK(cudaMemcpyAsync(d_pts, h->h_pts, sizeof(float4) * (size_t)N, cudaMemcpyHostToDevice, st));
     ECK(cudaMemsetAsync(err, 0, sizeof(int), st));
     ECK(cudaMemsetAsync(h->cell_first, 0xff, sizeof(int) * (size_t)cells, st));
     ndt::SortBuffers sb = ndt::sort_buffers(h->scratch, N);
     const unsigned blocks = (unsigned)((N + ec::kThreads - 1) / ec::kThreads);
-    ec::key_kernel<<<blocks, ec::kThreads, 0, st>>>(d_pts, N, P, sb.k0, parent);
+    ec::key_kernel<<<blocks, ec::kThreads, 0, st>>>(d_pts, N, P, sb.k0, least);
     ndt::sort_segments(sb, N, bits, (int32_t *)h->seg_start, (uint32_t *)h->seg_key, st, true);
-    ec::cell_index_kernel<<<blocks, ec::kThreads, 0, st>>>((const int32_t *)h->seg_start, (const uint32_t *)h->seg_key,
-                                                           sb.nseg, (int *)h->cell_first);
-    ec::join_kernel<<<dim3(blocks, 27 * ec::kSplit), ec::kThreads, 0, st>>>(
-        d_pts, sb.v0, sb.k0, N, (const int32_t *)h->seg_start, sb.nseg, (const int *)h->cell_first, P, parent, err);
-    ec::label_kernel<<<blocks, ec::kThreads, 0, st>>>(parent, N, err);
+    ec::gather_kernel<<<blocks, ec::kThreads, 0, st>>>(d_pts, sb.v0, N, (const uint32_t *)h->seg_key, sb.nseg,
+                                                       (float4 *)h->sorted, (int *)h->cell_first);
+    const float4 *sorted = (const float4 *)h->sorted;
+    const int32_t *seg_start = (const int32_t *)h->seg_start;
+    const int *cell_first = (const int *)h->cell_first;
+    const unsigned per_block = ec::kThreads / 32, wide = (N + per_block - 1) / per_block;
+    ec::hook_kernel<<<wide, ec::kThreads, 0, st>>>(sorted, sb.k0, N, seg_start, sb.nseg, cell_first, P, parent);
+    ec::root_kernel<<<blocks, ec::kThreads, 0, st>>>(parent, N, err);
+    ec::join_kernel<<<wide, ec::kThreads, 0, st>>>(sorted, sb.k0, N, seg_start, sb.nseg, cell_first, P, parent, err);
+    ec::least_kernel<<<blocks, ec::kThreads, 0, st>>>(parent, sb.v0, N, least, err);
+    ec::label_kernel<<<blocks, ec::kThreads, 0, st>>>(parent, sb.v0, N, least, label);
     ECK(cudaGetLastError());
-    ECK(cudaMemcpyAsync(h->h_labels, parent, sizeof(int) * (size_t)N, cudaMemcpyDeviceToHost, st));
+    ECK(cudaMemcpyAsync(h->h_labels, label, sizeof(int) * (size_t)N, cudaMemcpyDeviceToHost, st));
     int e = 0, sort_err = 0;
     ECK(cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, st));
     ECK(cudaMemcpyAsync(&sort_err, ndt::sort_error(sb, N), sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -360,7 +464,7 @@ void ndt_ec_destroy(ndt_ec *h) {
     if (!h) return;
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
-    for (void *p : {h->pts, h->scratch, h->parent, h->seg_start, h->seg_key, h->cell_first, h->flags})
+    for (void *p : {h->pts, h->sorted, h->scratch, h->parent, h->seg_start, h->seg_key, h->cell_first, h->flags})
         if (p) cudaFree(p);
     if (h->h_pts) cudaFreeHost(h->h_pts);
     if (h->h_labels) cudaFreeHost(h->h_labels);
