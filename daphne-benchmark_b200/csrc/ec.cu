@@ -12,18 +12,23 @@
 // [min, max] points are kept and ordered by size with std::sort over reverse
 // iterators.
 //
-// Here: points are sorted into cells of edge r * (1 + 1e-4) (cell indices in
-// FP64, so an accepted pair is never more than one cell apart on any axis;
-// at most 2^28 cells per cloud) with the voxel-grid
-// build's stable radix sort; a warp per point tests the earlier points of its
-// own and the neighbour cells with the same float operations.  A first pass
-// hangs every point under the first one it is joined to, a second joins the
-// trees in a lock-free union-find (the larger root is linked under the smaller
-// by atomicCAS); every label is its tree's smallest point index.  The host
-// groups the indices by label (ascending, so clusters come out in the
-// reference's order), filters by size and applies the same std::sort.
+// Here the points of all distance rings of up to 8 clouds go through one pass:
+// a kernel finds every point's part (cloud and ring) and the parts' bounding
+// boxes; points are sorted into cells of edge r * (1 + 1e-4) of their part
+// (cell indices in FP64, so an accepted pair is never more than one cell apart
+// on any axis; at most 2^28 cells in all) with the voxel-grid build's stable
+// radix sort; a warp per point tests the earlier points of its own and the
+// neighbour cells with the same float operations.  A first pass hangs every
+// point under the first one it is joined to, a second joins the trees in a
+// lock-free union-find (the larger root is linked under the smaller by
+// atomicCAS); every label is its tree's smallest point index.  A second sort, by
+// label, lists the clusters: in the reference's order, their points ascending.
+// The host applies the same std::sort to the sizes and spreads the clusters'
+// points, centroids and boxes over its threads.
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <limits.h>
 
 #include <algorithm>
 #include <cmath>
@@ -40,22 +45,39 @@
 namespace ec {
 
 constexpr int kThreads = 256;
+constexpr unsigned kAll = 0xffffffffu;
 constexpr int kUnionLimit = 1 << 20;  // CAS retries of one union (never reached in practice; flags an error)
 
-constexpr int kMaxParts = 40;  // clouds clustered in one pass (segmentByDistance: 5 rings of up to 8 clouds)
+constexpr int kMaxParts = 40;  // parts clustered in one pass (segmentByDistance: 5 rings of up to 8 clouds)
 
-// Geometry of the clouds of one pass: part p's points are [off[p], off[p + 1])
-// of the concatenation, its cells have edge cell[p] from minv[p] with dims
-// dim[p], and its cell keys are base[p] + x + dx (y + dy z).
+// Geometry of the parts of one pass: part p's cells have edge cell[p] from
+// minv[p] with dims dim[p], and its cell keys are base[p] + x + dx (y + dy z).
 struct Parts {
-    int np;
-    int off[kMaxParts + 1];
     long long base[kMaxParts + 1];
     float minv[kMaxParts][3];
     float cell[kMaxParts];
     float r2[kMaxParts];
     int dim[kMaxParts][3];
 };
+
+// Which part a point belongs to: the distance ring of its cloud, or one part
+// for all (rings == 1).
+constexpr int kRings = 5;
+struct Clouds {
+    int count, rings;
+    int off[kMaxParts / kRings + 1];
+};
+__host__ __device__ inline int ring_of(float x, float y) {
+    const float d = sqrtf(x * x + y * y);
+    return d < 15 ? 0 : (d < 30 ? 1 : (d < 45 ? 2 : (d < 60 ? 3 : 4)));
+}
+
+// A part's bounding box: the coordinates as integers of the same order.
+struct Box {
+    int lo[3], hi[3];
+    int points, bad;  // any points, any coordinate that is not finite
+};
+__host__ __device__ inline int ordered(int bits) { return bits ^ ((bits >> 31) & 0x7fffffff); }
 
 // Cell index in FP64 (the difference of two floats is exact there), so that
 // cell boundaries move by no more than ~1e-16 cells: with cells 1e-4 wider
@@ -65,23 +87,78 @@ __device__ __forceinline__ int cell_of(float v, float minv, float cell, int dim)
     return c < 0 ? 0 : (c >= dim ? dim - 1 : c);
 }
 
-// The part of point t (or of key k): the last p with first[p] <= t.
-template <class T>
-__device__ __forceinline__ int part_of(const T *first, int np, long long t) {
-    int lo = 0, hi = np;
+// The cloud of point t: the last c with off[c] <= t.
+__host__ __device__ inline int cloud_of(const Clouds &C, int t) {
+    int lo = 0, hi = C.count;
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
-        if ((long long)first[mid] <= t) lo = mid; else hi = mid;
+        if (C.off[mid] <= t) lo = mid; else hi = mid;
     }
     return lo;
+}
+
+// The points as float4 with their part in w, and the parts' boxes (lo starts at
+// INT_MAX, hi at INT_MIN).  A warp holds points of few parts: one reduction for
+// each of them, then the block's boxes in shared memory.
+__global__ void __launch_bounds__(kThreads) part_kernel(const float *__restrict__ xyz, int n,
+                                                        const __grid_constant__ Clouds C, float4 *__restrict__ pts,
+                                                        Box *__restrict__ boxes) {
+    __shared__ Box s_box[kMaxParts];
+    const int np = C.count * C.rings;
+    for (int k = threadIdx.x; k < np; k += kThreads)
+        s_box[k] = {{INT_MAX, INT_MAX, INT_MAX}, {INT_MIN, INT_MIN, INT_MIN}, 0, 0};
+    __syncthreads();
+    const int i = blockIdx.x * kThreads + threadIdx.x;
+    int q = -1, v[3] = {0, 0, 0};
+    bool bad = false;
+    if (i < n) {
+        const float x = xyz[3 * (size_t)i], y = xyz[3 * (size_t)i + 1], z = xyz[3 * (size_t)i + 2];
+        q = C.rings * cloud_of(C, i) + (C.rings > 1 ? ring_of(x, y) : 0);
+        bad = !(isfinite(x) && isfinite(y) && isfinite(z));
+        pts[i] = make_float4(x, y, z, __int_as_float(q));
+        v[0] = ordered(__float_as_int(x));
+        v[1] = ordered(__float_as_int(y));
+        v[2] = ordered(__float_as_int(z));
+    }
+    for (unsigned left = __ballot_sync(kAll, q >= 0); left;) {
+        const int part = __shfl_sync(kAll, q, __ffs(left) - 1);
+        const unsigned same = __ballot_sync(kAll, q == part);
+        left &= ~same;
+        if (q == part) {
+            const bool any_bad = __any_sync(same, bad);
+            const bool leader = (threadIdx.x & 31) == __ffs(same) - 1;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const int lo = __reduce_min_sync(same, v[k]), hi = __reduce_max_sync(same, v[k]);
+                if (leader) {
+                    atomicMin(&s_box[part].lo[k], lo);
+                    atomicMax(&s_box[part].hi[k], hi);
+                }
+            }
+            if (leader) {
+                s_box[part].points = 1;
+                if (any_bad) s_box[part].bad = 1;
+            }
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < 6 * np; k += kThreads) {
+        const int part = k / 6, c = k % 6;
+        if (!s_box[part].points) continue;
+        if (c < 3) atomicMin(&boxes[part].lo[c], s_box[part].lo[c]);
+        else atomicMax(&boxes[part].hi[c - 3], s_box[part].hi[c - 3]);
+        if (c == 0) boxes[part].points = 1;
+        if (c == 0 && s_box[part].bad) boxes[part].bad = 1;
+    }
 }
 
 __global__ void key_kernel(const float4 *__restrict__ pts, int n, const __grid_constant__ Parts P,
                            uint32_t *__restrict__ keys, int *__restrict__ least) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const int q = part_of(P.off, P.np, i);
     const float4 p = pts[i];
+    const int q = __float_as_int(p.w);
     const int cx = cell_of(p.x, P.minv[q][0], P.cell[q], P.dim[q][0]);
     const int cy = cell_of(p.y, P.minv[q][1], P.cell[q], P.dim[q][1]);
     const int cz = cell_of(p.z, P.minv[q][2], P.cell[q], P.dim[q][2]);
@@ -90,12 +167,13 @@ __global__ void key_kernel(const float4 *__restrict__ pts, int n, const __grid_c
 }
 
 // The points in sorted order and cell -> its segment s of the sorted order
-// (-1 where there are no points).
+// (-1 where there are no points).  No segments: the sort gave up, and nothing
+// after it may follow its order.
 __global__ void gather_kernel(const float4 *__restrict__ pts, const uint32_t *__restrict__ order, int n,
                               const uint32_t *__restrict__ seg_key, const int *__restrict__ nseg,
                               float4 *__restrict__ sorted, int *__restrict__ cell_first) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
+    if (t >= n || *nseg == 0) return;
     sorted[t] = pts[order[t]];
     if (t < *nseg) cell_first[seg_key[t]] = t;
 }
@@ -123,14 +201,12 @@ __device__ __forceinline__ int find_root(int *parent, int x) {
 // not whichever of its points comes first).  The cells of a row have
 // consecutive keys, so a row's points are one stretch of the sorted order;
 // lanes 0..14 of the warp look the 5 x 3 cells up at once.
-constexpr unsigned kAll = 0xffffffffu;
 constexpr int kRows = 5;
 struct Rows {
     int from[kRows], to[kRows];  // in ascending order
     float r2;
-    __device__ __forceinline__ Rows(int t, uint32_t key, int lane, const int32_t *__restrict__ seg_start, int n,
+    __device__ __forceinline__ Rows(int t, uint32_t key, int q, int lane, const int32_t *__restrict__ seg_start, int n,
                                     int nseg, const int *__restrict__ cell_first, const Parts &P) {
-        const int q = part_of(P.base, P.np, key);
         r2 = P.r2[q];
         const unsigned local = key - (uint32_t)P.base[q];
         const unsigned dx0 = P.dim[q][0], dy0 = P.dim[q][1];
@@ -178,9 +254,9 @@ __global__ void __launch_bounds__(kThreads) hook_kernel(
     const __grid_constant__ Parts P, int *__restrict__ parent) {
     const int t = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
-    if (t >= n) return;
-    const Rows R(t, keys[t], lane, seg_start, n, *nseg, cell_first, P);
+    if (t >= n || *nseg == 0) return;
     const float4 p = sorted[t];
+    const Rows R(t, keys[t], __float_as_int(p.w), lane, seg_start, n, *nseg, cell_first, P);
     int up = t;
 #pragma unroll
     for (int r = 0; r < kRows; ++r)
@@ -192,9 +268,9 @@ __global__ void __launch_bounds__(kThreads) hook_kernel(
     if (lane == 0) parent[t] = up;
 }
 
-__global__ void root_kernel(int *__restrict__ parent, int n, int *__restrict__ err) {
+__global__ void root_kernel(int *__restrict__ parent, int n, const int *__restrict__ nseg, int *__restrict__ err) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
+    if (t >= n || *nseg == 0) return;
     const int r = find_root(parent, t);
     if (r < 0) atomicOr(err, 2);
     else parent[t] = r;
@@ -214,9 +290,9 @@ __global__ void __launch_bounds__(kThreads) join_kernel(
     const __grid_constant__ Parts P, int *__restrict__ parent, int *__restrict__ err) {
     const int t = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
-    if (t >= n) return;
-    const Rows R(t, keys[t], lane, seg_start, n, *nseg, cell_first, P);
+    if (t >= n || *nseg == 0) return;
     const float4 p = sorted[t];
+    const Rows R(t, keys[t], __float_as_int(p.w), lane, seg_start, n, *nseg, cell_first, P);
     volatile int *up = parent;
     int ri = find_root(parent, t);
     bool bad = ri < 0;
@@ -250,7 +326,8 @@ __global__ void __launch_bounds__(kThreads) join_kernel(
 
 // The smallest point index of every tree, at its root (least[] starts at INT_MAX).
 __global__ void least_kernel(int *__restrict__ parent, const uint32_t *__restrict__ order, int n,
-                             int *__restrict__ least, int *__restrict__ err) {
+                             const int *__restrict__ nseg, int *__restrict__ least, int *__restrict__ err) {
+    if (*nseg == 0) return;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int r = t < n ? find_root(parent, t) : -1;
     if (t < n) {
@@ -267,12 +344,27 @@ __global__ void least_kernel(int *__restrict__ parent, const uint32_t *__restric
     }
 }
 
+// Point index -> label.  status[1] collects the errors: a sort that gave up is 4.
 __global__ void label_kernel(const int *__restrict__ parent, const uint32_t *__restrict__ order, int n,
-                             const int *__restrict__ least, int *__restrict__ label) {
+                             const int *__restrict__ nseg, const int *__restrict__ least,
+                             const int *__restrict__ sort_err, uint32_t *__restrict__ label,
+                             int *__restrict__ status) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    const int r = parent[t];
-    label[order[t]] = least[r];
+    if (t == 0 && *sort_err) atomicOr(status + 1, 4);
+    if (t >= n || *nseg == 0) return;
+    label[order[t]] = (uint32_t)least[parent[t]];
+}
+
+// The clusters of [lo, hi] points, as (first position, points) of the order by
+// label; status[0] counts them.
+__global__ void cluster_kernel(const int32_t *__restrict__ seg_start, const int *__restrict__ nseg, int n, int lo,
+                               int hi, const int *__restrict__ sort_err, int2 *__restrict__ rec,
+                               int *__restrict__ status) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s == 0 && *sort_err) atomicOr(status + 1, 4);
+    if (s >= *nseg) return;
+    const int b = seg_start[s], e = s + 1 < *nseg ? seg_start[s + 1] : n;
+    if (e - b >= lo && e - b <= hi) rec[atomicAdd(status, 1)] = make_int2(b, e - b);
 }
 
 }  // namespace ec
@@ -281,17 +373,16 @@ struct ndt_ec {
     int device = 0;
     cudaStream_t stream = nullptr;
     std::string err;
-    void *pts = nullptr, *sorted = nullptr, *scratch = nullptr, *parent = nullptr, *seg_start = nullptr, *seg_key = nullptr,
-         *cell_first = nullptr, *flags = nullptr;
-    size_t pts_cap = 0, sorted_cap = 0, scratch_cap = 0, parent_cap = 0, seg_start_cap = 0, seg_key_cap = 0, cell_cap = 0;
-    float4 *h_pts = nullptr;  // pinned staging
-    int *h_labels = nullptr;
-    size_t h_cap = 0;
+    void *work = nullptr, *cell_first = nullptr;  // all buffers sized by the points, the cell table
+    size_t work_cap = 0, cell_cap = 0;
+    char *host = nullptr;  // pinned: the points on their way in, indices and clusters on their way out
+    size_t host_cap = 0;
 };
 
 namespace {
 
-constexpr long long kMaxCells = 1LL << 28;  // dense cell table (4 B per cell) of one cloud, at most
+constexpr long long kMaxCells = 1LL << 28;  // dense cell table (4 B per cell), at most
+constexpr int kCopyPoints = 1 << 14;  // points per copy to the device (192 KiB)
 
 int fail(ndt_ec *h, int code, const std::string &msg) {
     if (h) h->err = msg;
@@ -315,116 +406,156 @@ cudaError_t ensure(void **p, size_t *cap, size_t bytes) {
         if (e_ != cudaSuccess) return fail(h, NDT_E_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
-// Component labels of up to kMaxParts clouds in one pass: labels[p][i] is the
-// smallest index within cloud p of point i's component (clouds never join).
-int labels_of(ndt_ec *h, const std::vector<const float *> &xyz, const std::vector<int> &n,
-              const std::vector<float> &tolerance, std::vector<std::vector<int>> &labels) {
+// One pass over the points of C.count clouds (C.off[C.count] of them, tolerance[r]
+// for ring r).  by_cluster: *index is the point indices, cluster by cluster, and
+// rec the clusters of [20, 100000] points in it, by smallest point index;
+// otherwise *index is every point's label, the smallest index of its component
+// (parts never join).  *points are the handle's copy of the points (the output
+// may overlay the input); both are valid until the handle's next call.
+constexpr int kMinCluster = 20, kMaxCluster = 100000;
+
+int cluster_pass(ndt_ec *h, const float *xyz, const ec::Clouds &C, const float *tolerance, bool by_cluster,
+                 const float **points, const int **index, std::vector<int2> &rec) {
     ndt::NvtxRange range("ec labels");
-    const int np = (int)xyz.size();
-    labels.assign(np, std::vector<int>());
+    rec.clear();
+    const int np = C.count * C.rings, N = C.off[C.count];
+    if (N == 0) return NDT_OK;
+    cudaStream_t st = h->stream;
+
+    // one device and one pinned block, cut into 256-byte aligned pieces
+    size_t bytes = 0;
+    auto piece = [&bytes](size_t b) {
+        const size_t at = bytes;
+        bytes += (b + 255) / 256 * 256;
+        return at;
+    };
+    const size_t max_rec = (size_t)N / kMinCluster + 1;
+    const size_t o_boxes = piece(sizeof(ec::Box) * ec::kMaxParts), o_status = piece(2 * sizeof(int)),
+                 o_rec = piece(sizeof(int2) * max_rec), o_xyz = piece(3 * sizeof(float) * (size_t)N);
+    const size_t host_bytes = bytes + sizeof(int) * (size_t)N;  // the indices come last
+    const size_t o_pts = piece(sizeof(float4) * (size_t)N), o_sorted = piece(sizeof(float4) * (size_t)N),
+                 o_parent = piece(sizeof(int) * (size_t)N), o_least = piece(sizeof(int) * (size_t)N),
+                 o_start = piece(sizeof(int) * (size_t)N), o_key = piece(sizeof(int) * (size_t)N),
+                 o_sort = piece(ndt::sort_scratch_bytes(N));
+    ECK(ensure(&h->work, &h->work_cap, bytes));
+    if (h->host_cap < host_bytes) {
+        if (h->host) cudaFreeHost(h->host);
+        h->host = nullptr;
+        h->host_cap = 0;
+        ECK(cudaMallocHost((void **)&h->host, host_bytes + host_bytes / 2));
+        h->host_cap = host_bytes + host_bytes / 2;
+    }
+    char *dev = (char *)h->work;
+    ec::Box *boxes = (ec::Box *)(dev + o_boxes), *h_boxes = (ec::Box *)(h->host + o_boxes);
+    int *status = (int *)(dev + o_status), *err = status + 1, *h_status = (int *)(h->host + o_status);
+    int2 *d_rec = (int2 *)(dev + o_rec), *h_rec = (int2 *)(h->host + o_rec);
+    float *d_xyz = (float *)(dev + o_xyz), *h_xyz = (float *)(h->host + o_xyz);
+    int *h_index = (int *)(h->host + host_bytes - sizeof(int) * (size_t)N);
+    float4 *pts = (float4 *)(dev + o_pts), *sorted = (float4 *)(dev + o_sorted);
+    int *parent = (int *)(dev + o_parent), *least = (int *)(dev + o_least);
+    int32_t *seg_start = (int32_t *)(dev + o_start);
+    uint32_t *seg_key = (uint32_t *)(dev + o_key);
+    ndt::SortBuffers sb = ndt::sort_buffers(dev + o_sort, N);
+    const unsigned blocks = (unsigned)((N + ec::kThreads - 1) / ec::kThreads);
+
+    // parts and boxes; the points go over in pieces, so that the copy into the
+    // pinned block runs beside the one to the device
+    for (int q = 0; q < np; ++q)
+        h_boxes[q] = {{INT_MAX, INT_MAX, INT_MAX}, {INT_MIN, INT_MIN, INT_MIN}, 0, 0};
+    h_status[0] = h_status[1] = 0;
+    ECK(cudaMemcpyAsync(boxes, h_boxes, o_status + 2 * sizeof(int) - o_boxes, cudaMemcpyHostToDevice, st));
+    for (int i = 0; i < N; i += kCopyPoints) {
+        const size_t at = 3 * (size_t)i, len = 3 * sizeof(float) * (size_t)std::min(kCopyPoints, N - i);
+        std::memcpy(h_xyz + at, xyz + at, len);
+        ECK(cudaMemcpyAsync(d_xyz + at, h_xyz + at, len, cudaMemcpyHostToDevice, st));
+    }
+    ec::part_kernel<<<blocks, ec::kThreads, 0, st>>>(d_xyz, N, C, pts, boxes);
+    ECK(cudaGetLastError());
+    ECK(cudaMemcpyAsync(h_boxes, boxes, sizeof(ec::Box) * np, cudaMemcpyDeviceToHost, st));
+    ECK(cudaStreamSynchronize(st));
+
     ec::Parts P;
     std::memset(&P, 0, sizeof(P));
-    P.np = np;
-    long long total = 0, cells = 0;
+    long long cells = 0;
     for (int q = 0; q < np; ++q) {
-        P.off[q] = (int)total;
+        const ec::Box &b = h_boxes[q];
+        const float tol = tolerance[q % C.rings];
         P.base[q] = cells;
-        total += n[q];
-        labels[q].assign(n[q], 0);
-        float mn[3] = {0.0f, 0.0f, 0.0f}, mx[3] = {0.0f, 0.0f, 0.0f};
-        for (int i = 0; i < n[q]; ++i) {
-            const float *v = xyz[q] + 3 * (size_t)i;
-            if (!std::isfinite(v[0]) || !std::isfinite(v[1]) || !std::isfinite(v[2]))
-                return fail(h, NDT_E_ARG, "non-finite point coordinates");
-            for (int k = 0; k < 3; ++k) {
-                mn[k] = i ? std::min(mn[k], v[k]) : v[k];
-                mx[k] = i ? std::max(mx[k], v[k]) : v[k];
-            }
-        }
-        P.cell[q] = tolerance[q] * 1.0001f;  // cells a little wider than the radius
-        P.r2[q] = tolerance[q] * tolerance[q];
+        P.cell[q] = tol * 1.0001f;  // cells a little wider than the radius
+        P.r2[q] = tol * tol;
+        if (!b.points) continue;
+        if (b.bad) return fail(h, NDT_E_ARG, "non-finite point coordinates");
         long long G = 1;
         for (int k = 0; k < 3; ++k) {
-            P.minv[q][k] = mn[k];
-            const double d = std::floor(((double)mx[k] - (double)mn[k]) / (double)P.cell[q]) + 1.0;
+            const int lo = ec::ordered(b.lo[k]), hi = ec::ordered(b.hi[k]);
+            float mn, mx;
+            std::memcpy(&mn, &lo, sizeof(mn));
+            std::memcpy(&mx, &hi, sizeof(mx));
+            P.minv[q][k] = mn;
+            const double d = std::floor(((double)mx - (double)mn) / (double)P.cell[q]) + 1.0;
             if (!(d >= 1.0 && d < 2147483647.0)) return fail(h, NDT_E_CAPACITY, "a cloud spans too many cells");
             P.dim[q][k] = (int)d;
             G *= P.dim[q][k];
             if (G > kMaxCells) break;
         }
-        cells += n[q] ? G : 0;
+        cells += G;
         if (cells > kMaxCells) return fail(h, NDT_E_CAPACITY, "the clouds span more than 2^28 cells of the tolerance");
     }
-    P.off[np] = (int)total;
     P.base[np] = cells;
-    const int N = (int)total;
-    if (N == 0) return NDT_OK;
-    cudaStream_t st = h->stream;
-    if (h->h_cap < (size_t)N) {
-        if (h->h_pts) cudaFreeHost(h->h_pts);
-        if (h->h_labels) cudaFreeHost(h->h_labels);
-        h->h_pts = nullptr;
-        h->h_labels = nullptr;
-        h->h_cap = 0;
-        const size_t want = (size_t)N + N / 2;
-        ECK(cudaMallocHost((void **)&h->h_pts, sizeof(float4) * want));
-        ECK(cudaMallocHost((void **)&h->h_labels, sizeof(int) * want));
-        h->h_cap = want;
-    }
-    for (int q = 0; q < np; ++q)
-        for (int i = 0; i < n[q]; ++i) {
-            const float *v = xyz[q] + 3 * (size_t)i;
-            h->h_pts[P.off[q] + i] = make_float4(v[0], v[1], v[2], 0.0f);
-        }
-    int bits = 1;
-    while (bits < 31 && (1LL << bits) < cells) ++bits;
-    ECK(ensure(&h->pts, &h->pts_cap, sizeof(float4) * (size_t)N));
-    ECK(ensure(&h->sorted, &h->sorted_cap, sizeof(float4) * (size_t)N));
-    ECK(ensure(&h->scratch, &h->scratch_cap, ndt::sort_scratch_bytes(N)));
-    ECK(ensure(&h->parent, &h->parent_cap, 3 * sizeof(int) * (size_t)N));
-    ECK(ensure(&h->seg_start, &h->seg_start_cap, sizeof(int) * (size_t)N));
-    ECK(ensure(&h->seg_key, &h->seg_key_cap, sizeof(int) * (size_t)N));
+    auto bits_for = [](long long values) {
+        int bits = 1;
+        while (bits < 31 && (1LL << bits) < values) ++bits;
+        return bits;
+    };
     ECK(ensure(&h->cell_first, &h->cell_cap, sizeof(int) * (size_t)cells));
-    size_t fcap = 0;
-    if (!h->flags) ECK(ensure(&h->flags, &fcap, 256));
-    float4 *d_pts = (float4 *)h->pts;
-    int *parent = (int *)h->parent, *least = parent + N, *label = least + N, *err = (int *)h->flags;
-    ECK(cudaMemcpyAsync(d_pts, h->h_pts, sizeof(float4) * (size_t)N, cudaMemcpyHostToDevice, st));
-    ECK(cudaMemsetAsync(err, 0, sizeof(int), st));
-    ECK(cudaMemsetAsync(h->cell_first, 0xff, sizeof(int) * (size_t)cells, st));
-    ndt::SortBuffers sb = ndt::sort_buffers(h->scratch, N);
-    const unsigned blocks = (unsigned)((N + ec::kThreads - 1) / ec::kThreads);
-    ec::key_kernel<<<blocks, ec::kThreads, 0, st>>>(d_pts, N, P, sb.k0, least);
-    ndt::sort_segments(sb, N, bits, (int32_t *)h->seg_start, (uint32_t *)h->seg_key, st, true);
-    ec::gather_kernel<<<blocks, ec::kThreads, 0, st>>>(d_pts, sb.v0, N, (const uint32_t *)h->seg_key, sb.nseg,
-                                                       (float4 *)h->sorted, (int *)h->cell_first);
-    const float4 *sorted = (const float4 *)h->sorted;
-    const int32_t *seg_start = (const int32_t *)h->seg_start;
-    const int *cell_first = (const int *)h->cell_first;
+    int *cell_first = (int *)h->cell_first;
+    ECK(cudaMemsetAsync(cell_first, 0xff, sizeof(int) * (size_t)cells, st));
+    ec::key_kernel<<<blocks, ec::kThreads, 0, st>>>(pts, N, P, sb.k0, least);
+    ndt::sort_segments(sb, N, bits_for(cells), seg_start, seg_key, st, true);
+    ec::gather_kernel<<<blocks, ec::kThreads, 0, st>>>(pts, sb.v0, N, seg_key, sb.nseg, sorted, cell_first);
     const unsigned per_block = ec::kThreads / 32, wide = (N + per_block - 1) / per_block;
     ec::hook_kernel<<<wide, ec::kThreads, 0, st>>>(sorted, sb.k0, N, seg_start, sb.nseg, cell_first, P, parent);
-    ec::root_kernel<<<blocks, ec::kThreads, 0, st>>>(parent, N, err);
+    ec::root_kernel<<<blocks, ec::kThreads, 0, st>>>(parent, N, sb.nseg, err);
     ec::join_kernel<<<wide, ec::kThreads, 0, st>>>(sorted, sb.k0, N, seg_start, sb.nseg, cell_first, P, parent, err);
-    ec::least_kernel<<<blocks, ec::kThreads, 0, st>>>(parent, sb.v0, N, least, err);
-    ec::label_kernel<<<blocks, ec::kThreads, 0, st>>>(parent, sb.v0, N, least, label);
+    ec::least_kernel<<<blocks, ec::kThreads, 0, st>>>(parent, sb.v0, N, sb.nseg, least, err);
+    ec::label_kernel<<<blocks, ec::kThreads, 0, st>>>(parent, sb.v0, N, sb.nseg, least, ndt::sort_error(sb, N), sb.k0,
+                                                      status);
+    if (by_cluster) {
+        ndt::sort_segments(sb, N, bits_for(N), seg_start, seg_key, st, true);
+        ec::cluster_kernel<<<blocks, ec::kThreads, 0, st>>>(seg_start, sb.nseg, N, kMinCluster, kMaxCluster,
+                                                            ndt::sort_error(sb, N), d_rec, status);
+    }
     ECK(cudaGetLastError());
-    ECK(cudaMemcpyAsync(h->h_labels, label, sizeof(int) * (size_t)N, cudaMemcpyDeviceToHost, st));
-    int e = 0, sort_err = 0;
-    ECK(cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, st));
-    ECK(cudaMemcpyAsync(&sort_err, ndt::sort_error(sb, N), sizeof(int), cudaMemcpyDeviceToHost, st));
+    ECK(cudaMemcpyAsync(h_status, status, by_cluster ? o_rec + sizeof(int2) * max_rec - o_status : 2 * sizeof(int),
+                        cudaMemcpyDeviceToHost, st));
+    ECK(cudaMemcpyAsync(h_index, by_cluster ? sb.v0 : sb.k0, sizeof(int) * (size_t)N, cudaMemcpyDeviceToHost, st));
     ECK(cudaStreamSynchronize(st));
-    if (sort_err) return fail(h, NDT_E_CUDA, "a wait between the sort's tiles gave up");
-    if (e) return fail(h, NDT_E_CUDA, "union-find retry limit reached");
-    for (int q = 0; q < np; ++q)
-        for (int i = 0; i < n[q]; ++i) labels[q][i] = h->h_labels[P.off[q] + i] - P.off[q];
+    if (h_status[1] & 4) return fail(h, NDT_E_CUDA, "a wait between the sort's tiles gave up");
+    if (h_status[1]) return fail(h, NDT_E_CUDA, "union-find retry limit reached");
+    *points = h_xyz;
+    *index = h_index;
+    if (by_cluster) {
+        rec.assign(h_rec, h_rec + h_status[0]);
+        std::sort(rec.begin(), rec.end(), [](int2 a, int2 b) { return a.x < b.x; });
+    }
     return NDT_OK;
+}
+
+// Labels of one cloud.
+int labels_of(ndt_ec *h, const float *xyz, int n, float tolerance, const int **labels) {
+    ec::Clouds C;
+    std::memset(&C, 0, sizeof(C));
+    C.count = C.rings = 1;
+    C.off[1] = n;
+    const float *points;
+    std::vector<int2> none;
+    return cluster_pass(h, xyz, C, &tolerance, false, &points, labels, none);
 }
 
 // The reference's clusters from component labels: components in order of
 // their smallest index, indices ascending, sizes in [lo, hi], then ordered by
 // size with std::sort over reverse iterators (extract, kernel.cpp:635-647).
-void clusters_of(const std::vector<int> &labels, int lo, int hi, std::vector<std::vector<int>> &out) {
-    const int n = (int)labels.size();
+void clusters_of(const int *labels, int n, int lo, int hi, std::vector<std::vector<int>> &out) {
     std::vector<int> size(n, 0), slot(n, -1);
     for (int i = 0; i < n; ++i) ++size[labels[i]];
     out.clear();
@@ -464,10 +595,9 @@ void ndt_ec_destroy(ndt_ec *h) {
     if (!h) return;
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
-    for (void *p : {h->pts, h->sorted, h->scratch, h->parent, h->seg_start, h->seg_key, h->cell_first, h->flags})
+    for (void *p : {h->work, h->cell_first})
         if (p) cudaFree(p);
-    if (h->h_pts) cudaFreeHost(h->h_pts);
-    if (h->h_labels) cudaFreeHost(h->h_labels);
+    if (h->host) cudaFreeHost(h->host);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
 }
@@ -478,9 +608,9 @@ int ndt_ec_labels(ndt_ec *h, const float *xyz, int n, float tolerance, int *labe
     if (!h || n < 0 || (n > 0 && (!xyz || !labels)) || !(tolerance > 0.0f) || !std::isfinite(tolerance))
         return fail(h, NDT_E_ARG, "bad argument");
     ECK(cudaSetDevice(h->device));
-    std::vector<std::vector<int>> lab;
-    if (int rc = labels_of(h, {xyz}, {n}, {tolerance}, lab)) return rc;
-    if (n) std::memcpy(labels, lab[0].data(), sizeof(int) * (size_t)n);
+    const int *lab = nullptr;
+    if (int rc = labels_of(h, xyz, n, tolerance, &lab)) return rc;
+    if (n) std::memcpy(labels, lab, sizeof(int) * (size_t)n);
     return NDT_OK;
 }
 
@@ -490,10 +620,10 @@ int ndt_ec_extract(ndt_ec *h, const float *xyz, int n, float tolerance, int min_
         !(tolerance > 0.0f) || !std::isfinite(tolerance))
         return fail(h, NDT_E_ARG, "bad argument");
     ECK(cudaSetDevice(h->device));
-    std::vector<std::vector<int>> lab;
-    if (int rc = labels_of(h, {xyz}, {n}, {tolerance}, lab)) return rc;
+    const int *lab = nullptr;
+    if (int rc = labels_of(h, xyz, n, tolerance, &lab)) return rc;
     std::vector<std::vector<int>> cl;
-    clusters_of(lab[0], min_size, max_size, cl);
+    clusters_of(lab, n, min_size, max_size, cl);
     int pos = 0;
     cluster_offsets[0] = 0;
     for (size_t c = 0; c < cl.size(); ++c) {
@@ -513,75 +643,53 @@ int ndt_ec_extract(ndt_ec *h, const float *xyz, int n, float tolerance, int min_
 namespace {
 int segment_clouds(ndt_ec *h, const float *xyz, const int *offsets, int c0, int c1, float *out_xyz, int *out_off,
                    double *boxes, int *box_off, double *centroids, int &np, int &nb) {
-    const double tol[5] = {0.5, 1.1, 1.6, 2.3, 2.6f};
-    const int C = c1 - c0;
-    std::vector<std::vector<float>> ring(5 * (size_t)C);
-    for (int c = 0; c < C; ++c)
-        for (int i = offsets[c0 + c]; i < offsets[c0 + c + 1]; ++i) {
-            const float *q = xyz + 3 * (size_t)i;
-            const float x = q[0], y = q[1];
-            const float d = std::sqrt(x * x + y * y);
-            const int r = d < 15 ? 0 : (d < 30 ? 1 : (d < 45 ? 2 : (d < 60 ? 3 : 4)));
-            ring[5 * (size_t)c + r].insert(ring[5 * (size_t)c + r].end(), q, q + 3);
-        }
-    std::vector<const float *> parts;
-    std::vector<int> sizes;
-    std::vector<float> tols;
-    for (int k = 0; k < 5 * C; ++k) {
-        parts.push_back(ring[k].data());
-        sizes.push_back((int)(ring[k].size() / 3));
-        tols.push_back((float)tol[k % 5]);
+    const float tol[ec::kRings] = {0.5f, 1.1f, 1.6f, 2.3f, 2.6f};
+    ec::Clouds C;
+    std::memset(&C, 0, sizeof(C));
+    C.count = c1 - c0;
+    C.rings = ec::kRings;
+    for (int c = 0; c <= C.count; ++c) C.off[c] = offsets[c0 + c] - offsets[c0];
+    const float *points = nullptr;
+    const int *index = nullptr;
+    std::vector<int2> rec;  // every ring of every cloud in one pass
+    if (int rc = cluster_pass(h, xyz + 3 * (size_t)offsets[c0], C, tol, true, &points, &index, rec)) return rc;
+    // by part, in order of the smallest index, then by size as extract() orders them
+    std::vector<std::vector<int2>> part((size_t)C.count * ec::kRings);
+    for (int2 r : rec) {
+        const int i = index[r.x];
+        const float *q = points + 3 * (size_t)i;
+        part[(size_t)ec::kRings * ec::cloud_of(C, i) + ec::ring_of(q[0], q[1])].push_back(r);
     }
-    std::vector<std::vector<int>> lab;
-    if (int rc = labels_of(h, parts, sizes, tols, lab)) return rc;  // every ring of every cloud in one pass
-    std::vector<std::vector<int>> cl;
-    std::vector<ec::YawJob> yaw;
-    for (int c = 0; c < C; ++c) {
+    std::vector<ec::ClusterJob> jobs;
+    jobs.reserve(rec.size());
+    std::vector<size_t> first(C.count + 1, 0);  // each cloud's first cluster
+    for (int c = 0; c < C.count; ++c) {
         out_off[c0 + c] = np;
-        box_off[c0 + c] = nb;
-        for (int r = 0; r < 5; ++r) {
-            const std::vector<float> &pts = ring[5 * (size_t)c + r];
-            if (pts.empty()) continue;
-            clusters_of(lab[5 * (size_t)c + r], 20, 100000, cl);
-            for (const std::vector<int> &idx : cl) {
-                double cen[3] = {0.0, 0.0, 0.0};
-                float lo[3] = {std::numeric_limits<float>::max(), std::numeric_limits<float>::max(),
-                               std::numeric_limits<float>::max()};
-                float hi[3] = {-lo[0], -lo[1], -lo[2]};
-                for (int i : idx) {
-                    const float *p = &pts[3 * (size_t)i];
-                    for (int k = 0; k < 3; ++k) {
-                        out_xyz[3 * (size_t)np + k] = p[k];
-                        cen[k] += p[k];
-                        if (p[k] < lo[k]) lo[k] = p[k];
-                        if (p[k] > hi[k]) hi[k] = p[k];
-                    }
-                    ++np;
-                }
-                for (int k = 0; k < 3; ++k) cen[k] /= idx.size();
-                const float l = hi[0] - lo[0], w = hi[1] - lo[1], ht = hi[2] - lo[2];
-                const double dim[3] = {l < 0 ? -1 * l : l, w < 0 ? -1 * w : w, ht < 0 ? -1 * ht : ht};
-                if (dim[0] > 0 && dim[1] > 0 && dim[2] > 0 && dim[0] < 15 && dim[1] > 0 && dim[1] < 15 &&
-                    hi[2] > -1.5 && lo[2] > -1.5 && lo[2] < 1.0) {
-                    // position, orientation (x, y, z, w: z and w by the yaw pass below), dimensions
-                    const double b[10] = {lo[0] + l / 2, lo[1] + w / 2, lo[2] + ht / 2, 0.0, 0.0, 0.0, 1.0,
-                                          dim[0], dim[1], dim[2]};
-                    std::memcpy(boxes + 10 * (size_t)nb, b, sizeof(b));
-                    // the yaw only of kept boxes: the others are not output
-                    yaw.push_back({out_xyz + 3 * (size_t)(np - (int)idx.size()), (int)idx.size(), lo[0], lo[1],
-                                   boxes + 10 * (size_t)nb + 5, boxes + 10 * (size_t)nb + 6});
-                    std::memcpy(centroids + 3 * (size_t)nb, cen, sizeof(cen));
-                    ++nb;
-                }
+        for (int r = 0; r < ec::kRings; ++r) {
+            std::vector<int2> &cl = part[(size_t)ec::kRings * c + r];
+            std::sort(cl.rbegin(), cl.rend(), [](const int2 &a, const int2 &b) { return a.y < b.y; });
+            for (int2 k : cl) {
+                jobs.push_back({index + k.x, k.y, out_xyz + 3 * (size_t)np});
+                np += k.y;
             }
         }
+        first[c + 1] = jobs.size();
     }
     out_off[c1] = np;
-    box_off[c1] = nb;
     {
-        ndt::NvtxRange range("ec yaw");
-        ec::box_yaws(yaw.data(), (int)yaw.size());
+        ndt::NvtxRange range("ec boxes");
+        ec::finish_clusters(points, jobs.data(), (int)jobs.size());
     }
+    for (int c = 0; c < C.count; ++c) {
+        box_off[c0 + c] = nb;
+        for (size_t j = first[c]; j < first[c + 1]; ++j) {
+            if (!jobs[j].kept) continue;
+            std::memcpy(boxes + 10 * (size_t)nb, jobs[j].box, sizeof(jobs[j].box));
+            std::memcpy(centroids + 3 * (size_t)nb, jobs[j].centroid, sizeof(jobs[j].centroid));
+            ++nb;
+        }
+    }
+    box_off[c1] = nb;
     return NDT_OK;
 }
 }  // namespace

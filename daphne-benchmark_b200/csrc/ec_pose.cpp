@@ -249,18 +249,55 @@ void box_yaw(const float *xyz, int n, float min_x, float min_y, double *qz, doub
 // passes on one thread.
 std::atomic<pid_t> g_pool_owner{0};
 
+// Threads for `count` clusters: at most kYawThreads, at most the cores there are.
+int pool_threads(int count) {
+    const int threads = std::max(1, std::min(kYawThreads, omp_get_num_procs()));
+    if (count <= 4 || threads == 1) return 1;
+    const pid_t me = getpid();
+    pid_t none = 0;
+    g_pool_owner.compare_exchange_strong(none, me);
+    return g_pool_owner.load() == me ? threads : 1;
+}
+
 void box_yaws(const YawJob *jobs, int count) {
-    // independent clusters over the host's threads (at most kYawThreads, at most the cores there are), in a
-    // dynamic schedule of small chunks so that one large cluster does not hold up the others' threads
-    int threads = std::max(1, std::min(kYawThreads, omp_get_num_procs()));
-    if (count > 4 && threads > 1) {
-        const pid_t me = getpid();
-        pid_t none = 0;
-        g_pool_owner.compare_exchange_strong(none, me);
-        if (g_pool_owner.load() != me) threads = 1;
-    }
-#pragma omp parallel for schedule(dynamic, 2) num_threads(threads) if (count > 4 && threads > 1)
+    // a dynamic schedule of small chunks, so that one large cluster does not hold up the others' threads
+    const int threads = pool_threads(count);
+#pragma omp parallel for schedule(dynamic, 2) num_threads(threads) if (threads > 1)
     for (int j = 0; j < count; ++j) box_yaw(jobs[j].xyz, jobs[j].n, jobs[j].min_x, jobs[j].min_y, jobs[j].qz, jobs[j].qw);
+}
+
+static void finish_cluster(const float *xyz, ClusterJob &job) {
+    double cen[3] = {0.0, 0.0, 0.0};
+    float lo[3] = {std::numeric_limits<float>::max(), std::numeric_limits<float>::max(),
+                   std::numeric_limits<float>::max()};
+    float hi[3] = {-lo[0], -lo[1], -lo[2]};
+    for (int i = 0; i < job.n; ++i) {
+        const float *p = xyz + 3 * (size_t)job.idx[i];
+        for (int k = 0; k < 3; ++k) {
+            job.out[3 * (size_t)i + k] = p[k];
+            cen[k] += p[k];
+            if (p[k] < lo[k]) lo[k] = p[k];
+            if (p[k] > hi[k]) hi[k] = p[k];
+        }
+    }
+    for (int k = 0; k < 3; ++k) job.centroid[k] = cen[k] / (size_t)job.n;
+    const float l = hi[0] - lo[0], w = hi[1] - lo[1], ht = hi[2] - lo[2];
+    const double dim[3] = {l < 0 ? -1 * l : l, w < 0 ? -1 * w : w, ht < 0 ? -1 * ht : ht};
+    job.kept = dim[0] > 0 && dim[1] > 0 && dim[2] > 0 && dim[0] < 15 && dim[1] > 0 && dim[1] < 15 && hi[2] > -1.5 &&
+               lo[2] > -1.5 && lo[2] < 1.0;
+    if (!job.kept) return;  // no yaw of boxes that are not output
+    const double b[10] = {lo[0] + l / 2, lo[1] + w / 2, lo[2] + ht / 2, 0.0, 0.0, 0.0, 1.0, dim[0], dim[1], dim[2]};
+    std::copy(b, b + 10, job.box);
+    box_yaw(job.out, job.n, lo[0], lo[1], &job.box[5], &job.box[6]);
+}
+
+void finish_clusters(const float *xyz, ClusterJob *jobs, int count) {
+    const int threads = pool_threads(count);
+    std::vector<int> largest_first(count);
+    for (int j = 0; j < count; ++j) largest_first[j] = j;
+    std::stable_sort(largest_first.begin(), largest_first.end(), [&](int a, int b) { return jobs[a].n > jobs[b].n; });
+#pragma omp parallel for schedule(dynamic, 1) num_threads(threads) if (threads > 1)
+    for (int j = 0; j < count; ++j) finish_cluster(xyz, jobs[largest_first[j]]);
 }
 
 }  // namespace ec

@@ -15,4 +15,18 @@ struct YawJob {
     double *qz, *qw;
 };
 void box_yaws(const YawJob *jobs, int count);
+
+// One cluster of the segmentation: the n points idx[] of xyz are written to out
+// in that order, with their centroid and, where the reference keeps one
+// (clusterAndColor, kernel.cpp:652-765), their box: position, orientation
+// (x, y, z, w) and dimensions.  Spread over the same host threads.
+struct ClusterJob {
+    const int *idx;
+    int n;
+    float *out;
+    bool kept;
+    double centroid[3];
+    double box[10];
+};
+void finish_clusters(const float *xyz, ClusterJob *jobs, int count);
 }  // namespace ec
