@@ -170,7 +170,7 @@ struct ndt_ctx {
     // batch
     DevBuf chunks, chunk_begin, num_chunks, big_begin, small_begin, num_big, dev_launches;
     DevBuf points, offsets, guesses, states, tiles, tile_begin, num_tiles, partials, exc, out_T, out_conv, out_fit,
-        out_status, ctl, p6, trans, flag_q, active_chunks, lane_sums, split_state;
+        out_status, ctl, p6, trans, queues, active_chunks, split_state;
     HostBuf h_offsets, h_active, h_counters, h_out;
     ndt_counters last{};
     long long launches = 0;
@@ -473,25 +473,26 @@ constexpr unsigned kFlagCap = 1u << 20;     // default side-queue capacity (pair
 constexpr unsigned kFlagCapMax = 1u << 24;  // largest capacity ndt_set_side_queue_capacity accepts
 
 int prepare_scratch(ndt_ctx *c, EvalArgs &ea) {
-    CK(c->flag_q.ensure(sizeof(int4) * c->flag_cap));
+    const int tile = kDerivVariants[c->variant].tile;
+    const int wide = wide_chunk_limit(c->num_sms, tile);
+    const size_t slots = (size_t)wide_chunk_limit(c->num_sms, 32);  // columns, and more than any tile's chunks
+    // the wide kernel's lane sums and the FP64 side queue in one buffer: an
+    // allocation costs a new context 0.36 ms whatever its size
+    const size_t lane_bytes = (sizeof(float) * kWideFloats * slots + 255) / 256 * 256;
+    CK(c->queues.ensure(lane_bytes + sizeof(int4) * c->flag_cap));
+    ea.lane_sums = c->queues.as<float>();
+    ea.flag_q = reinterpret_cast<int4 *>(c->queues.as<char>() + lane_bytes);
     CK(c->ctl.ensure(sizeof(RoundCtl)));
     RoundCtl *ctl = c->ctl.as<RoundCtl>();
-    ea.flag_q = c->flag_q.as<int4>();
     ea.flag_n = &ctl->flag_n;
     ea.flag_cap = c->flag_cap;
     ea.flag_overflow = &ctl->flag_overflow;
     ea.work_counter = &ctl->work_counter;
     ea.counters = &ctl->counters;
-    // the wide kernel's scratch
-    const int tile = kDerivVariants[c->variant].tile;
-    const int wide = wide_chunk_limit(c->num_sms, tile);
-    const size_t slots = (size_t)wide_chunk_limit(c->num_sms, 32);  // columns, and more than any tile's chunks
-    CK(c->lane_sums.ensure(sizeof(float) * kWideFloats * slots));
     if (!c->split_state.p) {
         CK(c->split_state.ensure(2 * sizeof(int) * slots));
         CK(cudaMemsetAsync(c->split_state.p, 0, 2 * sizeof(int) * slots, c->stream));
     }
-    ea.lane_sums = c->lane_sums.as<float>();
     ea.split_state = c->split_state.as<int>();
     ea.wide_chunks = wide;
     return NDT_OK;
@@ -1091,7 +1092,7 @@ void ndt_destroy(ndt_ctx *c) {
                       &c->big_begin, &c->small_begin, &c->num_big, &c->dev_launches,
                       &c->partials, &c->exc, &c->out_T, &c->out_conv,
                       &c->out_fit, &c->out_status, &c->ctl, &c->p6, &c->trans,
-                      &c->flag_q, &c->active_chunks, &c->lane_sums, &c->split_state};
+                      &c->queues, &c->active_chunks, &c->split_state};
     for (DevBuf *b : bufs) b->release();
     HostBuf *hb[] = {&c->h_offsets, &c->h_active, &c->h_counters, &c->h_out};
     for (HostBuf *b : hb) b->release();
