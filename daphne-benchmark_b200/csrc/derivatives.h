@@ -37,13 +37,13 @@ struct EvalArgs {  // (GridDev is in ndt_types.h)
     bool reset = true;     // launch_derivatives clears flag_n and work_counter (else the caller has)
     // FP32 pass: with at most wide_chunks chunks to evaluate, the wide kernel
     // takes them (derivatives_wide.cu; 0: never), which needs the lane sums of
-    // its columns (kWideFloats per column of wide_chunks chunks) and two
-    // counters per chunk (zero between passes).  min_chunks: a host-side lower
+    // its columns (kWideFloats per column of wide_chunks chunks) and a
+    // counter per chunk (zero between passes).  min_chunks: a host-side lower
     // bound of the chunks of every pass (0: none).
     int wide_chunks = 0;
     int min_chunks = 0;
     float *lane_sums = nullptr;
-    int *split_state = nullptr;
+    unsigned long long *split_state = nullptr;
 };
 
 constexpr int kWideFloats = 37 * 32;  // 37 FP32 sums of 32 lanes

@@ -6,7 +6,10 @@
 // dependent gathers (window offsets, entries, pair records) of about 5 us,
 // while most SMs have nothing to do.  One 8000-point scan is 11 chunks: 46.6
 // us per evaluation on B200.  This kernel gives every tile column a warp of
-// its own: 15.2 us for the same bits.
+// its own: 15.2 us for the same bits, 13.1 with one atomic for a column's end
+// (its pairs and its count together, after one fence), none for blocks that
+// have no second item, and the first tile and point read beside the state.
+// Reading the pairs' records ahead into L1 gained nothing.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -111,6 +114,7 @@ __global__ void __launch_bounds__(kBlock, kWideResident) derivative_wide_kernel(
     // atomic each).  (No block takes more than `items` items; the bound only
     // guards against a corrupted counter.)
     for (int it = 0; it <= items; ++it) {
+        if (it > 0 && items <= (int)gridDim.x) break;  // every block had its own
         if (threadIdx.x == 0)
             s_item[parity] = it == 0 ? (int)blockIdx.x : (int)gridDim.x + atomicAdd(args.work_counter, 1);
         __syncthreads();
@@ -120,6 +124,14 @@ __global__ void __launch_bounds__(kBlock, kWideResident) derivative_wide_kernel(
         const int slot_k = item / W, w = item % W;
         const Chunk ck = args.chunks[active_chunk(args, slot_k)];
         const AlignState *st = args.states + ck.align;
+        // this warp's tile and point of the first group, beside the state
+        Tile first_tile = {};
+        float4 first_x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (ck.first + warp < ck.end) {
+            first_tile = args.tiles[ck.first + warp];
+            const int i = first_tile.start + 32 * w + lane;
+            if (i < first_tile.end) first_x = args.points[i];
+        }
         if (threadIdx.x == 0) s_mode = st->eval_mode;
         if (threadIdx.x < 12) s_T[threadIdx.x] = st->T[threadIdx.x];
         if (threadIdx.x < kAngle) s_ang[threadIdx.x] = st->angf[threadIdx.x];
@@ -148,11 +160,11 @@ __global__ void __launch_bounds__(kBlock, kWideResident) derivative_wide_kernel(
             unsigned n_probe = 0, n_occ = 0;
             int n = 0, tile_points = 0;
             if (mine) {
-                const Tile tile = args.tiles[ck.first + g + warp];
+                const Tile tile = g == 0 ? first_tile : args.tiles[ck.first + g + warp];
                 i = tile.start + 32 * w + lane;
                 const bool valid = i < tile.end;
                 tile_points = tile.end - tile.start;
-                if (valid) x = args.points[i];
+                if (valid) x = g == 0 ? first_x : args.points[i];
                 // transformPointCloud (kernel.cpp:397-400), float, left to right
                 if (args.trans) {
                     const float4 y = valid ? args.trans[i] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -319,17 +331,18 @@ __global__ void __launch_bounds__(kBlock, kWideResident) derivative_wide_kernel(
             }
         }
         // the last of the chunk's columns adds them up
-        __threadfence();
-        __syncthreads();
+        // (the barrier above has the block's lane sums before thread 0's fence)
         if (threadIdx.x == 0) {
-            if (s_pairs) atomicAdd(args.split_state + 2 * slot_k + 1, (int)s_pairs);
+            unsigned long long *state = args.split_state + slot_k;  // columns done << 32 | their pairs
+            const unsigned long long add = 1ull << 32 | s_pairs;
             s_pairs = 0;
             __threadfence();
-            s_last = atomicAdd(args.split_state + 2 * slot_k, 1) == W - 1;
+            const unsigned long long sum = atomicAdd(state, add) + add;
+            s_last = (int)(sum >> 32) == W;
             if (s_last) {
                 __threadfence();
-                s_chunk_pairs = (unsigned)atomicExch(args.split_state + 2 * slot_k + 1, 0);
-                args.split_state[2 * slot_k] = 0;
+                s_chunk_pairs = (unsigned)sum;
+                *state = 0ull;
             }
         }
         __syncthreads();

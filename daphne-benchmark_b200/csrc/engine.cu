@@ -490,10 +490,10 @@ int prepare_scratch(ndt_ctx *c, EvalArgs &ea) {
     ea.work_counter = &ctl->work_counter;
     ea.counters = &ctl->counters;
     if (!c->split_state.p) {
-        CK(c->split_state.ensure(2 * sizeof(int) * slots));
-        CK(cudaMemsetAsync(c->split_state.p, 0, 2 * sizeof(int) * slots, c->stream));
+        CK(c->split_state.ensure(sizeof(unsigned long long) * slots));
+        CK(cudaMemsetAsync(c->split_state.p, 0, sizeof(unsigned long long) * slots, c->stream));
     }
-    ea.split_state = c->split_state.as<int>();
+    ea.split_state = c->split_state.as<unsigned long long>();
     ea.wide_chunks = wide;
     return NDT_OK;
 }
