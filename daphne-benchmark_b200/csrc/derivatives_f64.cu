@@ -1,7 +1,8 @@
 // The FP64 derivative pass (precision = 1): every (point, voxel) pair is
-// evaluated with the reference's literal FP64 expressions (updateDerivatives /
+// evaluated with the reference's FP64 operations, in its order (updateDerivatives /
 // updateHessian, src/CPU/ndt_mapping/kernel.cpp:438-493, 604-649, compat) or the
-// Magnusson eq. 6.13 Hessian (corrected), and accumulated in FP64.  The
+// Magnusson eq. 6.13 Hessian (corrected), and accumulated in FP64; products with
+// structural zeros are left out where the inverse covariance is finite.  The
 // neighbour search is the exact one of probe.cuh.  Compiled without
 // floating-point contraction, like the reference's x86-64 code.
 #include <cuda_runtime.h>
