@@ -38,10 +38,11 @@ struct EvalArgs {  // (GridDev is in ndt_types.h)
     // FP32 pass: with at most wide_chunks chunks to evaluate, the wide kernel
     // takes them (derivatives_wide.cu; 0: never), which needs the lane sums of
     // its columns (kWideFloats per column of wide_chunks chunks) and a
-    // counter per chunk (zero between passes).  min_chunks: a host-side lower
-    // bound of the chunks of every pass (0: none).
+    // counter per chunk (zero between passes).  expected_chunks: how many a pass
+    // has as far as the host can tell (0: no idea), from a bound of the points
+    // that the scans need not fill; it saves a launch and decides no result.
     int wide_chunks = 0;
-    int min_chunks = 0;
+    int expected_chunks = 0;
     float *lane_sums = nullptr;
     unsigned long long *split_state = nullptr;
 };
@@ -93,9 +94,12 @@ int launch_derivatives(const EvalArgs &args, int precision, int variant, int sms
 // The FP64 pass alone (256-point tiles).
 int launch_derivatives_f64(const EvalArgs &args, int sms, cudaStream_t st);
 // Kernel launches of one launch_derivatives call (FP32: one or both kernels of
-// the pass, and the flagged pairs; FP64: the pass).
-inline bool launches_wide(const EvalArgs &a) { return a.wide_chunks > 0 && a.min_chunks <= a.wide_chunks; }
-inline bool launches_many(const EvalArgs &a) { return a.max_tiles > a.wide_chunks; }
+// the pass, and the flagged pairs; FP64: the pass).  Where the wide kernel is
+// not launched (its empty launch is about 2 us a round), the other one takes
+// every pass, whatever its number of chunks; where both are, the number on the
+// device says which of them returns at once.
+inline bool launches_wide(const EvalArgs &a) { return a.wide_chunks > 0 && a.expected_chunks <= a.wide_chunks; }
+inline bool launches_many(const EvalArgs &a) { return !launches_wide(a) || a.max_tiles > a.wide_chunks; }
 inline int derivative_launches(const EvalArgs &a, int precision) {
     return precision == 1 ? 1 : 1 + (launches_wide(a) ? 1 : 0) + (launches_many(a) ? 1 : 0);
 }

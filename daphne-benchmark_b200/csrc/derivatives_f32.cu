@@ -484,14 +484,16 @@ int launch_derivatives(const EvalArgs &args, int precision, int variant, int sms
     }
     if (launches_wide(args)) launch_derivatives_wide(args, sms, st);
     if (launches_many(args)) {
+        EvalArgs many = args;
+        if (!launches_wide(args)) many.wide_chunks = 0;  // every pass is this kernel's
         switch (variant) {
-            case 0: launch_one<256, 2>(args, blocks, st); break;
-            case 1: launch_one<256, 1>(args, blocks, st); break;
-            case 2: launch_one<128, 4>(args, blocks, st); break;
-            case 3: launch_one<128, 3>(args, blocks, st); break;
-            case 5: launch_one<128, 5>(args, blocks, st); break;
-            case 6: launch_one<128, 6>(args, blocks, st); break;
-            default: launch_one<256, 3>(args, blocks, st); break;
+            case 0: launch_one<256, 2>(many, blocks, st); break;
+            case 1: launch_one<256, 1>(many, blocks, st); break;
+            case 2: launch_one<128, 4>(many, blocks, st); break;
+            case 3: launch_one<128, 3>(many, blocks, st); break;
+            case 5: launch_one<128, 5>(many, blocks, st); break;
+            case 6: launch_one<128, 6>(many, blocks, st); break;
+            default: launch_one<256, 3>(many, blocks, st); break;
         }
     }
     flagged_kernel<<<sms, 128, 0, st>>>(args);

@@ -724,8 +724,9 @@ int run_batch(ndt_ctx *c, int B, const float4 *d_points, const int *d_offsets, i
     // is fixed.
     R.fixed = R.P.compat && (R.P.step_max - R.P.step_min) > 0;
     R.max_rounds = R.fixed ? R.P.max_iterations + 3 : R.P.watchdog_evals + 1;
-    // every pass of a fixed batch hands out all its chunks, of at most kb tiles each
-    if (R.fixed) ea.min_chunks = total / (tile * R.kb);
+    // every pass of a fixed batch hands out all its chunks, of at most kb tiles
+    // each (fewer than this where `total` is a bound that the scans do not fill)
+    if (R.fixed) ea.expected_chunks = total / (tile * R.kb);
     if (!R.fixed && R.precision == 0) {
         // alignments finish at different rounds: each FP32 pass hands out only the chunks of active ones
         CK(c->active_chunks.ensure(sizeof(int) * (size_t)max_tiles));
@@ -1006,7 +1007,7 @@ int ctx_score_batch(ndt_ctx *c, int B, int scans, const float *d_points, const i
     R.precision = c->prm.precision;
     R.variant = c->variant;
     R.sms = c->num_sms;
-    ea.min_chunks = (int)(all_points / (tile * R.kb));
+    ea.expected_chunks = (int)(all_points / (tile * R.kb));  // (total_points is a bound)
     int np = 0;
     if (int rc = enqueue_prologue(c, R, st, &np)) return rc;
     int rc = launch_derivatives(R.ea, R.precision, R.variant, R.sms, st);
