@@ -157,15 +157,18 @@ __global__ void box_init_kernel(long long *__restrict__ box, int B) {
 // (base[B] = total), and the box reset for the next call.  flags[0] |= 1 when
 // a scan spans 2^31 leaves or more, |= 2 when the batch spans 2^31 - 1 or
 // more; flags[1] = total; flags[2], flags[3] = the largest leaf range and point
-// count of a scan.
+// count of a scan (INT_MAX when the offsets are not a partition of the n points
+// into scans: the boxes then hold each point in one scan, as the general path
+// takes them, and the ranges of points say something else).
 constexpr int kRangeThreads = 1024;
 
 __global__ void __launch_bounds__(kRangeThreads) range_kernel(long long *__restrict__ box, int B,
-                                                              const int *__restrict__ offsets,
+                                                              const int *__restrict__ offsets, int n,
                                                               ScanGeom *__restrict__ geom, int *__restrict__ base,
                                                               int *__restrict__ flags) {
     __shared__ long long s_sum[kRangeThreads];
     const int t = threadIdx.x;
+    if (t == 0 && (offsets[0] != 0 || offsets[B] != n)) atomicMax(flags + 3, INT_MAX);
     const int per = (B + kRangeThreads - 1) / kRangeThreads;
     const int b0 = t * per, b1 = b0 + per < B ? b0 + per : B;
     long long local = 0;
@@ -193,7 +196,8 @@ __global__ void __launch_bounds__(kRangeThreads) range_kernel(long long *__restr
         }
         atomicMax(flags + 2, (int)span);
         // (+ 1: a leaf that may hold all of a scan's points, which scan_kernel's 16-bit counts must not)
-        atomicMax(flags + 3, offsets[b + 1] - offsets[b] + (span <= 1 ? 1 : 0));
+        const int o0 = offsets[b], o1 = offsets[b + 1];
+        atomicMax(flags + 3, o0 >= 0 && o0 <= o1 && o1 <= n ? o1 - o0 + (span <= 1 ? 1 : 0) : INT_MAX);
         geom[b] = g;
         base[b] = (int)span;  // the range for now; the scan below makes it a base
         local += span;
@@ -267,6 +271,14 @@ inline bool scan_fits(int leaves, int n) {
 // 154 us against 111 / 134 / 150 / 185 / 250; 1 / 8 scans of 30000 points: 113
 // / 119 against 103 / 129; one of 2000: 80 against 96).
 inline bool scan_pays(int longest, int total) { return longest <= 20000 + total / 18; }
+
+// Whether a_bytes at a and b_bytes at b share any.  scan_kernel writes a scan's results
+// while other blocks still read theirs, so outputs over inputs (an in-place
+// call) take the general path, which has read all before it writes.
+inline bool overlap(const void *a, size_t a_bytes, const void *b, size_t b_bytes) {
+    const uintptr_t x = (uintptr_t)a, y = (uintptr_t)b;
+    return x < y + b_bytes && y < x + a_bytes;
+}
 
 struct ScanArgs {
     const float4 *pts;
@@ -774,7 +786,7 @@ int ndt_voxel_filter_device(ndt_filter *f, int B, const float *d_points, const i
             (const float4 *)d_points, d_offsets, B, n, r, box);
         FCK(cudaGetLastError());
     }
-    vf::range_kernel<<<1, vf::kRangeThreads, 0, st>>>(box, B, d_offsets, (vf::ScanGeom *)f->geom.p, base, flags);
+    vf::range_kernel<<<1, vf::kRangeThreads, 0, st>>>(box, B, d_offsets, n, (vf::ScanGeom *)f->geom.p, base, flags);
     FCK(cudaGetLastError());
     FCK(cudaMemcpyAsync(f->h_flags, flags, sizeof(int) * 4, cudaMemcpyDeviceToHost, st));
     FCK(cudaStreamSynchronize(st));
@@ -790,7 +802,12 @@ int ndt_voxel_filter_device(ndt_filter *f, int B, const float *d_points, const i
         return NDT_OK;
     }
     const int leaves = f->h_flags[2] > 0 ? f->h_flags[2] : 1, longest = f->h_flags[3];
-    if (vf::scan_fits(leaves, longest) && vf::scan_pays(longest, n)) {
+    const size_t pts_bytes = sizeof(float4) * (size_t)n, off_bytes = sizeof(int) * (size_t)(B + 1);
+    const bool in_place = vf::overlap(d_out, pts_bytes, d_points, pts_bytes) ||
+                          vf::overlap(d_out, pts_bytes, d_offsets, off_bytes) ||
+                          vf::overlap(d_out_offsets, off_bytes, d_points, pts_bytes) ||
+                          vf::overlap(d_out_offsets, off_bytes, d_offsets, off_bytes);
+    if (!in_place && vf::scan_fits(leaves, longest) && vf::scan_pays(longest, n)) {
         const size_t head = 256, bytes = head + sizeof(uint64_t) * (size_t)B;
         FCK(f->chain.ensure(bytes));
         FCK(f->keys.ensure(sizeof(uint16_t) * (size_t)n));
