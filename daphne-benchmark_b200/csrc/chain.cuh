@@ -24,11 +24,16 @@ constexpr int kLookback = 16;                   // words read at a time
 constexpr unsigned kChainPolls = 1u << 24;      // polls before a wait gives up (no healthy launch comes near)
 
 // Sum of the counts of the tiles before `tile` in column `col` of state
-// [tiles][cols]; *bad = true when a wait gave up.
+// [tiles][cols]; *bad = true when a wait gave up (after `limit` polls; 0: before
+// the first).
 template <class S>
-__device__ __forceinline__ S chain_before(const S *state, int tile, int cols, int col, bool &bad) {
+__device__ __forceinline__ S chain_before(const S *state, int tile, int cols, int col, unsigned limit, bool &bad) {
     S sum = 0;
     unsigned polls = 0;
+    if (limit == 0) {
+        bad = true;
+        return 0;
+    }
     for (int p = tile - 1; p >= 0;) {
         S v[kLookback];
 #pragma unroll
@@ -52,7 +57,7 @@ __device__ __forceinline__ S chain_before(const S *state, int tile, int cols, in
         if (end) break;
         p -= used;
         if (wait) {
-            if (++polls > kChainPolls) {
+            if (++polls > limit) {
                 bad = true;
                 break;
             }

@@ -254,15 +254,18 @@ __global__ void __launch_bounds__(kThreads) radix_hist_kernel(const uint32_t *__
 // inside a run come from the masks of the lanes with the same digit, so equal
 // digits keep their input order.  The tile is put in digit order in shared memory first,
 // so that its writes are runs of consecutive addresses.  vin == nullptr: the
-// values are the items' indices from iota on.  *err: a wait gave up (the pairs
-// are then not written).
+// values are the items' indices from iota on.  *err: a wait gave up.  The tile's
+// pairs are then not written, and what they should have been is no sort's input:
+// tiles that start later, of this pass and the next ones, do nothing (their
+// digit counts would not be the histogram's, and their writes go by both).
 template <int ITEMS, class S>
 __global__ void __launch_bounds__(kSortThreads) radix_pass_kernel(const uint32_t *__restrict__ kin,
                                                               const uint32_t *__restrict__ vin, uint32_t iota,
                                                               uint32_t *__restrict__ kout, uint32_t *__restrict__ vout,
                                                               int n, int shift, int bits,
                                                               const unsigned *__restrict__ hist, S *__restrict__ state,
-                                                              int *__restrict__ ticket, int *__restrict__ err) {
+                                                              int *__restrict__ ticket, unsigned polls,
+                                                              int *__restrict__ err) {
     constexpr int kTileItems = kSortThreads * ITEMS;
     extern __shared__ __align__(16) unsigned char s_dyn[];
     unsigned (*s_cnt)[kDigits] = reinterpret_cast<unsigned (*)[kDigits]>(s_dyn);
@@ -271,10 +274,11 @@ __global__ void __launch_bounds__(kSortThreads) radix_pass_kernel(const uint32_t
     __shared__ unsigned s_warp[2][kDigits / 32];
     __shared__ int s_tile;
     const int t = threadIdx.x, w = t >> 5, lane = t & 31;
-    if (t == 0) s_tile = atomicAdd(ticket, 1);
+    if (t == 0) s_tile = *(volatile int *)err ? -1 : atomicAdd(ticket, 1);
     for (int d = t; d < kSortWarps * kDigits; d += kSortThreads) (&s_cnt[0][0])[d] = 0;
     __syncthreads();
     const int tile = s_tile;
+    if (tile < 0) return;
     const long long base = (long long)tile * kTileItems;
     const int count = (int)(n - base < kTileItems ? n - base : kTileItems);
     const uint32_t mask = (1u << bits) - 1u;
@@ -348,7 +352,7 @@ __global__ void __launch_bounds__(kSortThreads) radix_pass_kernel(const uint32_t
         }
         S before = 0;
         if (tile > 0) {
-            before = chain_before<S>(state, tile, kDigits, t, bad);
+            before = chain_before<S>(state, tile, kDigits, t, polls, bad);
             if (!bad) Chain<S>::publish(mine, kUpToSum, before + (S)total);
         }
         s_base[t] = first + (unsigned)before - start;
@@ -500,7 +504,7 @@ size_t scan_part_ints(size_t n) { return (n + kScanTile - 1) / kScanTile + 1; }
 // Segments of equal keys in the sorted order = occupied cells: seg_start[s] and
 // seg_key[s] of every segment, in sorted order, and their number, in one read
 // of the keys (the tiles' counts are chained).  After a sort that gave up
-// (*err) there are none.
+// (*err), or a wait here that did, there are none.
 __global__ void __launch_bounds__(kSegThreads) segment_kernel(const uint32_t *__restrict__ keys, int n,
                                                            int *__restrict__ seg_start, uint32_t *__restrict__ seg_key,
                                                            int *__restrict__ nseg, uint64_t *__restrict__ state,
@@ -547,10 +551,17 @@ __global__ void __launch_bounds__(kSegThreads) segment_kernel(const uint32_t *__
         const uint64_t b = warp_chain_before(state, tile, bad);
         if (lane == 0) {
             if (!bad) Chain<uint64_t>::publish(state + tile, kUpToSum, b + total);
-            if (bad) atomicOr(err, 1);
             s_before = (unsigned)b;
             s_tile = bad ? -1 : tile;
-            if (tile == (int)gridDim.x - 1) *nseg = bad ? 0 : (int)(b + total);
+            // Whichever of the last tile and one that gives up comes second sees
+            // the other's write: the number ends up 0.
+            volatile int *out = nseg;
+            if (tile == (int)gridDim.x - 1) *out = (int)(b + total);
+            if (bad) atomicOr(err, 1);
+            if (bad || tile == (int)gridDim.x - 1) {
+                __threadfence();
+                if (*(volatile int *)err) *out = 0;
+            }
         }
     }
     __syncthreads();
@@ -1065,7 +1076,7 @@ void launch_pass(SortBuffers &b, const SortSync &y, int n, const RadixPlan &P, i
                  cudaStream_t st) {
     radix_pass_kernel<ITEMS, S><<<sort_tiles(n), kSortThreads, kPassSmem<ITEMS>, st>>>(
         b.k0, iota ? nullptr : b.v0, iota_base, b.k1, b.v1, n, pass * P.width, pass_bits(P, pass),
-        y.hist + pass * kDigits, (S *)(y.state + (size_t)pass * y.pass_bytes), y.ticket + pass, y.err);
+        y.hist + pass * kDigits, (S *)(y.state + (size_t)pass * y.pass_bytes), y.ticket + pass, b.polls, y.err);
 }
 
 }  // namespace
@@ -1125,6 +1136,7 @@ SortBuffers sort_buffers(void *scratch, int n) {
     b.v1 = (uint32_t *)take(sizeof(uint32_t) * (size_t)n);
     b.nseg = (int *)take(sizeof(int));
     b.sync = take(sync_bytes(n, kMaxPasses));
+    b.polls = kChainPolls;
     return b;
 }
 

@@ -53,11 +53,12 @@ int grid_windows(const GridMeta &meta_host, const int32_t *index, const float4 *
 // position of segment s, seg_key[s] = its key, *b.nseg = segment count
 // (device).  After the call b.k0 / b.v0 hold the sorted keys and values.
 // Returns the number of kernel launches.  *sort_error (device) is set when a
-// wait between tiles gave up; there are then no segments.
+// wait between tiles gave up (after `polls` polls); there are then no segments.
 struct SortBuffers {
     uint32_t *k0, *v0, *k1, *v1;
     int *nseg;
     void *sync;
+    unsigned polls;
 };
 // Per-device set-up (dynamic shared memory opt-in); call with the device current.
 int prepare_sort();
