@@ -28,6 +28,9 @@ int ctx_eval_view(ndt_ctx *c, CtxEvalView *v);
 // d_offsets (scans + 1 entries), total_points >= the scans' points.
 int ctx_score_batch(ndt_ctx *c, int B, int scans, const float *d_points, const int *d_offsets, int total_points,
                     const float *d_poses, double *d_score);
+// After a wait for the context's stream: NDT_OK, or the error of a map build or
+// append whose sort gave up (the context then has no map).
+int ctx_map_status(ndt_ctx *c);
 // Records an error message on the context (ndt_last_error).
 void ctx_set_error(ndt_ctx *c, const char *msg);
 

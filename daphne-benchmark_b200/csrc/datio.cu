@@ -339,6 +339,7 @@ int ndt_dat_align(ndt_ctx *ctx, ndt_dat *d, int first, int count, float *out16, 
     if (status) DCK(cudaMemcpyAsync(status, d->d_status, sizeof(int) * (size_t)count, cudaMemcpyDeviceToHost, st));
     DCK(cudaStreamSynchronize(st));
 #undef DCK
+    if (int rc = ndt::ctx_map_status(ctx)) return fail(d, rc, std::string("map: ") + ndt_last_error(ctx));
     return NDT_OK;
 }
 

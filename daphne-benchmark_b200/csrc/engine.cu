@@ -15,6 +15,7 @@
 
 #include "../../include/ndt_b200.h"
 #include "align.h"
+#include "chain.cuh"
 #include "ctx_view.h"
 #include "nvtx_range.h"
 #include "derivatives.h"
@@ -171,7 +172,8 @@ struct ndt_ctx {
     DevBuf chunks, chunk_begin, num_chunks, big_begin, small_begin, num_big, dev_launches;
     DevBuf points, offsets, guesses, states, tiles, tile_begin, num_tiles, partials, exc, out_T, out_conv, out_fit,
         out_status, ctl, p6, trans, queues, active_chunks, split_state;
-    HostBuf h_offsets, h_active, h_counters, h_out;
+    HostBuf h_offsets, h_active, h_counters, h_out;  // h_active: alignments asking; the map's sort gave up (map_status)
+    uint64_t sort_polls = kChainPolls;
     ndt_counters last{};
     long long launches = 0;
     int variant = kDefaultDerivVariant;  // FP32 derivative-pass launch shape (kDerivVariants)
@@ -292,6 +294,19 @@ int set_device(ndt_ctx *c) {
     return NDT_OK;
 }
 
+// A build or an append whose sort gave up leaves a map without voxels, or one
+// without the new points, and a sorted order that no append may merge with.
+// The kernels say so in h_active[1] (pinned, so it costs a good build no copy
+// and no wait); every call that has waited for the context's stream asks here.
+int map_status(ndt_ctx *c) {
+    volatile int *failed = c->h_active.p ? c->h_active.as<int>() + 1 : nullptr;
+    if (!failed || !*failed) return NDT_OK;
+    *failed = 0;
+    c->have_map = false;
+    c->have_windows = false;
+    return fail(c, NDT_E_CUDA, "the map's sort gave up waiting between its tiles: the map has to be set again");
+}
+
 constexpr long long kMaxWindows = 1LL << 28;        // probe windows (8 B offset and count each)
 constexpr long long kMaxWindowEntries = 1LL << 28;  // window entries (16 B each)
 
@@ -368,6 +383,10 @@ int build_grid(ndt_ctx *c, const float4 *d_map, int m) {
     c->have_map = false;
     c->have_windows = false;
     c->grid_timed = false;
+    if (!c->h_active.p) {
+        CK(c->h_active.ensure(2 * sizeof(int)));
+        c->h_active.as<int>()[1] = 0;
+    }
     if (c->profiling) {
         if (!c->grid_ev[0]) CK(cudaEventCreate(&c->grid_ev[0]));
         if (!c->grid_ev[1]) CK(cudaEventCreate(&c->grid_ev[1]));
@@ -384,6 +403,7 @@ int build_grid(ndt_ctx *c, const float4 *d_map, int m) {
     c->launches += 1;
     CK(cudaMemcpyAsync(&c->meta_host, c->meta.p, sizeof(GridMeta), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
+    if (int rc0 = map_status(c)) return rc0;  // (of the map before)
     if (c->meta_host.error == 2) return fail(c, NDT_E_ARG, "map has non-finite coordinates");
     if (c->meta_host.error) return fail(c, NDT_E_GRID, "voxel grid does not fit 32-bit cell indices");
     const size_t G = (size_t)c->meta_host.G;
@@ -394,6 +414,8 @@ int build_grid(ndt_ctx *c, const float4 *d_map, int m) {
     opt.compat = c->prm.compat;
     opt.min_points = c->prm.min_points_per_voxel;
     opt.eigen_ratio = c->prm.eigen_ratio;
+    opt.sort_polls = c->sort_polls;
+    opt.sort_failed = c->h_active.as<int>() + 1;
     bool windows = false;
     WindowBuffers wb;
     if (int rc0 = prepare_windows(c, m, windows, wb)) return rc0;
@@ -681,7 +703,6 @@ int run_batch(ndt_ctx *c, int B, const float4 *d_points, const int *d_offsets, i
     if (int rc0 = prepare_lists(c, B, max_tiles, R.L)) return rc0;
     CK(c->partials.ensure(sizeof(double) * kPartial * (size_t)max_tiles));
     CK(c->exc.ensure(sizeof(double) * kPartial * (size_t)B));
-    CK(c->h_active.ensure(sizeof(int)));
     cudaStream_t st = c->stream;
     if (first) c->ev_used = 0;
     R.P = step_params(c->prm);
@@ -770,6 +791,7 @@ int read_counters(ndt_ctx *c) {
     CK(cudaMemcpyAsync(c->h_counters.p, &c->ctl.as<RoundCtl>()->counters, sizeof(Counters), cudaMemcpyDeviceToHost,
                        c->stream));
     CK(cudaStreamSynchronize(c->stream));
+    if (int rc = map_status(c)) return rc;
     const Counters *k = c->h_counters.as<Counters>();
     c->last.rounds = (int64_t)k->rounds;
     unsigned long long dl = 0;
@@ -884,7 +906,7 @@ int staged_batch(ndt_ctx *c, int B, const int *off, const float *guesses, float 
     CK(cudaMemcpyAsync(fit, c->out_fit.p, sizeof(double) * (size_t)B, cudaMemcpyDeviceToHost, st));
     if (status) CK(cudaMemcpyAsync(status, c->out_status.p, sizeof(int) * (size_t)B, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    return NDT_OK;
+    return map_status(c);
 }
 
 int no_hook() { return NDT_OK; }
@@ -1018,6 +1040,8 @@ int ctx_score_batch(ndt_ctx *c, int B, int scans, const float *d_points, const i
     return NDT_OK;
 }
 
+int ctx_map_status(ndt_ctx *c) { return map_status(c); }
+
 void ctx_set_error(ndt_ctx *c, const char *msg) {
     if (c) c->err = msg;
 }
@@ -1117,7 +1141,7 @@ void *ndt_stream(ndt_ctx *c) { return c ? (void *)c->stream : nullptr; }
 int ndt_synchronize(ndt_ctx *c) {
     if (!c) return NDT_E_ARG;
     CK(cudaStreamSynchronize(c->stream));
-    return NDT_OK;
+    return map_status(c);
 }
 
 int ndt_set_map(ndt_ctx *c, const float *map, int m) {
@@ -1179,6 +1203,7 @@ int map_append(ndt_ctx *c, const float *pts, int k, bool host) {
     GridMeta nm;
     CK(cudaMemcpyAsync(&nm, c->meta_tmp.p, sizeof(GridMeta), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    if (int rc0 = map_status(c)) return rc0;
     if (nm.error == 2) return fail(c, NDT_E_ARG, "appended points have non-finite coordinates");
     bool inside = true;
     for (int e = 0; e < 3; ++e)
@@ -1201,6 +1226,8 @@ int map_append(ndt_ctx *c, const float *pts, int k, bool host) {
     opt.compat = c->prm.compat;
     opt.min_points = c->prm.min_points_per_voxel;
     opt.eigen_ratio = c->prm.eigen_ratio;
+    opt.sort_polls = c->sort_polls;
+    opt.sort_failed = c->h_active.as<int>() + 1;
     int nl = 0;
     rc = grid_append(map, m, k, c->meta_host, c->meta.as<GridMeta>(), opt, grid_buffers(c), c->sorted,
                      c->sorted_keys[out].as<uint32_t>(), c->sorted_order[out].as<uint32_t>(), c->append_scratch.p, st,
@@ -1304,6 +1331,12 @@ int ndt_set_side_queue_capacity(ndt_ctx *c, int pairs) {
     return NDT_OK;
 }
 
+int ndt_set_sort_wait_limit(ndt_ctx *c, int polls) {
+    if (!c) return NDT_E_ARG;
+    c->sort_polls = polls < 0 ? kChainPolls : (uint64_t)polls;
+    return NDT_OK;
+}
+
 int ndt_get_kernel_variant(ndt_ctx *c) { return c ? c->variant : NDT_E_ARG; }
 
 // Times a device batch with every launch shape of the FP32 derivative pass
@@ -1346,6 +1379,7 @@ int ndt_autotune_batch_device(ndt_ctx *c, int B, const float *d_points, const in
             if ((ee = cudaEventRecord(e1, c->stream)) != cudaSuccess || (ee = cudaEventSynchronize(e1)) != cudaSuccess ||
                 (ee = cudaEventElapsedTime(&ms, e0, e1)) != cudaSuccess)
                 return cuda_fail(c, ee, "autotune timing");
+            if (int rc = map_status(c)) return rc;
             if (best_ms < 0.0f || ms < best_ms) best_ms = ms;
         }
         return NDT_OK;
@@ -1441,6 +1475,7 @@ int ndt_grid_info(ndt_ctx *c, float *bbox6, int *dims3, int *occupied) {
     if (!c->have_map) return fail(c, NDT_E_NOMAP, "no map set");
     CK(cudaMemcpyAsync(&c->meta_host, c->meta.p, sizeof(GridMeta), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
+    if (int rc = map_status(c)) return rc;
     for (int e = 0; e < 3; ++e) {
         if (bbox6) {
             bbox6[e] = c->meta_host.minv[e];
@@ -1484,6 +1519,7 @@ int ndt_window_info(ndt_ctx *c, long long *windows, long long *entries) {
         int32_t e = 0;
         CK(cudaMemcpyAsync(&e, c->win_cursor.p, sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
+        if (int rc = map_status(c)) return rc;
         E = e;
     }
     if (windows) *windows = W;
@@ -1546,6 +1582,7 @@ int ndt_derivatives(ndt_ctx *c, const float *scan, const float *trans, int n, co
     std::vector<double> part((size_t)max_tiles * kPartial), exc(kPartial);
     CK(cudaMemcpyAsync(&nt, c->num_chunks.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    if (int rc2 = map_status(c)) return rc2;
     CK(cudaMemcpyAsync(part.data(), c->partials.p, sizeof(double) * kPartial * (size_t)nt, cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(exc.data(), c->exc.p, sizeof(double) * kPartial, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));

@@ -658,9 +658,12 @@ __device__ void compat_cell(const float4 *__restrict__ map, const uint32_t *__re
 __global__ void cell_finalize_compat_kernel(const float4 *__restrict__ map, const uint32_t *__restrict__ order,
                                             const int *__restrict__ seg_start, const uint32_t *__restrict__ seg_cell,
                                             const int *__restrict__ nseg, int n, GridMeta *__restrict__ meta,
-                                            GridBuffers buf) {
+                                            GridBuffers buf, const int *__restrict__ sort_err, int *sort_failed) {
     const int K = *nseg;
-    if (blockIdx.x == 0 && threadIdx.x == 0) meta->occupied = K;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        meta->occupied = K;
+        if (*sort_err) *sort_failed = 1;
+    }
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= K) return;
     const int lo = seg_start[s], hi = (s + 1 < K) ? seg_start[s + 1] : n;
@@ -771,9 +774,12 @@ __global__ void cell_finalize_corrected_kernel(const float4 *__restrict__ map, c
                                                const int *__restrict__ seg_start,
                                                const uint32_t *__restrict__ seg_cell, const int *__restrict__ nseg,
                                                int n, int min_points, double eig_ratio, GridMeta *__restrict__ meta,
-                                               GridBuffers buf) {
+                                               GridBuffers buf, const int *__restrict__ sort_err, int *sort_failed) {
     const int K = *nseg;
-    if (blockIdx.x == 0 && threadIdx.x == 0) meta->occupied = K;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        meta->occupied = K;
+        if (*sort_err) *sort_failed = 1;
+    }
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= K) return;
     const int lo = seg_start[s], hi = (s + 1 < K) ? seg_start[s + 1] : n;
@@ -786,9 +792,12 @@ __global__ void cell_finalize_corrected_kernel(const float4 *__restrict__ map, c
 // k_old = the slot count before the append.
 __global__ void append_mark_kernel(const uint32_t *__restrict__ new_keys, int k, const int32_t *__restrict__ slot_of,
                                    const GridMeta *__restrict__ meta, int *__restrict__ fresh,
-                                   int *__restrict__ k_old, const int *__restrict__ sort_err) {
+                                   int *__restrict__ k_old, const int *__restrict__ sort_err, int *sort_failed) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j == 0) *k_old = meta->occupied;
+    if (j == 0) {
+        *k_old = meta->occupied;
+        if (*sort_err) *sort_failed = 1;
+    }
     if (j >= k) return;
     if (*sort_err) {  // (a wait of the sort gave up: the keys are not sorted)
         fresh[j] = 0;
@@ -1148,16 +1157,16 @@ int key_bits(const GridMeta &meta_host) {
 }
 
 // Per-voxel records from the sorted order (one launch).
-int grid_finalize(const float4 *d_map, const uint32_t *order, int m, const int *nseg, GridMeta *d_meta,
-                  const NdtGridOptions &opt, GridBuffers buf, cudaStream_t st) {
+int grid_finalize(const float4 *d_map, const uint32_t *order, int m, const int *nseg, const int *sort_err,
+                  GridMeta *d_meta, const NdtGridOptions &opt, GridBuffers buf, cudaStream_t st) {
     // at most m segments: launch for m, kernels read the true count
     if (opt.compat) {
         cell_finalize_compat_kernel<<<div_up(m, 128), 128, 0, st>>>(d_map, order, buf.seg_start, buf.seg_cell, nseg,
-                                                                    m, d_meta, buf);
+                                                                    m, d_meta, buf, sort_err, opt.sort_failed);
     } else {
         cell_finalize_corrected_kernel<<<div_up(m, 128), 128, 0, st>>>(d_map, order, buf.seg_start, buf.seg_cell,
                                                                        nseg, m, opt.min_points, opt.eigen_ratio,
-                                                                       d_meta, buf);
+                                                                       d_meta, buf, sort_err, opt.sort_failed);
     }
     return 1;
 }
@@ -1165,6 +1174,7 @@ int grid_finalize(const float4 *d_map, const uint32_t *order, int m, const int *
 int grid_build(const float4 *d_map, int m, const GridMeta &meta_host, GridMeta *d_meta, const NdtGridOptions &opt,
                GridBuffers buf, void *scratch, cudaStream_t st, int *launches, SortedMap *sorted) {
     SortBuffers sb = sort_buffers((char *)scratch + kBboxBytes, m);  // after the bounding-box region
+    sb.polls = (unsigned)opt.sort_polls;
     int nl = 0;
 
     cudaMemsetAsync(buf.index, 0xff, sizeof(int32_t) * (size_t)meta_host.G, st);
@@ -1172,7 +1182,7 @@ int grid_build(const float4 *d_map, int m, const GridMeta &meta_host, GridMeta *
     cell_key_kernel<<<div_up(m, kThreads), kThreads, 0, st>>>(d_map, m, d_meta, sb.k0);
     ++nl;
     nl += sort_segments(sb, m, key_bits(meta_host), buf.seg_start, buf.seg_cell, st, true);
-    nl += grid_finalize(d_map, sb.v0, m, sb.nseg, d_meta, opt, buf, st);
+    nl += grid_finalize(d_map, sb.v0, m, sb.nseg, sort_error(sb, m), d_meta, opt, buf, st);
     if (sorted) {
         sorted->keys = sb.k0;
         sorted->order = sb.v0;
@@ -1196,6 +1206,7 @@ int grid_append(const float4 *d_map, int m_old, int k, const GridMeta &meta_host
         return (void *)r;
     };
     SortBuffers sb = sort_buffers(take(sort_scratch_bytes(k)), k);
+    sb.polls = (unsigned)opt.sort_polls;
     int *fresh = (int *)take(sizeof(int) * (size_t)k);
     int *small = (int *)take(2 * sizeof(int));  // n_fresh, k_old
     int *part = (int *)take(sizeof(int) * scan_part_ints((size_t)k));
@@ -1209,7 +1220,7 @@ int grid_append(const float4 *d_map, int m_old, int k, const GridMeta &meta_host
                                                            k, keys_out, order_out, sort_error(sb, k));
     // the touched cells: new slots in key order, records from all their points
     append_mark_kernel<<<div_up(k, kThreads), kThreads, 0, st>>>(sb.k0, k, buf.slot_of, d_meta, fresh, small + 1,
-                                                             sort_error(sb, k));
+                                                             sort_error(sb, k), opt.sort_failed);
     nl += 2;
     nl += scan_exclusive(fresh, k, small, part, st);
     append_cells_kernel<<<div_up(k, 128), 128, 0, st>>>(d_map, sb.k0, k, keys_out, order_out, n, fresh, small, small + 1,

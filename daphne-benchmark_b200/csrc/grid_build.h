@@ -21,10 +21,12 @@ struct GridBuffers {
     int32_t *slot_of;    // G dense cell -> its slot, usable or not (-1 = no points)
 };
 
-struct NdtGridOptions {
+struct NdtGridOptions {  // (no padding: part of a cached graph's key)
     int compat;
     int min_points;
     double eigen_ratio;
+    uint64_t sort_polls;  // SortBuffers::polls of the build's sort
+    int *sort_failed;     // set to 1 when that sort gave up (device-visible; the map is then without voxels)
 };
 
 // Probe-window table.  The FP32 derivative pass probes, for a point p, the

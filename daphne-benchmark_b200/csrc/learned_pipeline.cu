@@ -428,7 +428,12 @@ int ndt_align_batch_learned(ndt_mlp *c, ndt_ctx *const *levels, int n_levels, co
         LCK(cudaMemcpyAsync(choice, lb.h_choice.p, sizeof(int) * (size_t)B, cudaMemcpyDeviceToHost, s_last));
     if (start16)
         LCK(cudaMemcpyAsync(start16, lb.start.p, sizeof(float) * 16 * (size_t)B, cudaMemcpyDeviceToHost, s_last));
-    LCK(cudaStreamSynchronize(s_last));
+    LCK(cudaStreamSynchronize(s_last));  // (the other levels' work came before)
+    for (int l = 0; l < n_levels; ++l)
+        if (int rc = ndt::ctx_map_status(levels[l])) {
+            c->msg = std::string("a level's map: ") + ndt_last_error(levels[l]);
+            return rc;
+        }
     return NDT_OK;
 }
 

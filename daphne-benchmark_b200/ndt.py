@@ -106,6 +106,7 @@ def lib():
         L.ndt_kernel_variant_shape.argtypes = [C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int)]
         L.ndt_set_kernel_variant.argtypes = [ctxp, C.c_int]
         L.ndt_set_side_queue_capacity.argtypes = [ctxp, C.c_int]
+        L.ndt_set_sort_wait_limit.argtypes = [ctxp, C.c_int]
         L.ndt_get_kernel_variant.argtypes = [ctxp]
         L.ndt_set_chunk_tiles.argtypes = [ctxp, C.c_int]
         L.ndt_get_chunk_tiles.argtypes = [ctxp]
@@ -127,7 +128,7 @@ def lib():
                      "ndt_set_profiling", "ndt_kernel_variants", "ndt_kernel_variant_shape",
                      "ndt_set_kernel_variant", "ndt_window_info", "ndt_set_batch_graphs",
                      "ndt_set_side_queue_capacity", "ndt_get_kernel_variant", "ndt_autotune_batch_device",
-                     "ndt_score_batch_device", "ndt_set_chunk_tiles", "ndt_get_chunk_tiles"):
+                     "ndt_score_batch_device", "ndt_set_chunk_tiles", "ndt_get_chunk_tiles", "ndt_set_sort_wait_limit"):
             getattr(L, name).restype = C.c_int
         _LIB = L
     return _LIB
@@ -305,6 +306,10 @@ class Context:
     def set_side_queue_capacity(self, pairs=0):
         """FP64 side-queue capacity in pairs per derivative pass (0 = default 2^20)."""
         self._check(self.L.ndt_set_side_queue_capacity(self.h, int(pairs)), "set_side_queue_capacity")
+
+    def set_sort_wait_limit(self, polls=-1):
+        """Polls before a tile of the map's sort gives up (negative: the default; 0: before the first)."""
+        self._check(self.L.ndt_set_sort_wait_limit(self.h, int(polls)), "set_sort_wait_limit")
 
     def kernel_variant(self):
         return self._check(self.L.ndt_get_kernel_variant(self.h), "ndt_get_kernel_variant")

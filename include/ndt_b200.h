@@ -270,6 +270,15 @@ NDT_API int ndt_autotune_batch(ndt_ctx *ctx, int B, const float *points, const i
 NDT_API int ndt_set_side_queue_capacity(ndt_ctx *ctx, int pairs);
 
 /*
+ * Polls after which a tile of the map's sort gives up waiting for the tiles
+ * before it (< 0: the default, 2^24, which no healthy sort comes near; 0 gives
+ * up before the first poll, which exercises the error path).  A map whose sort
+ * gave up has no voxels: the next call that waits for the context's work (or
+ * ndt_synchronize) returns NDT_E_CUDA, and the map has to be set again.
+ */
+NDT_API int ndt_set_sort_wait_limit(ndt_ctx *ctx, int polls);
+
+/*
  * Grid inspection (tests): bbox (min xyz, max xyz), dims, number of occupied
  * cells, and for each occupied cell its linear index, point count, mean[3]
  * (FP64) and inverse covariance[9] (FP64) as the reference stores them.
