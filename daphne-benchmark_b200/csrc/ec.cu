@@ -344,15 +344,20 @@ __global__ void least_kernel(int *__restrict__ parent, const uint32_t *__restric
     }
 }
 
-// Point index -> label.  status[1] collects the errors: a sort that gave up is 4.
-__global__ void label_kernel(const int *__restrict__ parent, const uint32_t *__restrict__ order, int n,
+// Point index -> label.  The root is looked up again: least_kernel's store of it
+// may have been followed by another thread's path halving, whose older ancestor
+// is a node of the tree but has no least point.  status[1] collects the errors: a
+// sort that gave up is 4.
+__global__ void label_kernel(int *__restrict__ parent, const uint32_t *__restrict__ order, int n,
                              const int *__restrict__ nseg, const int *__restrict__ least,
                              const int *__restrict__ sort_err, uint32_t *__restrict__ label,
                              int *__restrict__ status) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t == 0 && *sort_err) atomicOr(status + 1, 4);
     if (t >= n || *nseg == 0) return;
-    label[order[t]] = (uint32_t)least[parent[t]];
+    const int r = find_root(parent, t);
+    if (r < 0) atomicOr(status + 1, 2);
+    label[order[t]] = r < 0 ? 0u : (uint32_t)least[r];
 }
 
 // The clusters of [lo, hi] points, as (first position, points) of the order by
