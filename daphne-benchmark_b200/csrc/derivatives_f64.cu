@@ -20,8 +20,9 @@ constexpr int kSums = 43;  // score, g[6], H[36]
 
 // The pair's contributions to the sums, in the reference's expressions as
 // written, or false when it has none.  For voxels whose inverse covariance is
-// not finite or beyond 1e30 (kSlotFlag), where a product with a zero of J or h can be
-// NaN.
+// not finite or beyond 1e30 (kSlotFlag) and points that are not finite (a caller's
+// transformed point beside them may be), where a product with a zero of J or h
+// can be NaN.
 __device__ __noinline__ bool pair_literal(double *out, const double *x, const double *ang, const double *xt,
                                           const double *C, double d1, double d2, bool hess, bool compat) {
     // point derivatives (computePointDerivatives, kernel.cpp:495-560)
@@ -89,7 +90,7 @@ __device__ __noinline__ bool pair_literal(double *out, const double *x, const do
     return true;
 }
 
-// The same for a voxel with a finite inverse covariance, added to A: every sum
+// The same for a finite point and inverse covariance, added to A: every sum
 // and product that can differ from zero, in the order and with the rounding of
 // pair_literal.  Left out are products with the zeros of J and h and the sums
 // with them (they change no bit of A: at most the sign of a zero that is added
@@ -247,6 +248,7 @@ __global__ void __launch_bounds__(kTile64, 1) derivative_f64_kernel(const __grid
         __syncwarp();
         pts[0][lane] = x.x; pts[1][lane] = x.y; pts[2][lane] = x.z;
         pts[3][lane] = px; pts[4][lane] = py; pts[5][lane] = pz;
+        const unsigned literal = __ballot_sync(kFull, !(isfinite(x.x) && isfinite(x.y) && isfinite(x.z)));
         double A[kSums];
 #pragma unroll
         for (int k = 0; k < kSums; ++k) A[k] = 0.0;
@@ -263,7 +265,7 @@ __global__ void __launch_bounds__(kTile64, 1) derivative_f64_kernel(const __grid
                 const double p0 = (double)pts[3][owner] - m.x, p1 = (double)pts[4][owner] - m.y,
                              p2 = (double)pts[5][owner] - m.z;
                 const double *icov = grid.icov64 + 9 * (size_t)slot;
-                if (code & 32u) {
+                if ((code & 32u) || ((literal >> owner) & 1u)) {
                     const double xo[3] = {x0, x1, x2}, xt[3] = {p0, p1, p2};
                     double c[kSums];
                     if (pair_literal(c, xo, s_ang, xt, icov, args.d1, args.d2, hess, COMPAT)) {
