@@ -5,21 +5,20 @@
 //
 // Work decomposition: the tile list holds ceil(n_a / TILE) tiles of TILE
 // consecutive points per alignment, handed out to the persistent blocks in
-// chunks of consecutive tiles.  Each lane keeps its FP32 sums of the current
-// alignment in shared memory and the block reduces them once per alignment
-// run, adding the FP32 lane sums in FP64 in a fixed order (across lanes, then
-// warps), writing the run's FP64 partial to the slot of its first tile (the
-// run's other slots get zeros).
+// chunks of consecutive tiles of one alignment.  Each lane keeps its FP32 sums
+// of the current chunk in shared memory and the block reduces them once per
+// chunk, adding the FP32 lane sums in FP64 in a fixed order (across warps, then
+// lanes), and writes the chunk's FP64 partial to its slot.
 //
 // Per point (one thread): the float transform and the reference's neighbour
 // search of probe.cuh (exact: the accepted pairs are the reference's), each
 // lane's pairs in its own column of shared memory.  Then, per warp:
 //   dense  (more than 32 pairs in the warp): each lane sums its own pairs
 //          into 16 FP32 point sums and contracts them with its point's
-//          Jacobian and Hessian terms once (factored form below);
+//          Jacobian and Hessian terms once (factored form: pair_f32.cuh);
 //   sparse: the pairs are appended to a per-warp ring and evaluated 32 at a
 //          time, one pair per lane, each contracted on its own; the ring is
-//          emptied at the end of the alignment run.
+//          emptied at the end of the chunk.
 // Both kinds go through one evaluation loop (eval_steps), so the pair sums
 // and the contraction appear once in the kernel; compat and corrected mode,
 // and maps with and without a probe-window table, are separate
@@ -30,8 +29,8 @@
 // infinities and NaNs propagate as in the reference.
 //
 // Passes with few chunks go to the wide kernel (derivatives_wide.cu), which
-// gives the same bits; launch_derivatives launches both where the number of
-// chunks is known on the device only, and one of them returns at once.
+// gives the same bits; launch_derivatives launches both unless the host expects
+// many chunks, and one of them returns at once.
 //
 // This file is compiled with floating-point contraction (the pair arithmetic
 // is FP32 with FMA); the exact parts live in probe.cuh with explicit

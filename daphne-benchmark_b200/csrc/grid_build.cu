@@ -901,7 +901,7 @@ __device__ __forceinline__ void write_entries(const int32_t *__restrict__ index,
 // with jobs of 1 / 2 / 3 / 4 / 16 layers.  Small tables have too few jobs of 4
 // layers to fill the chip (400k points at 1 m, 1520 jobs: 24 us, 12 us with
 // jobs of one layer): they take jobs of one.
-constexpr long long kDeepWindowJobs = 148 * 32;  // half of the chip's warps
+constexpr long long kDeepWindowJobs = 148 * 32;  // half of a B200's warps (148 SMs)
 
 template <int kWinZ>
 __global__ void __launch_bounds__(kThreads) window_kernel(const int32_t *__restrict__ index,

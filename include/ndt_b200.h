@@ -147,7 +147,8 @@ NDT_API int ndt_align_batch(ndt_ctx *ctx, int B, const float *const *scans, cons
  * Device-resident batch: scans concatenated in d_points (sum(ns) float[4]),
  * d_offsets = B+1 prefix offsets (int32, device), d_guesses = B x 16 floats
  * (device); results to device buffers d_out (B x 16), d_conv (B), d_fit (B),
- * d_status (B).  Enqueued on the context stream; call ndt_synchronize().
+ * d_status (B).  total_points sizes the scratch: d_offsets[B] or more (a
+ * buffer's capacity).  Enqueued on the context stream; call ndt_synchronize().
  */
 NDT_API int ndt_align_batch_device(ndt_ctx *ctx, int B, const float *d_points, const int *d_offsets,
                            int total_points, const float *d_guesses, float *d_out, int *d_conv,
@@ -489,7 +490,8 @@ NDT_API int ndt_dat_align(ndt_ctx *ctx, ndt_dat *dat, int first, int count, floa
  * d_out: room for total_points float4; d_out_offsets: B + 1 output offsets;
  * *out_total (host) = number of output points.  NDT_E_CAPACITY when a scan
  * spans 2^31 leaves or more, or the batch 2^31 - 1 leaves or more.  The call
- * blocks until the result is ready (it reads the key range back once).
+ * blocks until the result is ready (it reads the key range back once).  The
+ * outputs may overlay the inputs (d_out = d_points, d_out_offsets = d_offsets).
  */
 typedef struct ndt_filter ndt_filter;
 NDT_API int ndt_filter_create(int device, ndt_filter **out);
